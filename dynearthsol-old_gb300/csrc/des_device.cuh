@@ -30,9 +30,11 @@ struct Mix {
     double bulkm, shearm, cp, k;   // harmonic / arithmetic means
     double rho_qs;                 // bulkm / (pseudo_speed^2)  (geometry.cxx:356-357)
     double dt_maxwell;             // 0.5 visc_min / (1e-40 + shearm)  (geometry.cxx:303-304)
+    double lambda;                 // bulkm - 2/3 shearm  (rheology.cxx:24)
     int    count[kMaxMat];
     int    n;                      // total markers
     int    single;                 // >= 0: the only material present, with a power-of-two count
+    int    npresent, present[kMaxMat];   // the materials with a nonzero count, ascending
 };
 
 // Per-material constants (matprops.cxx:553-569 vectors, expanded to nmat).
@@ -40,6 +42,11 @@ struct MatTable {
     int    nmat, nmix;
     double rho0[kMaxMat], alpha[kMaxMat];
     double vexp_pw[kMaxMat], vexp_pw1[kMaxMat], vcoef_pow[kMaxMat], vQ[kMaxMat], vnR[kMaxMat];
+    int    visc_law[kMaxMat];      // the first material with the same four viscosity constants
+    int    visc_plain;             // for 1e-30 <= edot <= 1e30 and T > 0 every viscosity is a positive number
+    // FP32 copies for the bound of visc_clipped: pw, log2(0.25e6 vcoef_pow),
+    // log2(e) Q / nR, and log2 of the clip range
+    float  vpwf[kMaxMat], vlogf[kMaxMat], vqf[kMaxMat], vlog_min, vlog_max;
     double pls0[kMaxMat], pls1[kMaxMat], c0[kMaxMat], c1[kMaxMat], f0[kMaxMat], f1[kMaxMat];
     double d0[kMaxMat], d1[kMaxMat];
     double hslope[kMaxMat];        // (c1 - c0) / (pls1 - pls0)
@@ -66,28 +73,33 @@ __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b 
 template <class R>
 __device__ __forceinline__ R tr3(const R *s) { return s[0] + s[1] + s[2]; }
 
-// utils.hpp:78-87
-template <class R>
-__device__ __forceinline__ R second_invariant2(const R *t)
-{
-    R a = (t[0] + t[1] + t[2]) / R(3);
-    return (R(0.5) * ((t[0] - a) * (t[0] - a) + (t[1] - a) * (t[1] - a) + (t[2] - a) * (t[2] - a)) +
-            t[3] * t[3] + t[4] * t[4] + t[5] * t[5]);
-}
-
-// ---- MatProps -------------------------------------------------------------
-
-// Exact steps in the element's arithmetic type: for FP64 on the integer
-// pipes (0 + x, 2 x, x / 4, x / 3 as the FP64 unit rounds them, sf::*), for
-// FP32 the FP32 instructions themselves
+// Arithmetic in the element's type: for FP64 on the integer pipes, rounded as
+// the FP64 unit rounds it (sf::*), for FP32 the FP32 instructions themselves
 __device__ __forceinline__ double padd0(double x) { return sf::add0(x); }
 __device__ __forceinline__ float padd0(float x) { return 0.f + x; }
 __device__ __forceinline__ double ptwice(double x) { return sf::twice(x); }
 __device__ __forceinline__ float ptwice(float x) { return 2 * x; }
+__device__ __forceinline__ double phalf(double x) { return sf::half(x); }
+__device__ __forceinline__ float phalf(float x) { return 0.5f * x; }
 __device__ __forceinline__ double pquarter(double x) { return sf::quarter(x); }
 __device__ __forceinline__ float pquarter(float x) { return x / 4; }
 __device__ __forceinline__ double pdiv3(double x) { return sf::div3(x); }
 __device__ __forceinline__ float pdiv3(float x) { return x / 3; }
+__device__ __forceinline__ double pmul(double a, double b) { return sf::mul(a, b); }
+__device__ __forceinline__ float pmul(float a, float b) { return a * b; }
+__device__ __forceinline__ double pdiv(double a, double b) { return sf::div(a, b); }
+__device__ __forceinline__ float pdiv(float a, float b) { return a / b; }
+
+// utils.hpp:78-87
+template <class R>
+__device__ __forceinline__ R second_invariant2(const R *t)
+{
+    const R a = pdiv3(t[0] + t[1] + t[2]);
+    const R x = t[0] - a, y = t[1] - a, z = t[2] - a;
+    return (phalf(pmul(x, x) + pmul(y, y) + pmul(z, z)) + pmul(t[3], t[3]) + pmul(t[4], t[4]) + pmul(t[5], t[5]));
+}
+
+// ---- MatProps -------------------------------------------------------------
 
 // element mean temperature (matprops.cxx:613-618): ((((0 + a) + b) + c) + d) / 4
 template <class R>
@@ -107,7 +119,7 @@ __device__ __forceinline__ double mat_rho(const MatTable &M, const Mix &x, doubl
     if (x.single >= 0) {
         // (r * k) / k with k a power of two is r exactly
         int m = x.single;
-        return M.rho0[m] * (1 - M.alpha[m] * TinCelsius);
+        return sf::mul(M.rho0[m], 1 - sf::mul(M.alpha[m], TinCelsius));
     }
     double result = 0;
     int n = 0;
@@ -118,22 +130,58 @@ __device__ __forceinline__ double mat_rho(const MatTable &M, const Mix &x, doubl
     return result / n;
 }
 
-// matprops.cxx:607-643; edot_ii = second invariant of the (corrected) strain rate
+// Whether mat_visc's value is certainly clipped: +1 at visc_max, -1 at
+// visc_min, 0 if neither is sure.  log2 of each present material's viscosity
+// in FP32 from a bound on either side of the strain rate (FP32 rounding of
+// its deviator, 4e-7 of the largest component); the margin of 0.05 covers the
+// rounding of the rest, about 1e-4, many times over.  The mean lies between
+// the materials' least and largest viscosity.
+__device__ __forceinline__ int visc_clipped(const MatTable &M, const Mix &x, double T, const double *srate)
+{
+    float t[6], big = 0.f;
+    for (int i = 0; i < 6; ++i) {
+        t[i] = sf::to_float(srate[i]) * 1099511627776.f;      // 2^40: squares of 1e-19 stay normal
+        big = fmaxf(big, fabsf(t[i]));
+    }
+    const float Tf = sf::to_float(T);
+    const float e = sqrtf(second_invariant2(t)), err = 4e-7f * big;
+    if (!(e > 2.f * err) || !(e > 1e-17f && e < 1e17f) || !(Tf > 1.f)) return 0;
+    const float le_lo = log2f(e - err) - 40.f, le_hi = log2f(e + err) - 40.f;
+    bool above = true, below = true;
+    for (int k = 0; k < x.npresent; ++k) {
+        const int m = x.present[k];
+        const float c = M.vlogf[m] + M.vqf[m] / Tf, p0 = M.vpwf[m] * le_lo, p1 = M.vpwf[m] * le_hi;
+        above = above && c + fminf(p0, p1) > M.vlog_max + 0.05f;
+        below = below && c + fmaxf(p0, p1) < M.vlog_min - 0.05f;
+    }
+    return above ? 1 : below ? -1 : 0;
+}
+
+// matprops.cxx:607-643; srate = the (corrected) strain rate.  The reference
+// sums count / viscosity over all materials; the terms of absent ones are +0
+// and are skipped where their viscosity is a positive number, equal laws are
+// evaluated once, and where visc_clipped is sure the clip's end is the value.
 __device__ __forceinline__ double mat_visc(const MatTable &M, const Mix &x, double T,
                                            const double *srate)
 {
+    if (const int c = visc_clipped(M, x, T, srate))
+        return c > 0 ? smin(smax(M.visc_max, M.visc_min), M.visc_max) : smin(M.visc_min, M.visc_max);
     double edot = sqrt(second_invariant2(srate));
     edot = smax(edot, 1e-30);
-    double result = 0;
-    int n = 0;
-    for (int m = 0; m < M.nmat; m++) {
-        if (x.single >= 0 && m != x.single) continue;   // zero-count terms add +0
-        double visc0 = 0.25 * pow(edot, M.vexp_pw[m]) * M.vcoef_pow[m] *
-                       exp(M.vQ[m] / (M.vnR[m] * T)) * 1e6;
-        result += x.count[m] / visc0;
+    const bool skip = x.single >= 0 || (M.visc_plain && T > 0 && edot <= 1e30);
+    const int terms = skip ? x.npresent : M.nmat;
+    double result = 0, visc0 = 0;
+    int n = 0, law = -1;
+    for (int k = 0; k < terms; ++k) {
+        const int m = skip ? x.present[k] : k;
+        if (M.visc_law[m] != law) {
+            law = M.visc_law[m];
+            visc0 = 0.25 * pow(edot, M.vexp_pw[m]) * M.vcoef_pow[m] * exp(pdiv(M.vQ[m], pmul(M.vnR[m], T))) * 1e6;
+        }
+        result += pdiv((double)x.count[m], visc0);
         n += x.count[m];
     }
-    double v = n / result;
+    double v = pdiv((double)n, result);
     return smin(smax(v, M.visc_min), M.visc_max);
 }
 
@@ -418,33 +466,36 @@ __device__ __forceinline__ int principal3(const double *s, double p[3], double v
 
 // ---- rheology (rheology.cxx:108-302, 3D) ----------------------------------
 
-// a product as the FP64 unit rounds it, on the integer pipes for FP64
-// (sf::mul); FP32 products stay on the FP32 pipe
-__device__ __forceinline__ double pmul(double a, double b) { return sf::mul(a, b); }
-__device__ __forceinline__ float pmul(float a, float b) { return a * b; }
+// rheology.cxx:20-35 with lambda = bulkm - 2/3 shearm
+template <class R>
+__device__ __forceinline__ void elastic_lambda(R lambda, R shearm, const R *de, R *s)
+{
+    R dev = tr3(de);
+    const R g2 = ptwice(shearm);
+    const R ld = pmul(lambda, dev);
+    for (int i = 0; i < 3; ++i) s[i] += pmul(g2, de[i]) + ld;
+    for (int i = 3; i < 6; ++i) s[i] += pmul(g2, de[i]);
+}
 
 template <class R>
 __device__ __forceinline__ void elastic(R bulkm, R shearm, const R *de, R *s)
 {
-    R lambda = bulkm - R(2.) / R(3) * shearm;
-    R dev = tr3(de);
-    const R g2 = ptwice(shearm);
-    for (int i = 0; i < 3; ++i) s[i] += pmul(g2, de[i]) + pmul(lambda, dev);
-    for (int i = 3; i < 6; ++i) s[i] += pmul(g2, de[i]);
+    elastic_lambda(R(bulkm - R(2.) / R(3) * shearm), shearm, de, s);
 }
 
 template <class R>
 __device__ __forceinline__ void maxwell(R bulkm, R shearm, R viscosity, R dt, R dv, const R *de, R *s)
 {
-    R tmp = R(0.5) * dt * shearm / viscosity;
+    R tmp = pdiv(pmul(phalf(dt), shearm), viscosity);
     R f1 = 1 - tmp;
-    R f2 = 1 / (1 + tmp);
+    R f2 = pdiv(R(1), 1 + tmp);
     R dev = pdiv3(tr3(de));
     R s0 = pdiv3(tr3(s));
     const R g2 = ptwice(shearm);
+    const R bdv = pmul(bulkm, dv);
     for (int i = 0; i < 3; ++i)
-        s[i] = ((s[i] - s0) * f1 + g2 * (de[i] - dev)) * f2 + s0 + bulkm * dv;
-    for (int i = 3; i < 6; ++i) s[i] = (s[i] * f1 + g2 * de[i]) * f2;
+        s[i] = pmul(pmul(s[i] - s0, f1) + pmul(g2, de[i] - dev), f2) + s0 + bdv;
+    for (int i = 3; i < 6; ++i) s[i] = pmul(pmul(s[i], f1) + pmul(g2, de[i]), f2);
 }
 
 template <class R>
@@ -486,7 +537,7 @@ __device__ __forceinline__ bool surely_elastic(const double *s, double anphi, do
 // and of the bound many times over.
 __device__ __forceinline__ bool quick_elastic(const MatTable &M, const Mix &x, double pls, const double *s)
 {
-    const float pl = (float)pls;
+    const float pl = sf::to_float(pls);
     float c = 0.f, f = 0.f;
     int n = 0;
     for (int m = 0; m < M.nmat; ++m) {
@@ -526,11 +577,11 @@ __device__ __forceinline__ bool quick_elastic(const MatTable &M, const Mix &x, d
     }
     const float amc = 2.f * cohesion * sq;
     const float ten_max = (phi == 0.f) ? M.tension_maxf : fminf(M.tension_maxf, cohesion / tph);
-    float sf[6];
-    for (int i = 0; i < 6; ++i) sf[i] = (float)s[i];
-    const float mp = (sf[0] + sf[1] + sf[2]) * (1.f / 3.f);
-    const float a = sf[0] - mp, b = sf[1] - mp, cc = sf[2] - mp;
-    const float dev2 = a * a + b * b + cc * cc + 2.f * (sf[3] * sf[3] + sf[4] * sf[4] + sf[5] * sf[5]);
+    float t[6];
+    for (int i = 0; i < 6; ++i) t[i] = sf::to_float(s[i]);
+    const float mp = (t[0] + t[1] + t[2]) * (1.f / 3.f);
+    const float a = t[0] - mp, b = t[1] - mp, cc = t[2] - mp;
+    const float dev2 = a * a + b * b + cc * cc + 2.f * (t[3] * t[3] + t[4] * t[4] + t[5] * t[5]);
     const float R = sqrtf(dev2 * (2.f / 3.f)) * (1.f + 1e-5f);
     const float margin = 1e-4f * (fabsf(mp) + R) * (1.f + anphi) + 1e-30f;
     return ((mp - R) - anphi * (mp + R) + amc) > margin && ((mp + R) - ten_max) < -margin;
@@ -650,13 +701,9 @@ __device__ __forceinline__ double elem_quality(const double X[4][3], double vol,
     return nf * vol * vol / (area_sum * area_sum * area_sum);
 }
 
-// geometry.cxx:410-452; X[v][d] are the four vertex coordinates.  r1 and
-// r3 receive the bracketed cross products of nodes 1 and 3 (before the
-// scaling by iv); they are, bit for bit, the cross products tri_area forms
-// for the facets (2, 3, 0) and (0, 1, 2): each edge difference here is the
-// other's or its exact negative, and the products commute.
+// geometry.cxx:410-452; X[v][d] are the four vertex coordinates
 __device__ __forceinline__ void shape_fn(const double X[4][3], double vol, double dx[4], double dy[4],
-                                         double dz[4], double r1[3], double r3[3])
+                                         double dz[4])
 {
     const double *d0 = X[0], *d1 = X[1], *d2 = X[2], *d3 = X[3];
     double iv = 1 / (6 * vol);
@@ -666,31 +713,18 @@ __device__ __forceinline__ void shape_fn(const double X[4][3], double vol, doubl
     double y12 = d1[1] - d2[1], y13 = d1[1] - d3[1], y23 = d2[1] - d3[1];
     double z01 = d0[2] - d1[2], z02 = d0[2] - d2[2], z03 = d0[2] - d3[2];
     double z12 = d1[2] - d2[2], z13 = d1[2] - d3[2], z23 = d2[2] - d3[2];
-    r1[0] = y02 * z23 - y23 * z02;
-    r1[1] = z02 * x23 - z23 * x02;
-    r1[2] = x02 * y23 - x23 * y02;
-    r3[0] = y01 * z02 - y02 * z01;
-    r3[1] = z01 * x02 - z02 * x01;
-    r3[2] = x01 * y02 - x02 * y01;
     dx[0] = iv * (y13 * z12 - y12 * z13);
-    dx[1] = iv * r1[0];
+    dx[1] = iv * (y02 * z23 - y23 * z02);
     dx[2] = iv * (y13 * z03 - y03 * z13);
-    dx[3] = iv * r3[0];
+    dx[3] = iv * (y01 * z02 - y02 * z01);
     dy[0] = iv * (z13 * x12 - z12 * x13);
-    dy[1] = iv * r1[1];
+    dy[1] = iv * (z02 * x23 - z23 * x02);
     dy[2] = iv * (z13 * x03 - z03 * x13);
-    dy[3] = iv * r3[1];
+    dy[3] = iv * (z01 * x02 - z02 * x01);
     dz[0] = iv * (x13 * y12 - x12 * y13);
-    dz[1] = iv * r1[2];
+    dz[1] = iv * (x02 * y23 - x23 * y02);
     dz[2] = iv * (x13 * y03 - x03 * y13);
-    dz[3] = iv * r3[2];
-}
-
-__device__ __forceinline__ void shape_fn(const double X[4][3], double vol, double dx[4], double dy[4],
-                                         double dz[4])
-{
-    double r1[3], r3[3];
-    shape_fn(X, vol, dx, dy, dz, r1, r3);
+    dz[3] = iv * (x01 * y02 - x02 * y01);
 }
 
 // fields.cxx:193-241: D = sym(grad v) from the four nodal velocities V[i][d]
@@ -724,73 +758,6 @@ __device__ __forceinline__ void spin(const R V[4][3], const R *dx, const R *dy, 
     for (int i = 0; i < 4; ++i) w5 += R(0.5) * (V[i][1] * dz[i] - V[i][2] * dy[i]);
 }
 
-// FP64: the spin (fields.cxx:483-504) and the strain rate (fields.cxx:193-241)
-// of the same velocities and gradients share their products V_i,a dN_i/db,
-// formed once here.  Both sum 0.5 (bracket) over the four nodes; scaling by
-// 0.5 is exact and commutes with rounding, so 0.5 times the sum of the
-// brackets equals the reference's sum bit for bit (for terms above the
-// subnormal range).
-//
-// Each sum starts from zero in the reference; its first addition, 0 + x, is
-// x except for -0 and is formed on the integer pipes (sf::add0), as are the
-// exact scalings by 0.5 (sf::half).
-__device__ __forceinline__ void spin_and_rate(const double V[4][3], const double *dx, const double *dy,
-                                              const double *dz, double &w3, double &w4, double &w5,
-                                              double D[6])
-{
-    D[0] = sf::add0(V[0][0] * dx[0]);
-    for (int i = 1; i < 4; ++i) D[0] += V[i][0] * dx[i];
-    D[1] = sf::add0(V[0][1] * dy[0]);
-    for (int i = 1; i < 4; ++i) D[1] += V[i][1] * dy[i];
-    D[2] = sf::add0(V[0][2] * dz[0]);
-    for (int i = 1; i < 4; ++i) D[2] += V[i][2] * dz[i];
-    double t3, t4, t5, u3, u4, u5;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const double xy = V[i][0] * dy[i], yx = V[i][1] * dx[i];
-        const double xz = V[i][0] * dz[i], zx = V[i][2] * dx[i];
-        const double yz = V[i][1] * dz[i], zy = V[i][2] * dy[i];
-        if (i == 0) {
-            t3 = sf::add0(xy + yx);
-            u3 = sf::add0(xy - yx);
-            t4 = sf::add0(xz + zx);
-            u4 = sf::add0(xz - zx);
-            t5 = sf::add0(yz + zy);
-            u5 = sf::add0(yz - zy);
-        } else {
-            t3 += xy + yx;
-            u3 += xy - yx;
-            t4 += xz + zx;
-            u4 += xz - zx;
-            t5 += yz + zy;
-            u5 += yz - zy;
-        }
-    }
-    D[3] = sf::half(t3);
-    D[4] = sf::half(t4);
-    D[5] = sf::half(t5);
-    w3 = sf::half(u3);
-    w4 = sf::half(u4);
-    w5 = sf::half(u5);
-}
-
-// fields.cxx:419-433 in FP64: the reference's 2 s_ab w products appear twice
-// each; 2 (s_ab w) is formed once per pair and the factor 2 applied to the
-// sum (exact, as above; an exponent step on the integer pipes, sf::twice)
-__device__ __forceinline__ void jaumann64(double *s, double dt, double w3, double w4, double w5)
-{
-    // (products on the integer pipes, sf::mul)
-    const double p3 = sf::mul(s[3], w3), p4 = sf::mul(s[4], w4), p5 = sf::mul(s[5], w5);
-    double inc[6];
-    inc[0] = sf::twice(-p3 - p4);
-    inc[1] = sf::twice(p3 - p5);
-    inc[2] = sf::twice(p4 + p5);
-    inc[3] = sf::mul(s[0], w3) - sf::mul(s[1], w3) - sf::mul(s[4], w5) - sf::mul(s[5], w4);
-    inc[4] = sf::mul(s[0], w4) - sf::mul(s[2], w4) + sf::mul(s[3], w5) - sf::mul(s[5], w3);
-    inc[5] = sf::mul(s[1], w5) - sf::mul(s[2], w5) + sf::mul(s[3], w4) + sf::mul(s[4], w3);
-    for (int i = 0; i < 6; ++i) s[i] += sf::mul(dt, inc[i]);
-}
-
 // fields.cxx:419-433
 template <class R>
 __device__ __forceinline__ void jaumann(R *s, R dt, R w3, R w4, R w5)
@@ -811,19 +778,16 @@ __device__ __forceinline__ void jaumann(R *s, R dt, R w3, R w4, R w5)
 __device__ __forceinline__ void conduction(const double *dx, const double *dy, const double *dz,
                                            const double Tn[4], double kv, double tr[4])
 {
-    // (products on the integer pipes, sf::mul)
     double D[4][4];
     for (int i = 0; i < 4; ++i)
         for (int j = i; j < 4; ++j) {
-            D[i][j] = sf::mul(dx[i], dx[j]) + sf::mul(dy[i], dy[j]) + sf::mul(dz[i], dz[j]);
+            D[i][j] = dx[i] * dx[j] + dy[i] * dy[j] + dz[i] * dz[j];
             D[j][i] = D[i][j];
         }
-    // (the loops stay rolled: in E-A the shorter code runs faster than the
-    // matrix held in registers, which unrolling them would give)
     for (int i = 0; i < 4; ++i) {
-        double diffusion = sf::add0(sf::mul(D[i][0], Tn[0]));    // 0 + x (sf::add0)
-        for (int j = 1; j < 4; ++j) diffusion += sf::mul(D[i][j], Tn[j]);
-        tr[i] = sf::mul(diffusion, kv);
+        double diffusion = 0;
+        for (int j = 0; j < 4; ++j) diffusion += D[i][j] * Tn[j];
+        tr[i] = diffusion * kv;
     }
 }
 
@@ -836,19 +800,6 @@ __device__ __forceinline__ double min_height(const double X[4][3], double vol)
 {
     double m2 = smax(smax(tri_area2(X[0], X[1], X[2]), tri_area2(X[0], X[1], X[3])),
                      smax(tri_area2(X[2], X[3], X[0]), tri_area2(X[2], X[3], X[1])));
-    double maxa = sqrt(m2) / 2;
-    return 3 * vol / maxa;
-}
-
-// the same with the cross products of the facets (0, 1, 2) and (2, 3, 0)
-// taken from shape_fn (r3 and r1).  Out of line: E-A calls it every tenth
-// step, and kept apart its registers leave the pass's own allocation (E-A
-// 5.08 -> 5.01 ms per step on config 2).
-static __device__ __noinline__ double min_height(const double X[4][3], double vol, const double r1[3],
-                                                 const double r3[3])
-{
-    double m2 = smax(smax(r3[0] * r3[0] + r3[1] * r3[1] + r3[2] * r3[2], tri_area2(X[0], X[1], X[3])),
-                     smax(r1[0] * r1[0] + r1[1] * r1[1] + r1[2] * r1[2], tri_area2(X[2], X[3], X[1])));
     double maxa = sqrt(m2) / 2;
     return 3 * vol / maxa;
 }

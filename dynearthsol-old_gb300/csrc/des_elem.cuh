@@ -1,0 +1,473 @@
+// Element passes of the FP64 step, one thread per element: E-A (update_mesh's
+// element half, rotate_stress, the next step's contributions, the dt minimum)
+// as three kernels (geometry, rates and rotation, conduction), and E-C (NMD
+// correction, force vectors).
+//
+// What bounds them: GB300's FP64 pipe.  It retires 502 G instructions/s (a
+// warp's instruction every 20 clocks of an SM, measured with chains of DADD,
+// DMUL or DFMA at 4 to 32 warps per SM; one warp alone gets one per 68
+// clocks), and the reference's arithmetic for E-A is 385 of them per element.
+// Every product and quotient is on the integer pipes here (sf::prod on
+// operands taken apart once, sf::div), which leaves 162 (41 + 89 + 32 over
+// the three kernels; E-C 41).
+// Three kernels rather than one: the fused pass was limited by instruction
+// fetch (its 2,800 instructions of loop bodies exceed what the instruction
+// caches hold for warps at different places: a quarter of the warps' time
+// was "no instruction"), and the split bodies are 700 to 1,100 each.  The
+// gradients' way through memory that the split costs (192 B per element) is
+// cheap for a pass at a fifth of the DRAM rate.  Loops over nodes stay rolled for
+// the same reason.
+// On a 100x100x40 box (2.4M elements): E-A 1,248 us before (one kernel, 92
+// products on the integer pipes, 260 FP64 instructions), 971 us fused with
+// all products on them, 839 us split (geometry 228, rates and rotation 418
+// at the FP64 pipe's peak, conduction 193); E-C 258 -> 211 us.
+#pragma once
+
+#include "des_kernels.cuh"
+
+namespace des {
+
+// Operands and products of the pass: on the integer pipes (SOFT: sf::prod,
+// exact while the stage's operands are in sf::unpack's range) or on the
+// FP64 unit.  The results are the same bits.  put / get keep an operand in
+// shared memory, in an 8-byte column and (SOFT) a 4-byte column per thread.
+template <bool SOFT>
+struct Num;
+
+template <>
+struct Num<true> {
+    using Op = sf::Op;
+    __device__ __forceinline__ static Op op(double x, uint32_t &far) { return sf::unpack(x, far); }
+    __device__ __forceinline__ static double mul(const Op &a, const Op &b) { return sf::prod(a, b); }
+    // a / 2 (an operand in range)
+    __device__ __forceinline__ static Op half(Op a)
+    {
+        a.ex -= a.hi ? 1u << 20 : 0u;
+        return a;
+    }
+    __device__ __forceinline__ static void put(double *w, uint32_t *x, const Op &a)
+    {
+        *w = __hiloint2double((int)a.hi, (int)a.lo);
+        *x = a.ex;
+    }
+    __device__ __forceinline__ static Op get(const double *w, const uint32_t *x)
+    {
+        const double v = *w;
+        Op a;
+        a.lo = (uint32_t)__double2loint(v);
+        a.hi = (uint32_t)__double2hiint(v);
+        a.ex = *x;
+        return a;
+    }
+};
+
+template <>
+struct Num<false> {
+    using Op = double;
+    __device__ __forceinline__ static Op op(double x, uint32_t &) { return x; }
+    __device__ __forceinline__ static double mul(double a, double b) { return a * b; }
+    __device__ __forceinline__ static double half(double a) { return 0.5 * a; }
+    __device__ __forceinline__ static void put(double *w, uint32_t *, double a) { *w = a; }
+    __device__ __forceinline__ static double get(const double *w, const uint32_t *) { return *w; }
+};
+
+// ---- geometry ---------------------------------------------------------------
+
+// The edges X[i] - X[j] of the vertex pairs 01 02 03 12 13 23 in shared
+// memory, three components each, a column per thread.
+constexpr int kE01 = 0, kE02 = 3, kE03 = 6, kE12 = 9, kE13 = 12, kE23 = 15, kEdgeCols = 18;
+
+template <int BLK>
+__device__ __forceinline__ void load_edge(const double *se, int c, double a[3])
+{
+#pragma unroll
+    for (int k = 0; k < 3; ++k) a[k] = se[(c + k) * BLK];
+}
+
+// the squared norm of a x b (tri_area2's terms: the facet's cross product up
+// to the sign of both factors or of the whole, which the squares do not see)
+template <int BLK>
+__device__ __forceinline__ double edge_norm2(const double *se, int ca, int cb)
+{
+    double a[3], b[3];
+    load_edge<BLK>(se, ca, a);
+    load_edge<BLK>(se, cb, b);
+    const double d0 = a[1] * b[2] - a[2] * b[1], d1 = a[2] * b[0] - a[0] * b[2], d2 = a[0] * b[1] - a[1] * b[0];
+    return d0 * d0 + d1 * d1 + d2 * d2;
+}
+
+// min_height (geometry.cxx:280-293) from the edges: facets (0,1,2): e01 x e02,
+// (0,1,3): e01 x e03, (2,3,0): e02 x e23, (2,3,1): e12 x e23.  Out of line:
+// every tenth step calls it, and its registers stay out of the pass's own.
+template <int BLK>
+static __device__ __noinline__ double edge_min_height(const double *se, double vol)
+{
+    const double m2 = smax(smax(edge_norm2<BLK>(se, kE01, kE02), edge_norm2<BLK>(se, kE01, kE03)),
+                           smax(edge_norm2<BLK>(se, kE02, kE23), edge_norm2<BLK>(se, kE12, kE23)));
+    return 3 * vol / (sqrt(m2) / 2);
+}
+
+// The stages on the FP64 unit, for an element with an operand outside
+// sf::unpack's range (a subnormal or huge number, an infinity, NaN); out of
+// line, each from what the stage started from.
+template <int BLK>
+static __device__ __noinline__ double ea_volume_exact(const double *se)
+{
+    double a[3], b[3], c[3];                 // e01, e12, e23
+    load_edge<BLK>(se, kE01, a);
+    load_edge<BLK>(se, kE12, b);
+    load_edge<BLK>(se, kE23, c);
+    return sf::div6(a[0] * (c[1] * b[2] - b[1] * c[2]) + b[0] * (a[1] * c[2] - c[1] * a[2]) +
+                    c[0] * (b[1] * a[2] - a[1] * b[2]));
+}
+
+static __device__ __noinline__ void ea_gradients_exact(const Dev &d, int e, double vol)
+{
+    double X[4][3], dx[4], dy[4], dz[4];
+    load_xyz4(d, d.conn[e], X);
+    shape_fn(X, vol, dx, dy, dz);
+    store_shp(d, e, dx, dy, dz);
+}
+
+// volume, shape functions, mass contributions, dt minimum.  FP64 pipe 70 % and
+// integer ALU 70 % busy; 10 blocks of 128 per SM (8 or 12: the same within 1 %)
+template <bool SOFT, int BLK, int MINB>
+__global__ void __launch_bounds__(BLK, MINB) k_ea_geometry(Dev d, int e0, unsigned nblocks)
+{
+    using N = Num<SOFT>;
+    using Op = typename N::Op;
+    __shared__ double s_edge[kEdgeCols * BLK];
+    const int e = e0 + blockIdx.x * BLK + threadIdx.x;
+    const Consts &K = *d.K;
+    const bool dt_step = (K.fixed_dt == 0) && (d.clk->steps % 10 == 0);
+    if (e == 0) d.clk->mass_valid = 0;
+    const bool live = e < d.nelem;
+    double minh = 0;
+    if (live) {
+        const size_t E = d.nelem;
+        double *se = s_edge + threadIdx.x;
+        const int4 c = d.conn[e];
+        double vol;
+        {
+            double X[4][3];
+            load_xyz4(d, c, X);
+            double e01[3], e12[3], e23[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                e01[k] = X[0][k] - X[1][k];
+                e12[k] = X[1][k] - X[2][k];
+                e23[k] = X[2][k] - X[3][k];
+                se[(kE01 + k) * BLK] = e01[k];
+                se[(kE12 + k) * BLK] = e12[k];
+                se[(kE23 + k) * BLK] = e23[k];
+                se[(kE02 + k) * BLK] = X[0][k] - X[2][k];
+                se[(kE03 + k) * BLK] = X[0][k] - X[3][k];
+                se[(kE13 + k) * BLK] = X[1][k] - X[3][k];
+            }
+            // compute_volume (geometry.cxx:29-49)
+            uint32_t far = 0;
+            Op a[3], b[3], g[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                a[k] = N::op(e01[k], far);
+                b[k] = N::op(e12[k], far);
+                g[k] = N::op(e23[k], far);
+            }
+            const double c0 = N::mul(g[1], b[2]) - N::mul(b[1], g[2]);
+            const double c1 = N::mul(a[1], g[2]) - N::mul(g[1], a[2]);
+            const double c2 = N::mul(b[1], a[2]) - N::mul(a[1], b[2]);
+            vol = sf::div6(N::mul(a[0], N::op(c0, far)) + N::mul(b[0], N::op(c1, far)) + N::mul(g[0], N::op(c2, far)));
+            if (SOFT && !sf::in_range(far)) vol = ea_volume_exact<BLK>(se);
+        }
+        d.vol_old[e] = d.vol[e];
+        d.vol[e] = vol;
+        if (not_positive(vol)) atomicOr(&d.clk->status, 0x4u);
+        if (dt_step) minh = edge_min_height<BLK>(se, vol);
+        // compute_mass's element half (geometry.cxx:354-365)
+        {
+            const Mix &x = K.M.mix[d.mix[e]];
+            double Tn[4];
+            load_nodal4(d.T, c, Tn);
+            const double rT = mat_rho(K.M, x, elem_mean4(Tn[0], Tn[1], Tn[2], Tn[3]));
+            const double rho = K.is_qs ? x.rho_qs : rT;
+            d.c_mass[e] = sf::quarter(sf::mul(rho, vol));
+            if (K.thermal) d.c_tmass[e] = sf::quarter(sf::mul(sf::mul(rT, x.cp), vol));
+        }
+        // compute_shape_fn (geometry.cxx:410-452): node i's gradient is
+        // (a x b) / 6V with the edges (a, b) = (13, 12) (02, 23) (13, 03) (01, 02)
+        uint32_t far = 0;
+        const Op oiv = N::op(sf::div(1.0, sf::mul(6.0, vol)), far);
+#pragma unroll 1
+        for (int i = 0; i < 4; ++i) {
+            double ea[3], eb[3], g[3];
+            load_edge<BLK>(se, (0x0c3c >> (4 * i)) & 15, ea);
+            load_edge<BLK>(se, (0x36f9 >> (4 * i)) & 15, eb);
+            Op a[3], b[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                a[k] = N::op(ea[k], far);
+                b[k] = N::op(eb[k], far);
+            }
+            g[0] = N::mul(a[1], b[2]) - N::mul(a[2], b[1]);
+            g[1] = N::mul(a[2], b[0]) - N::mul(a[0], b[2]);
+            g[2] = N::mul(a[0], b[1]) - N::mul(a[1], b[0]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) d.shp[(size_t)(4 * k + i) * E + e] = N::mul(oiv, N::op(g[k], far));
+        }
+        if (SOFT && !sf::in_range(far)) ea_gradients_exact(d, e, vol);
+    }
+    if (dt_step) dt_reduce_and_finalize(d, minh, live, nblocks);
+}
+
+// ---- rates and rotation --------------------------------------------------------
+
+static __device__ __noinline__ void ea_rates_exact(const Dev &d, int e, double *out)
+{
+    double V[4][3], dx[4], dy[4], dz[4];
+    load_vel4(d, d.conn[e], V);
+    load_shp(d, e, dx, dy, dz);
+    strain_rate(V, dx, dy, dz, out);
+    spin(V, dx, dy, dz, out[6], out[7], out[8]);
+}
+
+static __device__ __noinline__ void ea_rotate_exact(const Dev &d, int e, double *arr, double w3, double w4, double w5)
+{
+    double s[6];
+    load6(arr, d.nelem, e, s);
+    jaumann(s, d.clk->step_dt, w3, w4, w5);
+    store6(arr, d.nelem, e, s);
+}
+
+// the next strain rate, its dvoldt contribution, rotate_stress.  89 FP64
+// instructions per element at 82 % of the nominal rate, the pipe's measured peak;
+// 7 blocks of 128 per SM (6: 2 % slower, 8 and 9 the same)
+template <bool SOFT, int BLK, int MINB>
+__global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0)
+{
+    using N = Num<SOFT>;
+    using Op = typename N::Op;
+    const int e = e0 + blockIdx.x * BLK + threadIdx.x;
+    if (e >= d.nelem) return;
+    const size_t E = d.nelem;
+    const int4 c = d.conn[e];
+    // The spin (fields.cxx:483-504) and the next strain rate
+    // (fields.cxx:193-241) of the same velocities and gradients share
+    // their products V_i,a dN_i/db.  Both sum 0.5 (bracket) over the four
+    // nodes; scaling by 0.5 is exact and commutes with rounding, so 0.5
+    // times the sum of the brackets equals the reference's sum bit for
+    // bit (for terms above the subnormal range).  A sum's first addition,
+    // 0 + x, is an integer select (sf::add0).
+    double D[6], u[3];
+    {
+        uint32_t far = 0;
+        double t[3];
+#pragma unroll 1
+        for (int i = 0; i < 4; ++i) {
+            const int n = i == 0 ? c.x : i == 1 ? c.y : i == 2 ? c.z : c.w;
+            const double *gp = d.shp + (size_t)i * E + e;
+            const Op v0 = N::op(__ldg(d.vx + n), far), v1 = N::op(__ldg(d.vy + n), far), v2 = N::op(__ldg(d.vz + n), far);
+            Op g[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) g[k] = N::op(gp[4 * k * E], far);
+            const double xx = N::mul(v0, g[0]), yy = N::mul(v1, g[1]), zz = N::mul(v2, g[2]);
+            const double xy = N::mul(v0, g[1]), yx = N::mul(v1, g[0]);
+            const double xz = N::mul(v0, g[2]), zx = N::mul(v2, g[0]);
+            const double yz = N::mul(v1, g[2]), zy = N::mul(v2, g[1]);
+            if (i == 0) {
+                D[0] = sf::add0(xx);
+                D[1] = sf::add0(yy);
+                D[2] = sf::add0(zz);
+                t[0] = sf::add0(xy + yx);
+                t[1] = sf::add0(xz + zx);
+                t[2] = sf::add0(yz + zy);
+                u[0] = sf::add0(xy - yx);
+                u[1] = sf::add0(xz - zx);
+                u[2] = sf::add0(yz - zy);
+            } else {
+                D[0] += xx;
+                D[1] += yy;
+                D[2] += zz;
+                t[0] += xy + yx;
+                t[1] += xz + zx;
+                t[2] += yz + zy;
+                u[0] += xy - yx;
+                u[1] += xz - zx;
+                u[2] += yz - zy;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) D[3 + k] = sf::half(t[k]);
+        if (SOFT && !sf::in_range(far)) {
+            double r[9];
+            ea_rates_exact(d, e, r);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) D[k] = r[k];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) u[k] = 2 * r[6 + k];
+        }
+    }
+    store6(d.srate_next, E, e, D);
+    d.c_trdv[e] = sf::mul(tr3(D), d.vol[e]);
+    // rotate_stress (fields.cxx:419-433) with u = 2 w, twice the spin:
+    // powers of two move through the products and sums exactly (the
+    // operands are in range), so dt inc is dt (sum with u) for the normal
+    // components, where the reference has 2 s_ab w, and (dt / 2) (sum
+    // with u) for the others
+    if (!(d.K->rheol & 1)) return;
+    uint32_t farw = 0;
+    const Op w3 = N::op(u[0], farw), w4 = N::op(u[1], farw), w5 = N::op(u[2], farw);
+    const Op odt = N::op(d.clk->step_dt, farw), hdt = N::half(odt);
+#pragma unroll 1
+    for (int f = 0; f < 2; ++f) {
+        double *arr = f ? d.strain : d.stress;
+        double s[6];
+        load6(arr, E, e, s);
+        uint32_t far = farw;
+        Op o[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) o[k] = N::op(s[k], far);
+        const double p3 = N::mul(o[3], w3), p4 = N::mul(o[4], w4), p5 = N::mul(o[5], w5);
+        s[0] += N::mul(odt, N::op(-p3 - p4, far));
+        s[1] += N::mul(odt, N::op(p3 - p5, far));
+        s[2] += N::mul(odt, N::op(p4 + p5, far));
+        s[3] += N::mul(hdt, N::op(N::mul(o[0], w3) - N::mul(o[1], w3) - N::mul(o[4], w5) - N::mul(o[5], w4), far));
+        s[4] += N::mul(hdt, N::op(N::mul(o[0], w4) - N::mul(o[2], w4) + N::mul(o[3], w5) - N::mul(o[5], w3), far));
+        s[5] += N::mul(hdt, N::op(N::mul(o[1], w5) - N::mul(o[2], w5) + N::mul(o[3], w4) + N::mul(o[4], w3), far));
+        if (!SOFT || sf::in_range(far))
+            store6(arr, E, e, s);
+        else
+            ea_rotate_exact(d, e, arr, 0.5 * u[0], 0.5 * u[1], 0.5 * u[2]);
+    }
+}
+
+// ---- conduction -------------------------------------------------------------------
+
+static __device__ __noinline__ void ea_conduction_exact(const Dev &d, int e, double kv)
+{
+    const size_t E = d.nelem;
+    double Tn[4], tr[4], dx[4], dy[4], dz[4];
+    load_shp(d, e, dx, dy, dz);
+    load_nodal4(d.T, d.conn[e], Tn);
+    conduction(dx, dy, dz, Tn, kv, tr);
+    for (int i = 0; i < 4; ++i) d.tmp[i * E + e] = tr[i];
+}
+
+// the conduction vector (fields.cxx:130-143) tr[i] = kv sum_j
+// (gradNi.gradNj) T_j.  gradNi.gradNj and gradNj.gradNi round
+// identically (the products commute and are summed in the same
+// order), so the 10 distinct dot products are formed once: those of
+// pairs go through shared memory, a node's own stays in its row.  Integer ALU
+// 74 %, FP64 pipe 65 % busy.
+template <bool SOFT, int BLK, int MINB>
+__global__ void __launch_bounds__(BLK, MINB) k_ea_conduction(Dev d, int e0)
+{
+    using N = Num<SOFT>;
+    using Op = typename N::Op;
+    __shared__ double s_col[18 * BLK];       // the gradients, then the dot products of pairs 01 02 03 12 13 23
+    __shared__ uint32_t s_ex[12 * BLK];
+    const int e = e0 + blockIdx.x * BLK + threadIdx.x;
+    if (e >= d.nelem) return;
+    const size_t E = d.nelem;
+    double *sg = s_col + threadIdx.x, *sd = sg + 12 * BLK;
+    uint32_t *sx = s_ex + threadIdx.x;
+    uint32_t far = 0;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) N::put(sg + k * BLK, sx + k * BLK, N::op(d.shp[k * E + e], far));   // 4 k + i: dN_i/dx_k
+#pragma unroll 1
+    for (int q = 0; q < 6; ++q) {
+        const int i = (0x211000 >> (4 * q)) & 3, j = (0x332321 >> (4 * q)) & 3;
+        double p[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            p[k] = N::mul(N::get(sg + (4 * k + i) * BLK, sx + (4 * k + i) * BLK),
+                          N::get(sg + (4 * k + j) * BLK, sx + (4 * k + j) * BLK));
+        sd[q * BLK] = p[0] + p[1] + p[2];
+    }
+    const double kv = sf::mul(d.K->M.mix[d.mix[e]].k, d.vol[e]);
+    const Op okv = N::op(kv, far);
+    double Tn[4];
+    load_nodal4(d.T, d.conn[e], Tn);
+    Op oT[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) oT[j] = N::op(Tn[j], far);
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        // the pair number of (i, j), j = 0..3 (the diagonal's nibble unused)
+        const unsigned pairs = i == 0 ? 0x2100u : i == 1 ? 0x4300u : i == 2 ? 0x5031u : 0x0542u;
+        double p[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const Op g = N::get(sg + (4 * k + i) * BLK, sx + (4 * k + i) * BLK);
+            p[k] = N::mul(g, g);
+        }
+        const double dii = p[0] + p[1] + p[2];
+        double diffusion = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const double off = sd[((pairs >> (4 * j)) & 15) * BLK];
+            const double pj = N::mul(N::op(i == j ? dii : off, far), oT[j]);
+            diffusion = j == 0 ? sf::add0(pj) : diffusion + pj;
+        }
+        d.tmp[(size_t)i * E + e] = N::mul(N::op(diffusion, far), okv);
+    }
+    if (SOFT && !sf::in_range(far)) ea_conduction_exact(d, e, kv);
+}
+
+// ---- E-C: NMD correction, element force vectors ---------------------------------
+
+static __device__ __noinline__ void ec_force_exact(const Dev &d, int e)
+{
+    double s[6];
+    load6(d.stress, d.nelem, e, s);
+    force_elem_body(d, e, d.conn[e], s);
+}
+
+// 12 blocks of 128 per SM (8: 349 us on 3.84M elements, 10: 332, 12: 330)
+template <bool SOFT, int BLK, int MINB>
+__global__ void __launch_bounds__(BLK, MINB) k_fe_c(Dev d)
+{
+    using N = Num<SOFT>;
+    using Op = typename N::Op;
+    const int e = blockIdx.x * BLK + threadIdx.x;
+    if (e >= d.nelem) return;
+    const size_t E = d.nelem;
+    const Consts &K = *d.K;
+    const int4 c = d.conn[e];
+    double s[6];
+    load6(d.stress, E, e, s);
+    double a[4];
+    load_nodal4(d.ntmp, c, a);
+    double dpe = sf::add0(a[0]);                // 0 + a0, then the rest; / 4, / 3
+    for (int i = 1; i < 4; ++i) dpe += a[i];
+    const double ddp = sf::div3(-d.dp[e] + sf::quarter(dpe));
+    for (int i = 0; i < 3; ++i) {
+        s[i] += ddp;
+        d.stress[i * E + e] = s[i];
+    }
+    double buoy = 0;
+    if (K.gravity != 0) {
+        double Tn[4];
+        load_nodal4(d.T, c, Tn);
+        buoy = sf::quarter(sf::mul(mat_rho(K.M, K.M.mix[d.mix[e]], elem_mean4(Tn[0], Tn[1], Tn[2], Tn[3])), K.gravity));
+    }
+    // fields.cxx:321-346, a node of the element per turn
+    uint32_t far = 0;
+    Op o[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) o[k] = N::op(s[k], far);
+    const Op ov = N::op(d.vol[e], far);
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        const Op gx = N::op(d.shp[(size_t)i * E + e], far), gy = N::op(d.shp[(size_t)(4 + i) * E + e], far),
+                 gz = N::op(d.shp[(size_t)(8 + i) * E + e], far);
+        const double fx = N::mul(o[0], gx) + N::mul(o[3], gy) + N::mul(o[4], gz);
+        const double fy = N::mul(o[3], gx) + N::mul(o[1], gy) + N::mul(o[5], gz);
+        const double fz = N::mul(o[4], gx) + N::mul(o[5], gy) + N::mul(o[2], gz) + buoy;
+        d.tmp[(size_t)i * E + e] = N::mul(N::op(fx, far), ov);
+        d.tmp[(size_t)(4 + i) * E + e] = N::mul(N::op(fy, far), ov);
+        d.tmp[(size_t)(8 + i) * E + e] = N::mul(N::op(fz, far), ov);
+    }
+    if (SOFT && !sf::in_range(far)) ec_force_exact(d, e);
+}
+
+}  // namespace des

@@ -12,6 +12,7 @@
 
 #include "des_gpu.h"
 #include "des_closure.cuh"
+#include "des_elem.cuh"
 #include "des_support.cuh"
 #include "des_topology.h"
 
@@ -223,6 +224,21 @@ int build_consts(des_gpu *g)
         M.d0[m] = mv(p.dilation_angle0, m);
         M.d1[m] = mv(p.dilation_angle1, m);
         M.hslope[m] = (M.c1[m] - M.c0[m]) / (M.pls1[m] - M.pls0[m]);
+        M.vpwf[m] = (float)M.vexp_pw[m];
+        M.vlogf[m] = (float)std::log2(0.25e6 * M.vcoef_pow[m]);
+        M.vqf[m] = (float)(M.vQ[m] / M.vnR[m] * 1.4426950408889634);
+        M.visc_law[m] = m;
+        for (int j = m - 1; j >= 0; --j)
+            if (M.vexp_pw[j] == M.vexp_pw[m] && M.vcoef_pow[j] == M.vcoef_pow[m] && M.vQ[j] == M.vQ[m] &&
+                M.vnR[j] == M.vnR[m])
+                M.visc_law[m] = M.visc_law[j];
+    }
+    M.vlog_min = (float)std::log2(p.visc_min);
+    M.vlog_max = (float)std::log2(p.visc_max);
+    M.visc_plain = 1;
+    for (int m = 0; m < g->nmat; ++m) {
+        const double span = 30 * std::fabs(M.vexp_pw[m]), base = std::log10(0.25e6 * M.vcoef_pow[m]);
+        if (!(base - span > -280 && base + span < 280 && span < 280 && M.vQ[m] / M.vnR[m] >= 0)) M.visc_plain = 0;
     }
     const double deg2rad = 3.1415926535897932384626433832795 / 180;
     M.phi_c = M.f0[0];
@@ -273,16 +289,19 @@ int build_consts(des_gpu *g)
         x.k = arith_mean(p.therm_cond, cnt);
         x.rho_qs = x.bulkm / (pseudo_speed * pseudo_speed);
         x.dt_maxwell = 0.5 * p.visc_min / (1e-40 + x.shearm);
+        x.lambda = x.bulkm - 2. / 3 * x.shearm;
         int n = 0, nonzero = 0, which = -1;
         for (int m = 0; m < g->nmat; ++m) {
             x.count[m] = cnt[m];
             n += cnt[m];
             if (cnt[m] != 0) {
+                x.present[nonzero] = m;
                 ++nonzero;
                 which = m;
             }
         }
         x.n = n;
+        x.npresent = nonzero;
         bool pow2 = which >= 0 && (cnt[which] & (cnt[which] - 1)) == 0;
         x.single = (nonzero == 1 && pow2) ? which : -1;
     }
@@ -536,9 +555,13 @@ void launch_eb_first(des_gpu *g, int b0, int b1)
         else
             kf_fe_b<<<n, kElemBlock, 0, st>>>(g->f, e0);
     } else if (g->d.ret_log) {
-        k_fe_b_t<true><<<n, kElemBlock, 0, st>>>(g->d, e0);
+        k_fe_b_t<true, 0><<<n, kElemBlock, 0, st>>>(g->d, e0);
+    } else if (g->hK.rheol == 7) {
+        k_fe_b_t<false, 7><<<n, kElemBlock, 0, st>>>(g->d, e0);
+    } else if (g->hK.rheol == 5) {
+        k_fe_b_t<false, 5><<<n, kElemBlock, 0, st>>>(g->d, e0);
     } else {
-        k_fe_b_t<false><<<n, kElemBlock, 0, st>>>(g->d, e0);
+        k_fe_b_t<false, 0><<<n, kElemBlock, 0, st>>>(g->d, e0);
     }
 }
 
@@ -588,7 +611,7 @@ void launch_pass(des_gpu *g, int k)
         switch (k) {
         case 0: k_fn_a<<<nb, kNodeBlock, 0, st>>>(d); break;
         case 2: k_sg_gather<<<nb, kNodeBlock, 0, st>>>(d); break;
-        case 3: k_fe_c<<<eb, kElemBlock, 0, st>>>(d); break;
+        case 3: k_fe_c<true, 128, 12><<<eb, kElemBlock, 0, st>>>(d); break;
         default:
             if (g->hK.stress_bc_sides && d.bf.nbf > 0)
                 k_stress_bc_facets<<<blocks(d.bf.nbf, 128), 128, 0, st>>>(d);
@@ -615,7 +638,12 @@ void launch_ea(des_gpu *g, int b0, int b1)
     if (g->prec == DES_PREC_FP32)
         kf_fe_a<<<b1 - b0, kElemBlock, 0, g->stream>>>(g->f, b0 * kElemBlock, nb);
     else
-        k_fe_a<<<b1 - b0, kElemBlock, 0, g->stream>>>(g->d, b0 * kElemBlock, nb);
+{
+        const int n = b1 - b0, e0 = b0 * kElemBlock;
+        k_ea_geometry<true, 128, 10><<<n, 128, 0, g->stream>>>(g->d, e0, nb);
+        k_ea_rotate<true, 128, 7><<<n, 128, 0, g->stream>>>(g->d, e0);
+        if (g->hK.thermal) k_ea_conduction<true, 128, 8><<<n, 128, 0, g->stream>>>(g->d, e0);
+    }
 }
 
 // the averaging of the output fields after a step (Output::average_fields)
@@ -719,7 +747,7 @@ __device__ __forceinline__ unsigned long long check_mix(unsigned long long z)
     return z ^ (z >> 31);
 }
 
-// sf::mul, sf::to_float, sf::add0, sf::twice, sf::half, sf::div6, sf::div3
+// sf::mul, sf::div, sf::to_float, sf::add0, sf::twice, sf::half, sf::div6, sf::div3
 // and sf::quarter against the FP64 unit's multiply, conversion, addition and
 // division
 __global__ void k_softf64_check(unsigned long long *bad, long long n, unsigned long long seed)
@@ -737,8 +765,12 @@ __global__ void k_softf64_check(unsigned long long *bad, long long n, unsigned l
         const double xs = (i & 1) ? x : sf::from_bits((r1 & keep) | ((r2 % 9) << 52));
         double h = __dmul_rn(x, y), g = sf::mul(x, y);
         nb[0] += sf::bits(h) != sf::bits(g) && !(h != h && g != g);
+        h = __ddiv_rn(x, y), g = sf::div(x, y);
+        nb[0] += sf::bits(h) != sf::bits(g) && !(h != h && g != g);
         h = __dmul_rn(x1, y1);
         g = sf::mul(x1, y1);
+        nb[1] += sf::bits(h) != sf::bits(g);
+        h = __ddiv_rn(x1, y1), g = sf::div(x1, y1);
         nb[1] += sf::bits(h) != sf::bits(g);
         float hf = __double2float_rn(x), gf = sf::to_float(x);
         nb[2] += __float_as_uint(hf) != __float_as_uint(gf) && !(hf != hf && gf != gf);
@@ -1107,7 +1139,8 @@ long long des_gpu_device_bytes(const des_gpu *g) { return g ? g->bytes : 0; }
 int des_gpu_kernels_per_step(const des_gpu *g)
 {
     if (!g) return 0;
-    int n = kStepKernels + ((g->hK.stress_bc_sides && g->d.bf.nbf > 0) ? 1 : 0);
+    int n = kStepKernels + (g->prec == DES_PREC_FP64 ? (g->hK.thermal ? 2 : 1) : 0) +   // FP64: E-A's three kernels
+            ((g->hK.stress_bc_sides && g->d.bf.nbf > 0) ? 1 : 0);
     if (g->P.surface_process_option == 1) n += g->d.bf.nbf > 0 ? 2 : 1;
     if (g->P.surface_process_option == 101) n += 1;
     // the FP32 form's elasto-plastic stress pass: the exact list, the network

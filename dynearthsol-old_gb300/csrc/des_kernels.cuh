@@ -71,6 +71,7 @@ struct Consts {
 
 struct Clock {
     double dt, time;
+    double step_dt;                    // the running step's dt (E-A forms the next one before it is done with it)
     int steps, mass_valid;
     unsigned long long minl;           // order_bits of the running minimum height
     unsigned blocks_done, status;
@@ -191,6 +192,8 @@ static __device__ __noinline__ int plastic_branch(const MatTable &M, const Mix &
     return plastic_return(x.bulkm, x.shearm, amc, anphi, anpsi, hardn, ten_max, depls, s);
 }
 
+// (RHEOL: the rheology where the kernel is built for one, 0 for K.rheol)
+template <int RHEOL>
 __device__ __forceinline__ int stress_body(const Dev &d, int e, int4 c, double edv, double dt,
                                            double s[6], double es[6], double edot[6], double &pls,
                                            double &dpls, double &dpress)
@@ -209,9 +212,9 @@ __device__ __forceinline__ int stress_body(const Dev &d, int e, int4 c, double e
     for (int i = 0; i < 6; ++i) de[i] = sf::mul(edot[i], dt);
     for (int i = 0; i < 6; ++i) es[i] += de[i];
     int flags = 0;
-    switch (K.rheol) {
+    switch (RHEOL ? RHEOL : K.rheol) {
     case 1:   // elastic
-        elastic(x.bulkm, x.shearm, de, s);
+        elastic_lambda(x.lambda, x.shearm, de, s);
         break;
     case 2: { // viscous
         double Tn[4];
@@ -223,14 +226,18 @@ __device__ __forceinline__ int stress_body(const Dev &d, int e, int4 c, double e
         double Tn[4];
         load_nodal4(d.T, c, Tn);
         double viscosity = mat_visc(M, x, elem_mean4(Tn[0], Tn[1], Tn[2], Tn[3]), edot);
-        double dv = d.vol[e] / d.vol_old[e] - 1;
+        double dv = sf::div(d.vol[e], d.vol_old[e]) - 1;
         maxwell(x.bulkm, x.shearm, viscosity, dt, dv, de, s);
     } break;
     case 5: { // elasto-plastic
         double depls = 0;
-        elastic(x.bulkm, x.shearm, de, s);
-        if (!quick_elastic(M, x, pls, s)) flags = plastic_branch(M, x, pls, depls, s);
-        pls += depls;
+        elastic_lambda(x.lambda, x.shearm, de, s);
+        if (!quick_elastic(M, x, pls, s)) {
+            flags = plastic_branch(M, x, pls, depls, s);
+            pls += depls;
+        } else {
+            pls = sf::add0(pls);         // pls + 0
+        }
         dpls = depls;
     } break;
     case 7: { // elasto-visco-plastic
@@ -238,14 +245,14 @@ __device__ __forceinline__ int stress_body(const Dev &d, int e, int4 c, double e
         double Tn[4];
         load_nodal4(d.T, c, Tn);
         double viscosity = mat_visc(M, x, elem_mean4(Tn[0], Tn[1], Tn[2], Tn[3]), edot);
-        double dv = d.vol[e] / d.vol_old[e] - 1;
+        double dv = sf::div(d.vol[e], d.vol_old[e]) - 1;
         double sv[6];
         for (int i = 0; i < 6; ++i) sv[i] = s[i];
         maxwell(x.bulkm, x.shearm, viscosity, dt, dv, de, sv);
         double svII = second_invariant2(sv);
         double sp[6];
         for (int i = 0; i < 6; ++i) sp[i] = s[i];
-        elastic(x.bulkm, x.shearm, de, sp);
+        elastic_lambda(x.lambda, x.shearm, de, sp);
         if (!quick_elastic(M, x, pls, sp)) flags = plastic_branch(M, x, pls, depls, sp);
         double spII = second_invariant2(sp);
         if (svII < spII) {
@@ -590,7 +597,7 @@ __global__ void k_stress(Dev d)
         load6(d.strain, E, e, es);
         load6(d.srate, E, e, edot);
         double pls = d.pls[e], dpls = d.dpls[e], dpress;
-        flags = stress_body(d, e, d.conn[e], d.edvoldt[e], d.clk->dt, s, es, edot, pls, dpls, dpress);
+        flags = stress_body<0>(d, e, d.conn[e], d.edvoldt[e], d.clk->dt, s, es, edot, pls, dpls, dpress);
         store6(d.stress, E, e, s);
         store6(d.strain, E, e, es);
         store6(d.srate, E, e, edot);
@@ -1013,6 +1020,7 @@ __global__ void k_fn_a(Dev d)
     if (n == 0) {
         d.clk->steps += 1;
         d.clk->time += dt;
+        d.clk->step_dt = dt;
     }
     if (n >= d.nnode) return;
     const size_t E = d.nelem;
@@ -1063,9 +1071,14 @@ constexpr int kRetRecord = 24;
 
 // (over the elements from e0, a multiple of the block size).  Registers
 // bounded for 8 blocks of 128 per SM, with the return map out of line
-// (plastic_branch): the spills fall there, where few elements go; config 2's
-// E-B 1.08 -> 0.86 ms, the yielding workload's 1.61 -> 1.42 ms.
-template <bool LOG>
+// (plastic_branch): the spills fall there, where few elements go (6 blocks
+// per SM: 8 % slower, 10: 11 %).  Built for one rheology at a time (rh_ep,
+// rh_evp): on 2.4M elements of config 2's physics E-B went from 224 to 180 us
+// with the conversions of the elastic bound, the remaining products and the
+// precomputed lambda off the FP64 pipe (44 -> 31 FP64 instructions per element;
+// 5.3 TB/s of DRAM traffic now), and on 396k elements of three layers of rh_evp
+// from 396 to 192 us (mat_visc, maxwell).
+template <bool LOG, int RHEOL>
 __global__ void __launch_bounds__(128, 8) k_fe_b_t(Dev d, int e0)
 {
     int e = e0 + gtid();
@@ -1090,7 +1103,7 @@ __global__ void __launch_bounds__(128, 8) k_fe_b_t(Dev d, int e0)
         const double pls_in = pls;
         if (LOG)
             for (int i = 0; i < 6; ++i) rec[i] = (float)s[i];
-        flags = stress_body(d, e, c, edv, d.clk->dt, s, es, edot, pls, dpls, dpress);
+        flags = stress_body<RHEOL>(d, e, c, edv, d.clk->dt, s, es, edot, pls, dpls, dpress);
         if (LOG) {
             double Tn[4];
             load_nodal4(d.T, c, Tn);
@@ -1113,7 +1126,7 @@ __global__ void __launch_bounds__(128, 8) k_fe_b_t(Dev d, int e0)
         d.pls[e] = pls;
         d.dpls[e] = dpls;
         d.dp[e] = dpress;
-        d.tmp_sg[e] = dpress * d.vol[e];
+        d.tmp_sg[e] = sf::mul(dpress, d.vol[e]);
     }
     count_eigen(d, flags);
     if (LOG) {
@@ -1129,27 +1142,6 @@ __global__ void __launch_bounds__(128, 8) k_fe_b_t(Dev d, int e0)
                 for (int i = 0; i < kRetRecord; ++i) d.ret_log[idx * kRetRecord + i] = rec[i];
         }
     }
-}
-
-// E-C: NMD correction + element force vectors (registers bounded for 9
-// blocks of 128 per SM: 1.06 -> 0.99 ms on config 2)
-__global__ void __launch_bounds__(128, 9) k_fe_c(Dev d)
-{
-    int e = gtid();
-    if (e >= d.nelem) return;
-    const size_t E = d.nelem;
-    int4 c = d.conn[e];
-    double a[4];
-    load_nodal4(d.ntmp, c, a);
-    double dpe = sf::add0(a[0]);                // 0 + a0, then the rest; / 4, / 3
-    for (int i = 1; i < 4; ++i) dpe += a[i];
-    double dp_el = sf::quarter(dpe);
-    double ddp = sf::div3(-d.dp[e] + dp_el);
-    double s[6];
-    load6(d.stress, E, e, s);
-    for (int i = 0; i < 3; ++i) s[i] += ddp;
-    for (int i = 0; i < 3; ++i) d.stress[i * E + e] = s[i];
-    force_elem_body(d, e, c, s);
 }
 
 // N-C: force gather, damping, velocity, velocity BCs, coordinates
@@ -1183,65 +1175,6 @@ __global__ void k_fn_c(Dev d)
     d.z[n] = z;
     // output.cxx:195-208 stops on NaN/Inf coordinates
     if (not_finite(x) || not_finite(y) || not_finite(z)) atomicOr(&d.clk->status, 0x2u);
-}
-
-// E-A: update_mesh element half, rotate_stress, next-step contributions, dt;
-// this launch covers the elements from e0 (a multiple of the block size), the
-// pass nblocks blocks in all.  Six blocks of 128 per SM (80 registers, a few
-// spilled): the pass waits on FP64 results and on instruction fetch more than
-// on any pipe, and the extra warps hide more of that (measured 5.16 against
-// 5.27 ms at five blocks on config 2)
-__global__ void __launch_bounds__(128, 6) k_fe_a(Dev d, int e0, unsigned nblocks)
-{
-    int e = e0 + gtid();
-    const Consts &K = *d.K;
-    const bool dt_step = (K.fixed_dt == 0) && (d.clk->steps % 10 == 0);
-    if (e == 0) d.clk->mass_valid = 0;
-    bool live = e < d.nelem;
-    double minh = 0;
-    if (live) {
-        const size_t E = d.nelem;
-        int4 c = d.conn[e];
-        double X[4][3];
-        load_xyz4(d, c, X);
-        double vol = tet_volume(X[0], X[1], X[2], X[3]);
-        d.vol_old[e] = d.vol[e];
-        d.vol[e] = vol;
-        if (not_positive(vol)) atomicOr(&d.clk->status, 0x4u);
-        double dx[4], dy[4], dz[4], r1[3], r3[3];
-        shape_fn(X, vol, dx, dy, dz, r1, r3);
-        store_shp(d, e, dx, dy, dz);
-        // the element's dt candidates here, so that the coordinates are dead
-        // before the rotation's registers are needed (geometry.cxx:280-300)
-        if (dt_step) {
-            minh = min_height(X, vol, r1, r3);
-        }
-        const Mix &x = K.M.mix[d.mix[e]];
-        {
-            double Tn[4];
-            load_nodal4(d.T, c, Tn);
-            double rT = mat_rho(K.M, x, elem_mean4(Tn[0], Tn[1], Tn[2], Tn[3]));
-            double rho = K.is_qs ? x.rho_qs : rT;
-            d.c_mass[e] = rho * vol / 4;
-            if (K.thermal) d.c_tmass[e] = rT * x.cp * vol / 4;
-        }
-        double V[4][3];
-        load_vel4(d, c, V);
-        double w3, w4, w5, D[6];
-        spin_and_rate(V, dx, dy, dz, w3, w4, w5, D);
-        if (K.rheol & 1) {
-            double s[6];
-            const double dt = d.clk->dt;
-            load6(d.stress, E, e, s);
-            jaumann64(s, dt, w3, w4, w5);
-            store6(d.stress, E, e, s);
-            load6(d.strain, E, e, s);
-            jaumann64(s, dt, w3, w4, w5);
-            store6(d.strain, E, e, s);
-        }
-        next_step_contrib_d(d, e, c, D, dx, dy, dz, vol);
-    }
-    if (dt_step) dt_reduce_and_finalize(d, minh, live, nblocks);
 }
 
 // nodal masses from the fused-pass contributions (used before a download)

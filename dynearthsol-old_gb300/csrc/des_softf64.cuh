@@ -169,39 +169,187 @@ DES_SF_HD uint64_t wide_mad(uint32_t x, uint32_t y, uint64_t c)
 #endif
 }
 
-// x * y as the FP64 unit rounds it.  Fast path (normal operands, normal
-// result) in 32-bit pieces: with the significands A = a1 2^32 + a0 and
-// B = b1 2^32 + b0 (a1, b1 of 21 bits), four 32x32 -> 64 products give the
-// 106-bit P = A B as p11 2^64 + mid 2^32 + low.  The significand of the
-// result is P >> (52 + t), t = 1 when P >= 2^105; the bits below it decide
-// the rounding (round bit, then a sticky OR of the rest).
+// An operand taken apart for products: the significand shifted left by 6
+// (hi 27 bits with the hidden bit, lo 32 bits) and the word of sign and
+// exponent.
+struct Op {
+    uint32_t lo, hi, ex;
+};
+
+// x taken apart.  far collects the largest distance of a nonzero operand's
+// exponent from the bottom of [2^-510, 2^511): while in_range(far), products
+// of the operands so far are zero or normal numbers.  A zero's significand is
+// 0 (no hidden bit).
+DES_SF_HD Op unpack(double x, uint32_t &far)
+{
+    const uint64_t b = bits(x);
+    const uint32_t h = (uint32_t)(b >> 32), l = (uint32_t)b, h2 = h + h;
+    const bool nz = (h2 | l) != 0;
+    const uint32_t f = nz ? h2 - (513u << 21) : 0u;
+    far = far > f ? far : f;
+    const uint32_t hh = nz ? ((h & 0xfffffu) | 0x100000u) : 0u;
+    Op u;
+    u.lo = l << 6;
+    u.hi = (hh << 6) | (l >> 26);
+    u.ex = h & 0xfff00000u;
+    return u;
+}
+DES_SF_HD bool in_range(uint32_t far) { return far < (1021u << 21); }
+
+// a b as the FP64 unit rounds it, for operands in unpack()'s range (any
+// bits otherwise).  With both significands shifted by 6, the 118-bit
+// product P holds the result's 53-bit significand at bit 64 (t = 0) or 65
+// (t = 1, P >= 2^117): four 32x32 -> 64 products, one shift by t, and the
+// rounding as one carry chain (2^63 - 1 added to the bits below, plus the
+// carry of the sticky bits and the significand's last bit: round to nearest
+// even).  The signs and exponents add in their word; the sum's range is
+// unpack()'s promise.  22 instructions and no branch, against 35 and a branch
+// for a product that checks its own operands: operands are taken apart once,
+// and a group of products is checked once.
+DES_SF_HD double prod(Op a, Op b)
+{
+    const uint32_t ex = a.ex + b.ex - (1024u << 20);
+    const uint32_t sign = (a.ex ^ b.ex) & 0x80000000u;
+    uint32_t lo, hi, top;
+#if defined(__CUDA_ARCH__)
+    asm("{\n\t.reg .b64 p, s, m;\n\t.reg .b32 low, mid, sl, sh, m0, m1, t, r, e;\n\t"
+        "mul.wide.u32 p, %3, %5;\n\t"
+        "mul.wide.u32 s, %3, %6;\n\t"
+        "mul.wide.u32 m, %4, %6;\n\t"
+        "mad.wide.u32 s, %4, %5, s;\n\t"
+        "mov.b64 {low, mid}, p;\n\t"
+        "mov.b64 {sl, sh}, s;\n\t"
+        "mov.b64 {m0, m1}, m;\n\t"
+        "add.cc.u32 mid, mid, sl;\n\t"
+        "addc.cc.u32 m0, m0, sh;\n\t"
+        "addc.u32 m1, m1, 0;\n\t"
+        "mov.b32 %2, m1;\n\t"
+        "shr.u32 t, m1, 21;\n\t"
+        "lop3.b32 low, mid, t, low, 0xEA;\n\t"      // the bit the shift drops joins the sticky bits
+        "shf.r.clamp.b32 mid, mid, m0, t;\n\t"
+        "shf.r.clamp.b32 m0, m0, m1, t;\n\t"
+        "shr.u32 m1, m1, t;\n\t"
+        "mad.lo.u32 e, t, 0x100000, %7;\n\t"
+        "lop3.b32 r, m0, 1, low, 0xEA;\n\t"
+        "add.cc.u32 r, r, 0xffffffff;\n\t"
+        "addc.cc.u32 mid, mid, 0x7fffffff;\n\t"
+        "addc.cc.u32 %0, m0, 0;\n\t"
+        "addc.u32 %1, m1, e;\n\t}"
+        : "=r"(lo), "=r"(hi), "=r"(top)
+        : "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(ex));
+#else
+    const uint64_t p = wide_mul(a.lo, b.lo), s = wide_mad(a.hi, b.lo, wide_mul(a.lo, b.hi));
+    const uint64_t c = (p >> 32) + (uint32_t)s;
+    uint64_t m = wide_mul(a.hi, b.hi) + (s >> 32) + (c >> 32);
+    top = (uint32_t)(m >> 32);
+    const uint32_t t = (uint32_t)(m >> 53);
+    const uint32_t low = (uint32_t)p | ((uint32_t)c & t);
+    const uint32_t mid = (uint32_t)(((m << 32) | (uint32_t)c) >> t);
+    m >>= t;
+    const uint64_t up = ((uint64_t)mid + 0x7fffffffu + (uint64_t)((low | ((uint32_t)m & 1)) != 0)) >> 32;
+    m += up;
+    lo = (uint32_t)m;
+    hi = (uint32_t)(m >> 32) + ex + (t << 20);
+#endif
+    if (top == 0) hi = sign;     // a zero operand (a nonzero product has top >= 2^20)
+    return from_bits(((uint64_t)hi << 32) | lo);
+}
+
+// x * y as the FP64 unit rounds it
 DES_SF_HD double mul(double x, double y)
 {
-    const uint64_t a = bits(x), b = bits(y);
-    const uint32_t ah = (uint32_t)(a >> 32), bh = (uint32_t)(b >> 32);
-    const uint32_t ea = (ah >> 20) & 0x7ff, eb = (bh >> 20) & 0x7ff;
-    if (ea - 1 < 2046u && eb - 1 < 2046u) {
-        const uint32_t a0 = (uint32_t)a, b0 = (uint32_t)b;
-        const uint32_t a1 = (ah & 0xfffffu) | 0x100000u, b1 = (bh & 0xfffffu) | 0x100000u;
-        const uint64_t p00 = wide_mul(a0, b0);
-        const uint64_t p01 = wide_mad(a0, b1, p00 >> 32);
-        const uint64_t p10 = wide_mad(a1, b0, p01);
-        const uint64_t p11 = wide_mad(a1, b1, p10 >> 32);
-        const uint32_t mid = (uint32_t)p10, low = (uint32_t)p00;
-        const uint32_t t = (uint32_t)(p11 >> 41);
-        const int e = (int)(ea + eb) - 1023 + (int)t;
-        if ((uint32_t)(e - 1) < 2046u) {
-            const uint32_t sh = 12 - t;
-            const uint64_t m = (p11 << sh) | (mid >> (32 - sh));
-            const uint32_t rem = mid << sh;
-            const uint32_t up = (rem >> 31) & (uint32_t)((((rem << 1) | low) != 0) | ((uint32_t)m & 1));
-            return from_bits(((((uint64_t)(e - 1)) << 52) + m + up) | ((a ^ b) & kSign));
-        }
-    }
-    // a zero times a finite number (frequent: zero velocity components and
-    // shape-function derivatives) without the call
-    if (((a & kAbs) == 0 && eb != 2047) || ((b & kAbs) == 0 && ea != 2047)) return from_bits((a ^ b) & kSign);
-    return from_bits(mul_slow(a, b));
+    uint32_t far = 0;
+    const Op a = unpack(x, far), b = unpack(y, far);
+    if (in_range(far)) return prod(a, b);
+    return from_bits(mul_slow(bits(x), bits(y)));
+}
+
+// ---- quotients ----------------------------------------------------------------
+// The FP64 unit's division takes about nine FP64 instructions; on the integer
+// pipes the reciprocal of the denominator's significand comes from an FP32
+// reciprocal and two Newton steps in fixed point (64 bits, relative error
+// below 2^-58), the quotient's significand from one high product, and its
+// remainder, exact in 64 bits, moves it to the nearest where the candidate is
+// one off.  A quotient of two 53-bit significands is never half way between
+// two of them, so the nearest is the rounded quotient.
+
+#if defined(__CUDACC__)
+static __host__ __device__ __noinline__
+#else
+static
+#endif
+double div_slow(double a, double b) { return a / b; }
+
+// A denominator: its significand and about 2^115 / m.
+struct Den {
+    uint64_t m, y;
+    uint32_t ex;
+};
+
+// the reciprocal seed: about 2^31 / x for the significand x in [1, 2) whose
+// top 23 fraction bits are f, within 2^-20 of it, in [2^30, 2^31)
+DES_SF_HD uint32_t rcp_seed(uint32_t f)
+{
+#if defined(__CUDA_ARCH__)
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(float_from_bits(0x3f800000u | f)));
+    uint32_t b = __float_as_uint(r);
+#else
+    const float r = 1.0f / float_from_bits(0x3f800000u | f);
+    uint32_t b;
+    memcpy(&b, &r, 4);
+#endif
+    b = b > 0x3f000000u ? b : 0x3f000000u;
+    return b >= 0x3f800000u ? 0x7fffffffu : ((b & 0x7fffffu) | 0x800000u) << 7;
+}
+
+// b as a denominator; far as in unpack (a zero is out of range here)
+DES_SF_HD Den denominator(double b, uint32_t &far)
+{
+    const uint64_t v = bits(b);
+    const uint32_t f = ((uint32_t)(v >> 32) << 1) - (513u << 21);
+    far = far > f ? far : f;
+    Den d;
+    d.m = (v & kFrac) | kHidden;
+    d.ex = (uint32_t)(v >> 32) & 0xfff00000u;
+    const uint64_t M = d.m << 11;
+    const uint32_t y0 = rcp_seed((uint32_t)(M >> 40) & 0x7fffffu);
+    // e0 = 2^62 - M y0 / 2^32 (M y0 is near 2^94)
+    const uint64_t p = wide_mad((uint32_t)(M >> 32), y0, wide_mul((uint32_t)M, y0) >> 32);
+    const int32_t e0 = (int32_t)((int64_t)((1ull << 62) - p) >> 11);
+    const uint64_t y1 = ((uint64_t)y0 << 32) + (uint64_t)(((int64_t)e0 * (int64_t)y0) >> 19);
+    const int32_t e1 = (int32_t)((1ull << 62) - mulhi64(M, y1));
+    d.y = y1 + (uint64_t)(((int64_t)e1 * (int64_t)(y1 >> 32)) >> 30);
+    return d;
+}
+
+// a / b as the FP64 unit rounds it, for a in unpack's range (collected in
+// far) and b from denominator()
+DES_SF_HD double quotient(double a, const Den &b, uint32_t &far)
+{
+    const uint64_t v = bits(a);
+    const uint32_t h = (uint32_t)(v >> 32), h2 = h + h;
+    const bool nz = (h2 | (uint32_t)v) != 0;
+    const uint32_t f = nz ? h2 - (513u << 21) : 0u;
+    far = far > f ? far : f;
+    const uint64_t m = (v & kFrac) | kHidden;
+    const uint32_t s = (uint32_t)(m < b.m);              // a quotient below 1 takes one more bit
+    const uint32_t sh = 10 - s;
+    uint64_t q = (mulhi64(m << 11, b.y) + (1ull << (sh - 1))) >> sh;
+    const int64_t r = (int64_t)((m << (52 + s)) - q * b.m), half = (int64_t)(b.m >> 1);
+    q += (uint64_t)(r > half) - (uint64_t)(r < -half);
+    const uint32_t ex = (h & 0xfff00000u) - b.ex + ((1022u - s) << 20);
+    const uint64_t w = q + ((uint64_t)ex << 32);
+    return from_bits(nz ? w : (uint64_t)((h ^ b.ex) & 0x80000000u) << 32);
+}
+
+// x / y as the FP64 unit rounds it
+DES_SF_HD double div(double x, double y)
+{
+    uint32_t far = 0;
+    const Den d = denominator(y, far);
+    const double q = quotient(x, d, far);
+    return in_range(far) ? q : div_slow(x, y);
 }
 
 // 0.0 + x as the FP64 unit rounds it: x itself, except that -0.0 gives
@@ -221,7 +369,8 @@ DES_SF_HD double twice(double x)
     const uint64_t b = bits(x);
     const uint32_t e = (uint32_t)(b >> 52) & 0x7ff;
     if (e - 1 < 2045u) return from_bits(b + (1ull << 52));
-    return mul(x, 2.0);
+    if ((b & kAbs) == 0) return x;
+    return from_bits(mul_slow(b, 0x4000000000000000ull));
 }
 
 DES_SF_HD double half(double x)
@@ -229,7 +378,8 @@ DES_SF_HD double half(double x)
     const uint64_t b = bits(x);
     const uint32_t e = (uint32_t)(b >> 52) & 0x7ff;
     if (e - 2 < 2045u) return from_bits(b - (1ull << 52));
-    return mul(x, 0.5);
+    if ((b & kAbs) == 0) return x;
+    return from_bits(mul_slow(b, 0x3fe0000000000000ull));
 }
 
 // x / 4 (x * 0.25) as the FP64 unit rounds it
@@ -238,7 +388,8 @@ DES_SF_HD double quarter(double x)
     const uint64_t b = bits(x);
     const uint32_t e = (uint32_t)(b >> 52) & 0x7ff;
     if (e - 3 < 2044u) return from_bits(b - (2ull << 52));
-    return mul(x, 0.25);
+    if ((b & kAbs) == 0) return x;
+    return from_bits(mul_slow(b, 0x3fd0000000000000ull));
 }
 
 // x / (3 2^k), k = 0 or 1, for the cases the fast path of div3k leaves:

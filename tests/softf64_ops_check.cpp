@@ -1,0 +1,82 @@
+// Host check of the grouped integer-pipe product (unpack, prod, in_range), the
+// quotient (div) of dynearthsol-old_gb300/csrc/des_softf64.cuh against the
+// host's IEEE arithmetic, bit for bit.
+//   softf64_ops_check <pairs per kind>  -> one line per kind; exit 1 on a mismatch
+#include "des_softf64.cuh"
+
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+
+using namespace des::sf;
+
+static uint64_t splitmix(uint64_t &s)
+{
+    uint64_t z = (s += 0x9e3779b97f4a7c15ull);
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+    return z ^ (z >> 31);
+}
+
+// significands: any, zero, all ones, few bits at the top, few at the bottom
+static double mk(uint64_t &s, uint64_t e)
+{
+    const uint64_t r = splitmix(s), k = splitmix(s);
+    uint64_t f = r & kFrac;
+    switch (k % 8) {
+    case 0: f = 0; break;
+    case 1: f = kFrac; break;
+    case 2: f &= ~((1ull << (k >> 8) % 52) - 1); break;
+    case 3: f &= (1ull << (k >> 8) % 52) - 1; break;
+    }
+    return from_bits((r & kSign) | (e << 52) | f);
+}
+
+// exponents: 0 near 1; 1 the edges of unpack's range; 2 any; 3 zeros,
+// subnormals, infinities, NaN against anything; 4 equal or adjacent operands
+static void pair(int kind, uint64_t &s, double &x, double &y)
+{
+    const uint64_t a = splitmix(s), b = splitmix(s);
+    switch (kind) {
+    case 0: x = mk(s, 1000 + a % 47); y = mk(s, 1000 + b % 47); break;
+    case 1: x = mk(s, (a & 1 ? 510 : 1530) + (a >> 8) % 6); y = mk(s, (b & 1 ? 510 : 1530) + (b >> 8) % 6); break;
+    case 2: x = mk(s, a % 2047); y = mk(s, b % 2047); break;
+    case 3:
+        x = mk(s, a & 1 ? 0 : 2047);
+        y = mk(s, b & 1 ? (b >> 8) % 2048 : 1000 + (b >> 8) % 47);
+        if (a & 2) x = from_bits(bits(x) & (kSign | kInf));
+        if (b & 2) { const double t = x; x = y; y = t; }
+        break;
+    default: x = mk(s, 1000 + a % 47); y = from_bits(bits(x) + b % 7 - 3); break;
+    }
+}
+
+static bool same(double a, double b) { return bits(a) == bits(b) || (std::isnan(a) && std::isnan(b)); }
+
+int main(int argc, char **argv)
+{
+    const long long per = argc > 1 ? atoll(argv[1]) : 1000000;
+    long long total = 0;
+    for (int kind = 0; kind < 5; ++kind) {
+        uint64_t s = 0xd1f0000ull + 1000003ull * kind;
+        long long bad = 0, grouped = 0;
+        for (long long i = 0; i < per; ++i) {
+            double x, y;
+            pair(kind, s, x, y);
+            volatile double vx = x, vy = y;
+            const double m = vx * vy, q = vx / vy;
+            uint32_t far = 0;
+            const Op a = unpack(x, far), b = unpack(y, far);
+            if (in_range(far)) {
+                ++grouped;
+                bad += bits(m) != bits(prod(a, b));
+            }
+            bad += !same(q, div(x, y));
+        }
+        // the range itself: kinds 0 and 4 lie inside it, kind 3's infinities never do
+        if ((kind == 0 || kind == 4) && grouped != per) ++bad;
+        printf("kind %d: %lld pairs, %lld mismatches\n", kind, per, bad);
+        total += bad;
+    }
+    return total ? 1 : 0;
+}
