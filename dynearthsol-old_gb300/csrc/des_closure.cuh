@@ -224,13 +224,13 @@ template <int RHEOL>
 __global__ void __launch_bounds__(128, 12) kf_fe_b_ep(DevF d, int e0)
 {
     const int e = e0 + gtid();
-    if (e == 0) d.clk->mass_valid = 1;
     const bool live = e < d.nelem;
+    const int4 c = live ? d.conn[e] : int4{0, 0, 0, 0};
+    if (e == 0) d.clk->mass_valid = 1;
     bool pending = false;
     if (live) {
         const size_t E = d.nelem;
         const ConstsF &F = *d.F;
-        const int4 c = d.conn[e];
         const MixF &xf = F.mix[d.mix[e]];
         const float edv = (d.ntmp[c.x] + d.ntmp[c.y] + d.ntmp[c.z] + d.ntmp[c.w]) * 0.25f;
         d.edvoldt[e] = edv;
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(128, 12) kf_fe_b_ep(DevF d, int e0)
         f_load6(d.stress, E, e, so);
         f_load6(d.strain, E, e, es);
         f_load6(d.srate_next, E, e, edot);
-        const float dt = (float)d.clk->dt;
+        const float dt = sf::to_float(d.clk->dt);
         const float div = tr3(edot);
         for (int i = 0; i < 3; ++i) edot[i] += (edv - div) * (1.f / 3.f);
         float de[6], st[6];
@@ -250,9 +250,9 @@ __global__ void __launch_bounds__(128, 12) kf_fe_b_ep(DevF d, int e0)
         f_store6(d.strain, E, e, es);
         f_store6(d.srate, E, e, edot);
         elastic(xf.bulkm, xf.shearm, de, st);
-        const float s0f = (float)d.s0[e];
+        const float s0f = sf::to_float(d.s0[e]);
         float amc, anphi, ten_max;
-        f_plastic_props(F, xf, (float)d.pls[e], amc, anphi, ten_max);
+        f_plastic_props(F, xf, sf::to_float(d.pls[e]), amc, anphi, ten_max);
         bool clear = f_surely_elastic(st, s0f, anphi, amc, ten_max);
         if (!clear) {
             float p[3];
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(128, 12) kf_fe_b_ep(DevF d, int e0)
             bool plastic = true;
             if (RHEOL == 7) {
                 const float visc = f_visc(F, xf, f_elem_T(d, c), edot);
-                const float dv = (float)(d.vol[e] / d.vol_old[e] - 1);
+                const float dv = sf::to_float(sf::div(d.vol[e], d.vol_old[e]) - 1);
                 float sv[6];
                 for (int i = 0; i < 6; ++i) sv[i] = so[i];
                 maxwell(xf.bulkm, xf.shearm, visc, dt, dv, de, sv);

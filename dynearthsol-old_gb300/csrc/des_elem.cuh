@@ -139,14 +139,14 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_geometry(Dev d, int e0, unsign
     __shared__ double s_edge[kEdgeCols * BLK];
     const int e = e0 + blockIdx.x * BLK + threadIdx.x;
     const Consts &K = *d.K;
+    const bool live = e < d.nelem;
+    const int4 c = live ? d.conn[e] : int4{0, 0, 0, 0};
     const bool dt_step = (K.fixed_dt == 0) && (d.clk->steps % 10 == 0);
     if (e == 0) d.clk->mass_valid = 0;
-    const bool live = e < d.nelem;
     double minh = 0;
     if (live) {
         const size_t E = d.nelem;
         double *se = s_edge + threadIdx.x;
-        const int4 c = d.conn[e];
         double vol;
         {
             double X[4][3];
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0)
         for (int i = 0; i < 4; ++i) {
             const int n = i == 0 ? c.x : i == 1 ? c.y : i == 2 ? c.z : c.w;
             const double *gp = d.shp + (size_t)i * E + e;
-            const Op v0 = N::op(__ldg(d.vx + n), far), v1 = N::op(__ldg(d.vy + n), far), v2 = N::op(__ldg(d.vz + n), far);
+            const Op v0 = N::op(d.vx[n], far), v1 = N::op(d.vy[n], far), v2 = N::op(d.vz[n], far);
             Op g[3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) g[k] = N::op(gp[4 * k * E], far);
@@ -368,6 +368,7 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_conduction(Dev d, int e0)
     const int e = e0 + blockIdx.x * BLK + threadIdx.x;
     if (e >= d.nelem) return;
     const size_t E = d.nelem;
+    const int4 c = d.conn[e];
     double *sg = s_col + threadIdx.x, *sd = sg + 12 * BLK;
     uint32_t *sx = s_ex + threadIdx.x;
     uint32_t far = 0;
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_conduction(Dev d, int e0)
     const double kv = sf::mul(d.K->M.mix[d.mix[e]].k, d.vol[e]);
     const Op okv = N::op(kv, far);
     double Tn[4];
-    load_nodal4(d.T, d.conn[e], Tn);
+    load_nodal4(d.T, c, Tn);
     Op oT[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) oT[j] = N::op(Tn[j], far);

@@ -123,9 +123,9 @@ __device__ __forceinline__ void load_xyz4(const Dev &d, int4 c, double X[4][3])
     const int n[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        X[i][0] = __ldg(d.x + n[i]);
-        X[i][1] = __ldg(d.y + n[i]);
-        X[i][2] = __ldg(d.z + n[i]);
+        X[i][0] = d.x[n[i]];
+        X[i][1] = d.y[n[i]];
+        X[i][2] = d.z[n[i]];
     }
 }
 __device__ __forceinline__ void load_vel4(const Dev &d, int4 c, double V[4][3])
@@ -133,17 +133,17 @@ __device__ __forceinline__ void load_vel4(const Dev &d, int4 c, double V[4][3])
     const int n[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        V[i][0] = __ldg(d.vx + n[i]);
-        V[i][1] = __ldg(d.vy + n[i]);
-        V[i][2] = __ldg(d.vz + n[i]);
+        V[i][0] = d.vx[n[i]];
+        V[i][1] = d.vy[n[i]];
+        V[i][2] = d.vz[n[i]];
     }
 }
 __device__ __forceinline__ void load_nodal4(const double *a, int4 c, double out[4])
 {
-    out[0] = __ldg(a + c.x);
-    out[1] = __ldg(a + c.y);
-    out[2] = __ldg(a + c.z);
-    out[3] = __ldg(a + c.w);
+    out[0] = a[c.x];
+    out[1] = a[c.y];
+    out[2] = a[c.z];
+    out[3] = a[c.w];
 }
 __device__ __forceinline__ void load_shp(const Dev &d, int e, double dx[4], double dy[4],
                                          double dz[4])
@@ -177,6 +177,42 @@ __device__ __forceinline__ void store6(double *a, size_t E, int e, const double 
 #pragma unroll
     for (int i = 0; i < 6; ++i) a[i * E + e] = s[i];
 }
+
+// A walk over a node's support list: f(value) in the list's order, with the
+// loads of kBatch entries in flight at a time.  (One entry after the other, a
+// walk waits out two memory latencies per entry; the FP64 sums below wait for
+// the FP64 pipe besides.)
+template <int kBatch, class Load, class F>
+__device__ __forceinline__ void walk(const unsigned *ent, int q0, int q1, Load load, F f)
+{
+    int q = q0;
+    for (; q + kBatch <= q1; q += kBatch) {
+        unsigned p[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) p[k] = __ldg(ent + q + k);
+        decltype(load(0u)) v[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) v[k] = load(p[k]);
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) f(v[k]);
+    }
+    if (q < q1) {
+        unsigned p[kBatch - 1];
+#pragma unroll
+        for (int k = 0; k < kBatch - 1; ++k) p[k] = __ldg(ent + min(q + k, q1 - 1));
+        decltype(load(0u)) v[kBatch - 1];
+#pragma unroll
+        for (int k = 0; k < kBatch - 1; ++k) v[k] = load(p[k]);
+#pragma unroll
+        for (int k = 0; k < kBatch - 1; ++k)
+            if (q + k < q1) f(v[k]);
+    }
+}
+
+template <class R>
+struct Three {
+    R x, y, z;
+};
 
 // ---- shared per-element / per-node bodies ---------------------------------
 
@@ -566,10 +602,11 @@ __global__ void k_sg_gather(Dev d)
 {
     int n = gtid();
     if (n >= d.nnode) return;
+    const int q0 = d.sup_off[n], q1 = d.sup_off[n + 1];
     double s = 0.;
-    for (int q = d.sup_off[n]; q < d.sup_off[n + 1]; ++q) s += d.tmp_sg[__ldg(d.sup_ent + q) >> 2];
-    s /= d.vol_n[n];
-    d.ntmp[n] = s;
+    walk<4>(d.sup_ent, q0, q1, [&](unsigned p) { return d.tmp_sg[p >> 2]; },
+            [&](double v) { s += v; });
+    d.ntmp[n] = sf::div(s, d.vol_n[n]);
 }
 
 // geometry.cxx:166-174
@@ -1011,53 +1048,98 @@ __global__ void k_prime(Dev d)
     next_step_contrib(d, e, c, V, dx, dy, dz, d.vol[e]);
 }
 
-// N-A: start of a step (dynearthsol.cxx:358-362, 365 node half)
-__global__ void k_fn_a(Dev d)
+// the nodal masses (geometry.cxx:370-381) from E-A's contributions on the FP64
+// unit: for a node whose sums leave sf::PosSum's range
+static __device__ __noinline__ void node_masses_exact(const Dev &d, int q0, int q1, double out[3])
+{
+    double vn = 0, m = 0, tm = 0;
+    for (int q = q0; q < q1; ++q) {
+        const size_t e = __ldg(d.sup_ent + q) >> 2;
+        vn += d.vol[e];
+        m += d.c_mass[e];
+        if (d.K->thermal) tm += d.c_tmass[e];
+    }
+    out[0] = vn;
+    out[1] = m;
+    out[2] = tm;
+}
+
+// the same as sums of positive numbers on the integer pipes
+__device__ __forceinline__ void node_masses(const Dev &d, int q0, int q1, double &vn, double &m, double &tm)
+{
+    const bool thermal = d.K->thermal;
+    vn = m = tm = 0;
+    if (q0 == q1) return;
+    const size_t e0 = __ldg(d.sup_ent + q0) >> 2;
+    sf::PosSum sv = sf::pos_first(d.vol[e0]), sm = sf::pos_first(d.c_mass[e0]),
+               st = sf::pos_first(thermal ? d.c_tmass[e0] : 1.0);
+    walk<4>(
+        d.sup_ent, q0 + 1, q1,
+        [&](unsigned p) {
+            const size_t e = p >> 2;
+            return Three<double>{d.vol[e], d.c_mass[e], thermal ? d.c_tmass[e] : 1.0};
+        },
+        [&](const Three<double> &t) {
+            sf::pos_add(sv, t.x);
+            sf::pos_add(sm, t.y);
+            sf::pos_add(st, t.z);
+        });
+    vn = sf::value(sv);
+    m = sf::value(sm);
+    tm = thermal ? sf::value(st) : 0.0;
+    if (!(sf::exact(sv) && sf::exact(sm) && sf::exact(st))) {
+        double r[3];
+        node_masses_exact(d, q0, q1, r);
+        vn = r[0];
+        m = r[1];
+        tm = r[2];
+    }
+}
+
+// N-A: start of a step (dynearthsol.cxx:358-362, 365 node half).  The masses'
+// additions (12 of the pass's 20 per element) and the two divisions are on
+// the integer pipes, the signed sums on the FP64 unit, so that both work:
+// 25 FP64 instructions per element before, at the pipe's measured peak, 9.7 now
+// (2.4M elements: 130 -> 90 us).  4 blocks of 256 per SM (5: 12 % slower, 6:
+// 26 %, for the spills).
+__global__ void __launch_bounds__(256, 4) k_fn_a(Dev d)
 {
     int n = gtid();
     const Consts &K = *d.K;
+    const bool live = n < d.nnode;
+    const int q0 = live ? d.sup_off[n] : 0, q1 = live ? d.sup_off[n + 1] : 0;
     const double dt = d.clk->dt;
     if (n == 0) {
         d.clk->steps += 1;
         d.clk->time += dt;
         d.clk->step_dt = dt;
     }
-    if (n >= d.nnode) return;
+    if (!live) return;
     const size_t E = d.nelem;
-    const int q0 = d.sup_off[n], q1 = d.sup_off[n + 1];
     double vn, tm;
     if (d.clk->mass_valid) {
         vn = d.vol_n[n];
         tm = d.tmass[n];
     } else {
-        double m = 0;
-        vn = 0;
-        tm = 0;
-        for (int q = q0; q < q1; ++q) {
-            size_t e = __ldg(d.sup_ent + q) >> 2;
-            vn += d.vol[e];
-            m += d.c_mass[e];
-            if (K.thermal) tm += d.c_tmass[e];
-        }
+        double m;
+        node_masses(d, q0, q1, vn, m, tm);
         d.vol_n[n] = vn;
         d.mass[n] = m;
         d.tmass[n] = tm;
     }
     if (K.thermal) {
         double tdot = 0;
-        for (int q = q0; q < q1; ++q) {
-            unsigned p = __ldg(d.sup_ent + q);
-            tdot += d.tmp[(p & 3u) * E + (p >> 2)];
-        }
+        walk<4>(
+            d.sup_ent, q0, q1, [&](unsigned p) { return d.tmp[(p & 3u) * E + (p >> 2)]; },
+            [&](double v) { tdot += v; });
         if (d.bcflag[n] & kBoundZ1)
             d.T[n] = K.surface_temperature;
         else
-            d.T[n] -= tdot * dt / tm;
+            d.T[n] -= sf::div(sf::mul(tdot, dt), tm);
     }
     double dv = 0.;
-    for (int q = q0; q < q1; ++q) dv += d.c_trdv[__ldg(d.sup_ent + q) >> 2];
-    dv /= vn;
-    d.ntmp[n] = dv;
+    walk<4>(d.sup_ent, q0, q1, [&](unsigned p) { return d.c_trdv[p >> 2]; }, [&](double v) { dv += v; });
+    d.ntmp[n] = sf::div(dv, vn);
 }
 
 // E-B: edvoldt + update_stress + dp * volume
@@ -1082,13 +1164,13 @@ template <bool LOG, int RHEOL>
 __global__ void __launch_bounds__(128, 8) k_fe_b_t(Dev d, int e0)
 {
     int e = e0 + gtid();
-    if (e == 0) d.clk->mass_valid = 1;
     bool live = e < d.nelem;
+    const int4 c = live ? d.conn[e] : int4{0, 0, 0, 0};
+    if (e == 0) d.clk->mass_valid = 1;
     int flags = 0;
     float rec[kRetRecord];
     if (live) {
         const size_t E = d.nelem;
-        int4 c = d.conn[e];
         double a[4];
         load_nodal4(d.ntmp, c, a);
         double dj = sf::add0(a[0]);            // 0 + a0, then the rest; / 4
@@ -1144,15 +1226,31 @@ __global__ void __launch_bounds__(128, 8) k_fe_b_t(Dev d, int e0)
     }
 }
 
-// N-C: force gather, damping, velocity, velocity BCs, coordinates
+// N-C: force gather, damping, velocity, velocity BCs, coordinates.  Its
+// products and its three divisions by one mass are on the integer pipes (20.6
+// -> 17.0 FP64 instructions per element, at the pipe's peak: 108 -> 91 us for
+// 2.4M elements); its 12 signed additions are not: one on the integer pipes
+// takes about as long as on the FP64 unit.
 __global__ void k_fn_c(Dev d)
 {
     int n = gtid();
     if (n >= d.nnode) return;
     const Consts &K = *d.K;
+    const int q0 = d.sup_off[n], q1 = d.sup_off[n + 1];
     const double dt = d.clk->dt;
-    double f[3];
-    force_gather(d, n, f);
+    double f[3] = {0, 0, 0};
+    const size_t E = d.nelem;
+    walk<4>(
+        d.sup_ent, q0, q1,
+        [&](unsigned p) {
+            const double *t = d.tmp + (size_t)(p & 3u) * E + (p >> 2);
+            return Three<double>{t[0], t[4 * E], t[8 * E]};
+        },
+        [&](const Three<double> &t) {
+            f[0] -= t.x;
+            f[1] -= t.y;
+            f[2] -= t.z;
+        });
     stress_bc_node(K, d.bf, n, d.bcflag[n], d.z[n], d.z0[n], f);
     double v[3] = {d.vx[n], d.vy[n], d.vz[n]};
     if (K.is_qs) {
@@ -1163,13 +1261,22 @@ __global__ void k_fn_c(Dev d)
     d.fx[n] = f[0];
     d.fy[n] = f[1];
     d.fz[n] = f[2];
-    double m = d.mass[n];
-    for (int j = 0; j < 3; ++j) v[j] += dt * f[j] / m;
+    // v += dt f / m: one reciprocal of m on the integer pipes for the three
+    const double m = d.mass[n];
+    uint32_t far = 0;
+    const sf::Den dm = sf::denominator(m, far);
+    for (int j = 0; j < 3; ++j) {
+        const double a = sf::mul(dt, f[j]);
+        uint32_t fa = far;
+        double q = sf::quotient(a, dm, fa);
+        if (!sf::in_range(fa)) q = sf::div_slow(a, m);
+        v[j] += q;
+    }
     vbc_node(K, d.bcflag[n], v);
     d.vx[n] = v[0];
     d.vy[n] = v[1];
     d.vz[n] = v[2];
-    const double x = d.x[n] + v[0] * dt, y = d.y[n] + v[1] * dt, z = d.z[n] + v[2] * dt;
+    const double x = d.x[n] + sf::mul(v[0], dt), y = d.y[n] + sf::mul(v[1], dt), z = d.z[n] + sf::mul(v[2], dt);
     d.x[n] = x;
     d.y[n] = y;
     d.z[n] = z;

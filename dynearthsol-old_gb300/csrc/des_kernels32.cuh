@@ -80,9 +80,9 @@ __device__ __forceinline__ void f_load_vel4(const DevF &d, int4 c, float V[4][3]
     const int n[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        V[i][0] = __ldg(d.vx + n[i]);
-        V[i][1] = __ldg(d.vy + n[i]);
-        V[i][2] = __ldg(d.vz + n[i]);
+        V[i][0] = d.vx[n[i]];
+        V[i][1] = d.vy[n[i]];
+        V[i][2] = d.vz[n[i]];
     }
 }
 __device__ __forceinline__ void f_load_xyz4(const DevF &d, int4 c, double X[4][3])
@@ -90,9 +90,9 @@ __device__ __forceinline__ void f_load_xyz4(const DevF &d, int4 c, double X[4][3
     const int n[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        X[i][0] = __ldg(d.x + n[i]);
-        X[i][1] = __ldg(d.y + n[i]);
-        X[i][2] = __ldg(d.z + n[i]);
+        X[i][0] = d.x[n[i]];
+        X[i][1] = d.y[n[i]];
+        X[i][2] = d.z[n[i]];
     }
 }
 __device__ __forceinline__ void f_load_shp(const DevF &d, int e, float dx[4], float dy[4], float dz[4])
@@ -118,8 +118,8 @@ __device__ __forceinline__ void f_store6(float *a, size_t E, int e, const float 
 // element mean temperature in FP32 (from the FP64 accumulator)
 __device__ __forceinline__ float f_elem_T(const DevF &d, int4 c)
 {
-    return elem_mean4(sf::to_float(__ldg(d.T + c.x)), sf::to_float(__ldg(d.T + c.y)),
-                      sf::to_float(__ldg(d.T + c.z)), sf::to_float(__ldg(d.T + c.w)));
+    return elem_mean4(sf::to_float(d.T[c.x]), sf::to_float(d.T[c.y]),
+                      sf::to_float(d.T[c.z]), sf::to_float(d.T[c.w]));
 }
 
 // matprops.cxx:707-728 in FP32
@@ -327,9 +327,9 @@ __device__ __forceinline__ void f_next_contrib(const DevF &d, int e, int4 c, con
     if (d.F->thermal) {
         // conduction vector kv (grad N_i . grad T) with grad T from temperature
         // differences (sum_j grad N_j = 0), differences taken in FP64
-        double T0 = __ldg(d.T + c.x);
-        float t1 = sf::to_float(__ldg(d.T + c.y) - T0), t2 = sf::to_float(__ldg(d.T + c.z) - T0),
-              t3 = sf::to_float(__ldg(d.T + c.w) - T0);
+        double T0 = d.T[c.x];
+        float t1 = sf::to_float(d.T[c.y] - T0), t2 = sf::to_float(d.T[c.z] - T0),
+              t3 = sf::to_float(d.T[c.w] - T0);
         float gx = dx[1] * t1 + dx[2] * t2 + dx[3] * t3;
         float gy = dy[1] * t1 + dy[2] * t2 + dy[3] * t3;
         float gz = dz[1] * t1 + dz[2] * t2 + dz[3] * t3;
@@ -405,6 +405,8 @@ __global__ void kf_fn_a(DevF d)
 {
     int n = gtid();
     const ConstsF &F = *d.F;
+    const bool live = n < d.nnode;
+    const int q0 = live ? d.sup_off[n] : 0, q1 = live ? d.sup_off[n + 1] : 0;
     const double dt = d.clk->dt;
     if (n == 0) {
         d.clk->steps += 1;
@@ -412,9 +414,8 @@ __global__ void kf_fn_a(DevF d)
         d.clk->npend = 0;
         d.clk->nexact = 0;
     }
-    if (n >= d.nnode) return;
+    if (!live) return;
     const size_t E = d.nelem;
-    const int q0 = d.sup_off[n], q1 = d.sup_off[n + 1];
     float vn, tm;
     if (d.clk->mass_valid) {
         vn = d.vol_n[n];
@@ -423,29 +424,34 @@ __global__ void kf_fn_a(DevF d)
         float m = 0.f;
         vn = 0.f;
         tm = 0.f;
-        for (int q = q0; q < q1; ++q) {
-            size_t e = __ldg(d.sup_ent + q) >> 2;
-            vn += d.c_vol[e];
-            m += d.c_mass[e];
-            if (F.thermal) tm += d.c_tmass[e];
-        }
+        const bool thermal = F.thermal;
+        walk<4>(
+            d.sup_ent, q0, q1,
+            [&](unsigned p) {
+                const size_t e = p >> 2;
+                return Three<float>{d.c_vol[e], d.c_mass[e], thermal ? d.c_tmass[e] : 0.f};
+            },
+            [&](const Three<float> &t) {
+                vn += t.x;
+                m += t.y;
+                if (thermal) tm += t.z;
+            });
         d.vol_n[n] = vn;
         d.mass[n] = m;
         d.tmass[n] = tm;
     }
     if (F.thermal) {
         float tdot = 0.f;
-        for (int q = q0; q < q1; ++q) {
-            unsigned p = __ldg(d.sup_ent + q);
-            tdot += d.tmp[(p & 3u) * E + (p >> 2)];
-        }
+        walk<4>(
+            d.sup_ent, q0, q1, [&](unsigned p) { return d.tmp[(p & 3u) * E + (p >> 2)]; },
+            [&](float v) { tdot += v; });
         if (d.bcflag[n] & kBoundZ1)
             d.T[n] = d.K->surface_temperature;
         else
-            d.T[n] -= (double)tdot * dt / (double)tm;
+            d.T[n] -= sf::div(sf::mul(sf::widen(tdot), dt), sf::widen(tm));
     }
     float dv = 0.f;
-    for (int q = q0; q < q1; ++q) dv += d.c_trdv[__ldg(d.sup_ent + q) >> 2];
+    walk<4>(d.sup_ent, q0, q1, [&](unsigned p) { return d.c_trdv[p >> 2]; }, [&](float v) { dv += v; });
     d.ntmp[n] = dv / vn;
 }
 
@@ -542,8 +548,10 @@ __global__ void kf_sg_gather(DevF d)
 {
     int n = gtid();
     if (n >= d.nnode) return;
+    const int q0 = d.sup_off[n], q1 = d.sup_off[n + 1];
     float s = 0.f;
-    for (int q = d.sup_off[n]; q < d.sup_off[n + 1]; ++q) s += d.tmp_sg[__ldg(d.sup_ent + q) >> 2];
+    walk<4>(d.sup_ent, q0, q1, [&](unsigned p) { return d.tmp_sg[p >> 2]; },
+            [&](float v) { s += v; });
     d.ntmp[n] = s / d.vol_n[n];
 }
 
@@ -586,33 +594,41 @@ __global__ void kf_fn_c(DevF d)
     if (n >= d.nnode) return;
     const size_t E = d.nelem;
     const Consts &K = *d.K;
+    const int q0 = d.sup_off[n], q1 = d.sup_off[n + 1];
     const double dt = d.clk->dt;
-    const float dtf = (float)dt;
+    const float dtf = sf::to_float(dt);
     float g[3] = {0.f, 0.f, 0.f};
     double h[3] = {0.0, 0.0, 0.0};
     // the FP64 reference part and the FP32 part in two walks over the
     // support list, each streaming its own arrays (one walk over both:
     // 282 against 194 B per element read from DRAM, 0.46 against 0.35 ms
     // on config 2)
-    const int q0 = d.sup_off[n], q1 = d.sup_off[n + 1];
-    for (int q = q0; q < q1; ++q) {
-        unsigned p = __ldg(d.sup_ent + q);
-        size_t e = p >> 2, i = p & 3u;
-        h[0] -= d.f0[(i)*E + e];
-        h[1] -= d.f0[(i + 4) * E + e];
-        h[2] -= d.f0[(i + 8) * E + e];
-    }
-    for (int q = q0; q < q1; ++q) {
-        unsigned p = __ldg(d.sup_ent + q);
-        size_t e = p >> 2, i = p & 3u;
-        g[0] -= d.tmp[(i)*E + e];
-        g[1] -= d.tmp[(i + 4) * E + e];
-        g[2] -= d.tmp[(i + 8) * E + e];
-    }
+    walk<4>(
+        d.sup_ent, q0, q1,
+        [&](unsigned p) {
+            const double *t = d.f0 + (size_t)(p & 3u) * E + (p >> 2);
+            return Three<double>{t[0], t[4 * E], t[8 * E]};
+        },
+        [&](const Three<double> &t) {
+            h[0] -= t.x;
+            h[1] -= t.y;
+            h[2] -= t.z;
+        });
+    walk<4>(
+        d.sup_ent, q0, q1,
+        [&](unsigned p) {
+            const float *t = d.tmp + (size_t)(p & 3u) * E + (p >> 2);
+            return Three<float>{t[0], t[4 * E], t[8 * E]};
+        },
+        [&](const Three<float> &t) {
+            g[0] -= t.x;
+            g[1] -= t.y;
+            g[2] -= t.z;
+        });
     // the boundary tractions balance the FP64 reference part: FP64 as well
     stress_bc_node(K, d.bf, n, d.bcflag[n], d.z[n], d.z0[n], h);
-    float f[3] = {(float)(h[0] + (double)g[0]), (float)(h[1] + (double)g[1]),
-                  (float)(h[2] + (double)g[2])};
+    float f[3];
+    for (int j = 0; j < 3; ++j) f[j] = sf::to_float(h[j] + sf::widen(g[j]));
     float v[3] = {d.vx[n], d.vy[n], d.vz[n]};
     if (d.F->is_qs) {
         f[0] = damp(K, f[0], v[0]);
@@ -628,8 +644,8 @@ __global__ void kf_fn_c(DevF d)
     d.vx[n] = v[0];
     d.vy[n] = v[1];
     d.vz[n] = v[2];
-    const double x = d.x[n] + (double)v[0] * dt, y = d.y[n] + (double)v[1] * dt,
-                 z = d.z[n] + (double)v[2] * dt;
+    const double x = d.x[n] + sf::mul(sf::widen(v[0]), dt), y = d.y[n] + sf::mul(sf::widen(v[1]), dt),
+                 z = d.z[n] + sf::mul(sf::widen(v[2]), dt);
     d.x[n] = x;
     d.y[n] = y;
     d.z[n] = z;
@@ -675,13 +691,13 @@ __global__ void __launch_bounds__(128, 9) kf_fe_a(DevF d, int e0, unsigned nbloc
     int e = e0 + gtid();
     const Consts &K = *d.K;
     const ConstsF &F = *d.F;
+    bool live = e < d.nelem;
+    const int4 c = live ? d.conn[e] : int4{0, 0, 0, 0};
     const bool dt_step = (K.fixed_dt == 0) && (d.clk->steps % 10 == 0);
     if (e == 0) d.clk->mass_valid = 0;
-    bool live = e < d.nelem;
     double minh = 0;
     if (live) {
         const size_t E = d.nelem;
-        int4 c = d.conn[e];
         float dx[4], dy[4], dz[4];
         double c2max = 0;
         double vol = f_geometry(d, e, c, dx, dy, dz, dt_step ? &c2max : nullptr);
@@ -701,7 +717,7 @@ __global__ void __launch_bounds__(128, 9) kf_fe_a(DevF d, int e0, unsigned nbloc
         if (F.rheol & 1) {
             float w3, w4, w5, s[6];
             spin(V, dx, dy, dz, w3, w4, w5);
-            const float dt = (float)d.clk->dt;
+            const float dt = sf::to_float(d.clk->dt);
             f_load6(d.stress, E, e, s);
             jaumann(s, dt, w3, w4, w5);
             f_store6(d.stress, E, e, s);
@@ -808,7 +824,7 @@ __global__ void kf_init_stress(DevF d)
     const Consts &K = *d.K;
     const double ks = K.M.mix[d.mix[K.ref_pressure_option != 0 ? e : 0]].bulkm;
     int4 c = d.conn[e];
-    double zc = elem_mean4(__ldg(d.z + c.x), __ldg(d.z + c.y), __ldg(d.z + c.z), __ldg(d.z + c.w));
+    double zc = elem_mean4(d.z[c.x], d.z[c.y], d.z[c.z], d.z[c.w]);
     double p = ref_pressure(K.ref_pressure_option, K.rho0_0, K.gravity, zc);
     d.s0[e] = -p;
     for (int i = 0; i < 3; ++i) {

@@ -1,5 +1,6 @@
 // Host check of the grouped integer-pipe product (unpack, prod, in_range), the
-// quotient (div) of dynearthsol-old_gb300/csrc/des_softf64.cuh against the
+// quotient (div), the running
+// sum of positive numbers (PosSum) and the FP32 -> FP64 conversion (widen) of dynearthsol-old_gb300/csrc/des_softf64.cuh against the
 // host's IEEE arithmetic, bit for bit.
 //   softf64_ops_check <pairs per kind>  -> one line per kind; exit 1 on a mismatch
 #include "des_softf64.cuh"
@@ -78,5 +79,42 @@ int main(int argc, char **argv)
         printf("kind %d: %lld pairs, %lld mismatches\n", kind, per, bad);
         total += bad;
     }
+    // sums of 1-30 terms whose exponents spread over 1, 4 or 14 binades; now and
+    // then a zero, a negative, an infinite or a subnormal term among them
+    const int spread[3] = {1, 4, 14};
+    for (int kind = 0; kind < 3; ++kind) {
+        uint64_t s = 0x5005000ull + kind;
+        long long bad = 0, sums = 0;
+        for (long long i = 0; i < per / 4; ++i) {
+            const int n = 1 + (int)(splitmix(s) % 30), odd = i % 50 == 0 ? (int)(splitmix(s) % n) : -1;
+            const uint64_t base = 200 + splitmix(s) % 1500;
+            PosSum p = pos_first(1.0);
+            volatile double h = 0;
+            for (int j = 0; j < n; ++j) {
+                double x = std::fabs(mk(s, base + splitmix(s) % spread[kind]));
+                if (j == odd) x = i % 200 == 0 ? 0.0 : i % 200 == 50 ? -x : i % 200 == 100 ? INFINITY : 5e-324;
+                h = h + x;
+                if (j)
+                    pos_add(p, x);
+                else
+                    p = pos_first(x);
+            }
+            if (exact(p)) {
+                ++sums;
+                bad += bits(h) != bits(value(p));
+            }
+        }
+        // terms of one binade always stay within the sum's reach, unless one is odd
+        if (kind == 0 && sums < per / 4 * 97 / 100) ++bad;
+        printf("sums %d: %lld, %lld mismatches\n", kind, sums, bad);
+        total += bad;
+    }
+    long long bad = 0;
+    for (uint64_t i = 0; i < (1ull << 32); i += 257) {
+        const float f = float_from_bits((uint32_t)i);
+        bad += !same((double)f, widen(f));
+    }
+    printf("widen: %lld mismatches\n", bad);
+    total += bad;
     return total ? 1 : 0;
 }
