@@ -342,30 +342,63 @@ __device__ __forceinline__ void f_next_contrib(const DevF &d, int e, int4 c, con
 // products c_i = 6 V grad(N_i) (the cofactors; c_0 = -(c_1 + c_2 + c_3)) and
 // the volume det / 6, the same quantities compute_volume (geometry.cxx:29-49)
 // and compute_shape_fn (geometry.cxx:388-470) form, grouped so that the
-// volume and the four gradients share one set of products.
-__device__ __forceinline__ double f_cofactors(const double X[4][3], double cf[4][3])
+// volume and the four gradients share one set of products.  (Fused
+// multiply-adds: this form is held to a tolerance, not to the reference's
+// rounding.)
+__device__ __forceinline__ void f_edges(const double X[4][3], double a[3], double b[3], double q[3])
 {
-    double a[3], b[3], q[3];
     for (int k = 0; k < 3; ++k) {
         a[k] = X[1][k] - X[0][k];
         b[k] = X[2][k] - X[0][k];
         q[k] = X[3][k] - X[0][k];
     }
-    // (fused multiply-adds: this form is held to a tolerance, not to the
-    // reference's rounding)
-    // (the plain products on the integer pipes, sf::mul, rounded as the FP64
-    // unit rounds them)
-    cf[1][0] = fma(b[1], q[2], -sf::mul(b[2], q[1]));
-    cf[1][1] = fma(b[2], q[0], -sf::mul(b[0], q[2]));
-    cf[1][2] = fma(b[0], q[1], -sf::mul(b[1], q[0]));
-    cf[2][0] = fma(q[1], a[2], -sf::mul(q[2], a[1]));
-    cf[2][1] = fma(q[2], a[0], -sf::mul(q[0], a[2]));
-    cf[2][2] = fma(q[0], a[1], -sf::mul(q[1], a[0]));
-    cf[3][0] = fma(a[1], b[2], -sf::mul(a[2], b[1]));
-    cf[3][1] = fma(a[2], b[0], -sf::mul(a[0], b[2]));
-    cf[3][2] = fma(a[0], b[1], -sf::mul(a[1], b[0]));
-    for (int k = 0; k < 3; ++k) cf[0][k] = -(cf[1][k] + cf[2][k] + cf[3][k]);
-    return fma(a[0], cf[1][0], fma(a[1], cf[1][1], sf::mul(a[2], cf[1][2])));     // 6 V
+}
+
+// on the FP64 unit, out of line: for edges outside sf::unpack's range
+static __device__ __noinline__ double f_cofactors_exact(const DevF &d, int4 c, double out[12])
+{
+    double X[4][3], a[3], b[3], q[3];
+    f_load_xyz4(d, c, X);
+    f_edges(X, a, b, q);
+    for (int k = 0; k < 3; ++k) {
+        const int i = (k + 1) % 3, j = (k + 2) % 3;
+        out[3 + k] = fma(b[i], q[j], -(b[j] * q[i]));
+        out[6 + k] = fma(q[i], a[j], -(q[j] * a[i]));
+        out[9 + k] = fma(a[i], b[j], -(a[j] * b[i]));
+        out[k] = -(out[3 + k] + out[6 + k] + out[9 + k]);
+    }
+    return fma(a[0], out[3], fma(a[1], out[4], a[2] * out[5]));
+}
+
+__device__ __forceinline__ double f_cofactors(const DevF &d, int4 c, const double X[4][3], double cf[4][3])
+{
+    double a[3], b[3], q[3];
+    f_edges(X, a, b, q);
+    // (the plain products on the integer pipes)
+    uint32_t far = 0;
+    sf::Op oa[3], ob[3], oq[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        oa[k] = sf::unpack(a[k], far);
+        ob[k] = sf::unpack(b[k], far);
+        oq[k] = sf::unpack(q[k], far);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int i = (k + 1) % 3, j = (k + 2) % 3;
+        cf[1][k] = fma(b[i], q[j], -sf::prod(ob[j], oq[i]));
+        cf[2][k] = fma(q[i], a[j], -sf::prod(oq[j], oa[i]));
+        cf[3][k] = fma(a[i], b[j], -sf::prod(oa[j], ob[i]));
+        cf[0][k] = -(cf[1][k] + cf[2][k] + cf[3][k]);
+    }
+    double det = fma(a[0], cf[1][0], fma(a[1], cf[1][1], sf::prod(oa[2], sf::unpack(cf[1][2], far))));     // 6 V
+    if (!sf::in_range(far)) {
+        double r[12];
+        det = f_cofactors_exact(d, c, r);
+#pragma unroll
+        for (int k = 0; k < 12; ++k) cf[k / 3][k % 3] = r[k];
+    }
+    return det;
 }
 
 // FP64 part of the element force vectors for the next step: s0 grad(N_i) V
@@ -376,10 +409,19 @@ __device__ __forceinline__ void f_reference_force(const DevF &d, int e, const do
     const size_t E = d.nelem;
     const double s6 = sf::mul(d.s0[e], 1.0 / 6.0);
     const double buoy = d.F->gravity != 0.f ? sf::mul(d.F->mix[d.mix[e]].rho_g4, vol) : 0.0;
+    // (the plain products on the integer pipes)
+    uint32_t far = 0;
+    const sf::Op o6 = sf::unpack(s6, far);
     for (int i = 0; i < 4; ++i) {
-        d.f0[(i)*E + e] = s6 * cf[i][0];
-        d.f0[(i + 4) * E + e] = s6 * cf[i][1];
+        d.f0[(i)*E + e] = sf::prod(o6, sf::unpack(cf[i][0], far));
+        d.f0[(i + 4) * E + e] = sf::prod(o6, sf::unpack(cf[i][1], far));
         d.f0[(i + 8) * E + e] = fma(s6, cf[i][2], buoy);
+    }
+    if (!sf::in_range(far)) {
+        for (int i = 0; i < 4; ++i) {
+            d.f0[(i)*E + e] = sf::from_bits(sf::mul_slow(sf::bits(s6), sf::bits(cf[i][0])));
+            d.f0[(i + 4) * E + e] = sf::from_bits(sf::mul_slow(sf::bits(s6), sf::bits(cf[i][1])));
+        }
     }
 }
 
@@ -394,7 +436,7 @@ __global__ void kf_prime(DevF d)
     {
         double X[4][3], cf[4][3];
         f_load_xyz4(d, c, X);
-        f_cofactors(X, cf);
+        f_cofactors(d, c, X, cf);
         f_reference_force(d, e, cf, d.vol[e]);
     }
     f_next_contrib(d, e, c, V, dx, dy, dz, (float)d.vol[e]);
@@ -662,7 +704,7 @@ __device__ __forceinline__ double f_geometry(const DevF &d, int e, int4 c, float
     double X[4][3];
     f_load_xyz4(d, c, X);
     double cf[4][3];
-    const double det = f_cofactors(X, cf);
+    const double det = f_cofactors(d, c, X, cf);
     const double vol = sf::mul(det, 1.0 / 6.0);
     f_reference_force(d, e, cf, vol);
     if (c2max) {
@@ -684,8 +726,11 @@ __device__ __forceinline__ double f_geometry(const DevF &d, int e, int4 c, float
 }
 
 // E-A, over the elements from e0 (a multiple of the block size); the pass
-// has nblocks blocks in all.  Registers bounded for 9 blocks of 128 per SM
-// (1.07 -> 1.01 ms on config 2).
+// has nblocks blocks in all.  The FP64 pipe bounds it: 37 FP64 instructions per
+// element with the plain products (the cofactors', the volume's, the reference
+// force's) on the integer pipes, checked together (45 with a check for
+// each, and more instructions: 400 -> 353 us for 3.84M elements).  Registers
+// bounded for 9 blocks of 128 per SM (8: 359 us, 10: 361).
 __global__ void __launch_bounds__(128, 9) kf_fe_a(DevF d, int e0, unsigned nblocks)
 {
     int e = e0 + gtid();
