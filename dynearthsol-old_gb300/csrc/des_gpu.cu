@@ -23,6 +23,7 @@ namespace {
 const int kElemBlock = 128;
 const int kNodeBlock = 256;
 const int kStepKernels = 6;
+const int kGraphSteps = 10;  // steps of the larger captured graph
 const int kEaChunks = 8;   // E-A launches of the host-buffer step (downloads overlap them)
 const int kEbChunks = 8;   // E-B launches of the host-buffer step (its inputs come up chunk by chunk)
 
@@ -45,7 +46,8 @@ struct des_gpu {
     long long bytes = 0;
     double *staging = nullptr;
     long long staging_elems = 0;
-    cudaGraphExec_t graph = nullptr;
+    cudaGraphExec_t graph = nullptr;      // one step
+    cudaGraphExec_t graph_many = nullptr; // kGraphSteps steps
     bool primed = false;
     int prec = DES_PREC_FP64;
     DevF f;
@@ -545,23 +547,22 @@ void launch_surface(des_gpu *g)
 // the first kernel of pass E-B over the element blocks [b0, b1)
 void launch_eb_first(des_gpu *g, int b0, int b1)
 {
-    cudaStream_t st = g->stream;
     const int n = b1 - b0, e0 = b0 * kElemBlock;
     if (g->prec == DES_PREC_FP32) {
         if (g->hF.rheol == 7)
-            kf_fe_b_ep<7><<<n, kElemBlock, 0, st>>>(g->f, e0);
+            kf_fe_b_ep<7><<<n, kElemBlock, 0, g->stream>>>(g->f, e0);
         else if (g->hF.rheol == 5)
-            kf_fe_b_ep<5><<<n, kElemBlock, 0, st>>>(g->f, e0);
+            kf_fe_b_ep<5><<<n, kElemBlock, 0, g->stream>>>(g->f, e0);
         else
-            kf_fe_b<<<n, kElemBlock, 0, st>>>(g->f, e0);
+            kf_fe_b<<<n, kElemBlock, 0, g->stream>>>(g->f, e0);
     } else if (g->d.ret_log) {
-        k_fe_b_t<true, 0><<<n, kElemBlock, 0, st>>>(g->d, e0);
+        k_fe_b_t<true, 0><<<n, kElemBlock, 0, g->stream>>>(g->d, e0);
     } else if (g->hK.rheol == 7) {
-        k_fe_b_t<false, 7><<<n, kElemBlock, 0, st>>>(g->d, e0);
+        k_fe_b_t<false, 7><<<n, kElemBlock, 0, g->stream>>>(g->d, e0);
     } else if (g->hK.rheol == 5) {
-        k_fe_b_t<false, 5><<<n, kElemBlock, 0, st>>>(g->d, e0);
+        k_fe_b_t<false, 5><<<n, kElemBlock, 0, g->stream>>>(g->d, e0);
     } else {
-        k_fe_b_t<false, 0><<<n, kElemBlock, 0, st>>>(g->d, e0);
+        k_fe_b_t<false, 0><<<n, kElemBlock, 0, g->stream>>>(g->d, e0);
     }
 }
 
@@ -571,15 +572,14 @@ void launch_eb_first(des_gpu *g, int b0, int b1)
 void launch_eb_rest(des_gpu *g)
 {
     if (g->prec != DES_PREC_FP32 || (g->hF.rheol != 5 && g->hF.rheol != 7)) return;
-    cudaStream_t st = g->stream;
     const DevF &f = g->f;
     const int nn_grid = 4 * g->sms, exact_grid = 8 * g->sms;
     if (g->hF.rheol == 7) {
-        if (g->closure) kf_nn_list<7><<<nn_grid, kNnListBlock, sizeof(NnListSmem), st>>>(f, g->dnet);
-        kf_exact_list<7><<<exact_grid, 128, 0, st>>>(f, g->closure ? 0 : 1);
+        if (g->closure) kf_nn_list<7><<<nn_grid, kNnListBlock, sizeof(NnListSmem), g->stream>>>(f, g->dnet);
+        kf_exact_list<7><<<exact_grid, 128, 0, g->stream>>>(f, g->closure ? 0 : 1);
     } else {
-        if (g->closure) kf_nn_list<5><<<nn_grid, kNnListBlock, sizeof(NnListSmem), st>>>(f, g->dnet);
-        kf_exact_list<5><<<exact_grid, 128, 0, st>>>(f, g->closure ? 0 : 1);
+        if (g->closure) kf_nn_list<5><<<nn_grid, kNnListBlock, sizeof(NnListSmem), g->stream>>>(f, g->dnet);
+        kf_exact_list<5><<<exact_grid, 128, 0, g->stream>>>(f, g->closure ? 0 : 1);
     }
 }
 
@@ -587,7 +587,6 @@ void launch_eb_rest(des_gpu *g)
 void launch_pass(des_gpu *g, int k)
 {
     const int nb = blocks(g->nnode, kNodeBlock), eb = blocks(g->nelem, kElemBlock);
-    cudaStream_t st = g->stream;
     if (k == 1) {
         launch_eb_first(g, 0, eb);
         launch_eb_rest(g);
@@ -596,26 +595,26 @@ void launch_pass(des_gpu *g, int k)
     if (g->prec == DES_PREC_FP32) {
         const DevF &f = g->f;
         switch (k) {
-        case 0: kf_fn_a<<<nb, kNodeBlock, 0, st>>>(f); break;
-        case 2: kf_sg_gather<<<nb, kNodeBlock, 0, st>>>(f); break;
-        case 3: kf_fe_c<<<eb, kElemBlock, 0, st>>>(f); break;
+        case 0: kf_fn_a<<<nb, kNodeBlock, 0, g->stream>>>(f); break;
+        case 2: kf_sg_gather<<<nb, kNodeBlock, 0, g->stream>>>(f); break;
+        case 3: kf_fe_c<<<eb, kElemBlock, 0, g->stream>>>(f); break;
         default:
             if (g->hK.stress_bc_sides && g->d.bf.nbf > 0)
-                k_stress_bc_facets<<<blocks(g->d.bf.nbf, 128), 128, 0, st>>>(g->d);
-            kf_fn_c<<<nb, kNodeBlock, 0, st>>>(f);
+                k_stress_bc_facets<<<blocks(g->d.bf.nbf, 128), 128, 0, g->stream>>>(g->d);
+            kf_fn_c<<<nb, kNodeBlock, 0, g->stream>>>(f);
             launch_surface(g);
             break;
         }
     } else {
         const Dev &d = g->d;
         switch (k) {
-        case 0: k_fn_a<<<nb, kNodeBlock, 0, st>>>(d); break;
-        case 2: k_sg_gather<<<nb, kNodeBlock, 0, st>>>(d); break;
-        case 3: k_fe_c<true, 128, 12><<<eb, kElemBlock, 0, st>>>(d); break;
+        case 0: k_fn_a<<<nb, kNodeBlock, 0, g->stream>>>(d); break;
+        case 2: k_sg_gather<<<nb, kNodeBlock, 0, g->stream>>>(d); break;
+        case 3: k_fe_c<true, 128, 12><<<eb, kElemBlock, 0, g->stream>>>(d); break;
         default:
             if (g->hK.stress_bc_sides && d.bf.nbf > 0)
-                k_stress_bc_facets<<<blocks(d.bf.nbf, 128), 128, 0, st>>>(d);
-            k_fn_c<<<nb, kNodeBlock, 0, st>>>(d);
+                k_stress_bc_facets<<<blocks(d.bf.nbf, 128), 128, 0, g->stream>>>(d);
+            k_fn_c<<<nb, kNodeBlock, 0, g->stream>>>(d);
             launch_surface(g);
             break;
         }
@@ -727,16 +726,43 @@ int ensure_download_buffer(des_gpu *g, long long n)
     return DES_OK;
 }
 
-int capture_step_graph(des_gpu *g)
+int capture_steps(des_gpu *g, int nsteps, cudaGraphExec_t *out)
 {
     cudaGraph_t graph;
     DES_CUDA(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
-    launch_step(g, nullptr);
+    for (int i = 0; i < nsteps; ++i) launch_step(g, nullptr);
     cudaError_t e = cudaStreamEndCapture(g->stream, &graph);
     if (e != cudaSuccess) return DES_ERR_CUDA;
-    e = cudaGraphInstantiate(&g->graph, graph, 0);
+    e = cudaGraphInstantiate(out, graph, 0);
     cudaGraphDestroy(graph);
     return cuda_rc(e);
+}
+
+// the captured steps are rebuilt at the next call
+void drop_graphs(des_gpu *g)
+{
+    if (g->graph) cudaGraphExecDestroy(g->graph);
+    if (g->graph_many) cudaGraphExecDestroy(g->graph_many);
+    g->graph = g->graph_many = nullptr;
+}
+
+// the graphs that a call for nsteps launches: the one of kGraphSteps steps is
+// built for a call that uses it often enough to pay for its instantiation
+int ensure_graphs(des_gpu *g, int nsteps)
+{
+    int rc = DES_OK;
+    if (!g->graph_many && nsteps >= 4 * kGraphSteps) rc = capture_steps(g, kGraphSteps, &g->graph_many);
+    if (!rc && !g->graph && (!g->graph_many || nsteps % kGraphSteps)) rc = capture_steps(g, 1, &g->graph);
+    return rc;
+}
+
+int launch_graphs(des_gpu *g, int nsteps)
+{
+    int i = 0;
+    if (g->graph_many)
+        for (; i + kGraphSteps <= nsteps; i += kGraphSteps) DES_CUDA(cudaGraphLaunch(g->graph_many, g->stream));
+    for (; i < nsteps; ++i) DES_CUDA(cudaGraphLaunch(g->graph, g->stream));
+    return DES_OK;
 }
 
 __device__ __forceinline__ unsigned long long check_mix(unsigned long long z)
@@ -1090,7 +1116,7 @@ int des_gpu_destroy(des_gpu *g)
     if (g->up_done) cudaEventDestroy(g->up_done);
     if (g->snap_done) cudaEventDestroy(g->snap_done);
     if (g->stream) cudaStreamSynchronize(g->stream);
-    if (g->graph) cudaGraphExecDestroy(g->graph);
+    drop_graphs(g);
     for (void *p : g->allocs) cudaFree(p);
     if (g->stream) cudaStreamDestroy(g->stream);
     delete g;
@@ -1109,8 +1135,7 @@ int des_gpu_set_params(des_gpu *g, const des_params *p)
     if (rc) return rc;
     // the captured step depends on the rheology (closure) and on whether
     // boundary tractions apply
-    if (g->graph) cudaGraphExecDestroy(g->graph);
-    g->graph = nullptr;
+    drop_graphs(g);
     if (g->closure && g->hF.rheol != 5 && g->hF.rheol != 7) g->closure = false;
     return DES_OK;
 }
@@ -1622,8 +1647,7 @@ int des_gpu_set_averaging(des_gpu *g, int interval)
             (rc = dev_alloc(g, &g->avg_time0, 1)))
             return rc;
     }
-    if (g->graph) cudaGraphExecDestroy(g->graph);
-    g->graph = nullptr;
+    drop_graphs(g);
     g->avg_interval = interval;
     return DES_OK;
 }
@@ -1646,8 +1670,7 @@ int des_gpu_download_averages(des_gpu *g, double *coord0, double *strain0, doubl
 int des_gpu_set_closure(des_gpu *g, const des_mlp *net)
 {
     if (!g) return DES_ERR_ARG;
-    if (g->graph) cudaGraphExecDestroy(g->graph);
-    g->graph = nullptr;
+    drop_graphs(g);
     if (!net) {
         g->closure = false;
         return DES_OK;
@@ -1723,11 +1746,8 @@ int des_gpu_step(des_gpu *g, int nsteps, des_step_report *report)
 {
     if (!g || nsteps < 0) return DES_ERR_ARG;
     if (int rc = prime(g)) return rc;
-    if (!g->graph) {
-        int rc = capture_step_graph(g);
-        if (rc) return rc;
-    }
-    for (int i = 0; i < nsteps; ++i) DES_CUDA(cudaGraphLaunch(g->graph, g->stream));
+    if (int rc = ensure_graphs(g, nsteps)) return rc;
+    if (int rc = launch_graphs(g, nsteps)) return rc;
     if (!report) return DES_OK;
     int rc = des_gpu_report(g, report);
     if (rc) return rc;
@@ -1741,16 +1761,13 @@ int des_gpu_time_steps(des_gpu *g, int nsteps, double *ms)
 {
     if (!g || nsteps < 0 || !ms) return DES_ERR_ARG;
     if (int rc = prime(g)) return rc;
-    if (!g->graph) {
-        int rc = capture_step_graph(g);
-        if (rc) return rc;
-    }
+    if (int rc = ensure_graphs(g, nsteps)) return rc;
     cudaEvent_t a, b;
     DES_CUDA(cudaEventCreate(&a));
     DES_CUDA(cudaEventCreate(&b));
     DES_CUDA(cudaStreamSynchronize(g->stream));
     DES_CUDA(cudaEventRecord(a, g->stream));
-    for (int i = 0; i < nsteps; ++i) DES_CUDA(cudaGraphLaunch(g->graph, g->stream));
+    if (int rc = launch_graphs(g, nsteps)) return rc;
     DES_CUDA(cudaEventRecord(b, g->stream));
     DES_CUDA(cudaEventSynchronize(b));
     float f = 0;
