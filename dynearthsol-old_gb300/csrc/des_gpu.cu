@@ -13,6 +13,7 @@
 #include "des_gpu.h"
 #include "des_closure.cuh"
 #include "des_elem.cuh"
+#include "des_small.cuh"
 #include "des_support.cuh"
 #include "des_topology.h"
 
@@ -544,6 +545,23 @@ void launch_surface(des_gpu *g)
     k_surface_nodes<<<blocks(g->nnode, kNodeBlock), kNodeBlock, 0, g->stream>>>(g->d);
 }
 
+// Where the kernels of des_small.cuh run: up to so many nodes (elements) per
+// multiprocessor, the crossing points measured on boxes of 144 to 396k elements
+// (us, lanes shared / one thread each).  FP64: N-A 10.7 / 18.5 at 2.2k nodes,
+// 14.9 / 19.3 at 10.6k, 19.1 / 19.2 at 21.9k; N-B 7.9 / 8.2, 10.3 / 8.4; N-C
+// 10.3 / 16.3, 14.3 / 16.4, 20.5 / 17.4.  FP32: N-A 9.3 / 14.2 at 5.6k, 12.8 /
+// 14.1 at 21.9k, 19.8 / 17.1 at 48k; N-B 5.8 / 8.2, 6.5 / 8.1, 8.2 / 8.4; N-C
+// 12.3 / 18.4, 20.5 / 18.4.  E-A 15.6 / 31.3 at 9.6k elements, 28.1 / 35.8 at
+// 27.6k, 46.2 / 42.2 at 54k; E-C 8.2 / 10.3, 12.3 / 12.3, 16.4 / 13.9.
+const int kOctetNodes[2][3] = {{128, 32, 90}, {200, 300, 96}};   // [FP64, FP32][N-A, N-B, N-C]
+const int kQuadElemsEa = 280, kQuadElemsEc = 180;
+bool octets(const des_gpu *g, int pass)
+{
+    return g->nnode <= kOctetNodes[g->prec == DES_PREC_FP32][pass] * g->sms;
+}
+bool quads_ea(const des_gpu *g) { return g->nelem <= kQuadElemsEa * g->sms; }
+bool quads_ec(const des_gpu *g) { return g->nelem <= kQuadElemsEc * g->sms; }
+
 // the first kernel of pass E-B over the element blocks [b0, b1)
 void launch_eb_first(des_gpu *g, int b0, int b1)
 {
@@ -573,7 +591,7 @@ void launch_eb_rest(des_gpu *g)
 {
     if (g->prec != DES_PREC_FP32 || (g->hF.rheol != 5 && g->hF.rheol != 7)) return;
     const DevF &f = g->f;
-    const int nn_grid = 4 * g->sms, exact_grid = 8 * g->sms;
+    const int nn_grid = 4 * g->sms, exact_grid = std::min(8 * g->sms, blocks(g->nelem, 128));
     if (g->hF.rheol == 7) {
         if (g->closure) kf_nn_list<7><<<nn_grid, kNnListBlock, sizeof(NnListSmem), g->stream>>>(f, g->dnet);
         kf_exact_list<7><<<exact_grid, 128, 0, g->stream>>>(f, g->closure ? 0 : 1);
@@ -587,6 +605,7 @@ void launch_eb_rest(des_gpu *g)
 void launch_pass(des_gpu *g, int k)
 {
     const int nb = blocks(g->nnode, kNodeBlock), eb = blocks(g->nelem, kElemBlock);
+    const int ob = blocks((long long)kNodeLanes * g->nnode, kSmallBlock);
     if (k == 1) {
         launch_eb_first(g, 0, eb);
         launch_eb_rest(g);
@@ -595,26 +614,57 @@ void launch_pass(des_gpu *g, int k)
     if (g->prec == DES_PREC_FP32) {
         const DevF &f = g->f;
         switch (k) {
-        case 0: kf_fn_a<<<nb, kNodeBlock, 0, g->stream>>>(f); break;
-        case 2: kf_sg_gather<<<nb, kNodeBlock, 0, g->stream>>>(f); break;
+        case 0:
+            if (octets(g, 0))
+                kf_fn_a_small<<<ob, kSmallBlock, 0, g->stream>>>(f);
+            else
+                kf_fn_a<<<nb, kNodeBlock, 0, g->stream>>>(f);
+            break;
+        case 2:
+            if (octets(g, 1))
+                kf_sg_gather_small<<<ob, kSmallBlock, 0, g->stream>>>(f);
+            else
+                kf_sg_gather<<<nb, kNodeBlock, 0, g->stream>>>(f);
+            break;
         case 3: kf_fe_c<<<eb, kElemBlock, 0, g->stream>>>(f); break;
         default:
             if (g->hK.stress_bc_sides && g->d.bf.nbf > 0)
                 k_stress_bc_facets<<<blocks(g->d.bf.nbf, 128), 128, 0, g->stream>>>(g->d);
-            kf_fn_c<<<nb, kNodeBlock, 0, g->stream>>>(f);
+            if (octets(g, 2))
+                kf_fn_c_small<<<ob, kSmallBlock, 0, g->stream>>>(f);
+            else
+                kf_fn_c<<<nb, kNodeBlock, 0, g->stream>>>(f);
             launch_surface(g);
             break;
         }
     } else {
         const Dev &d = g->d;
         switch (k) {
-        case 0: k_fn_a<<<nb, kNodeBlock, 0, g->stream>>>(d); break;
-        case 2: k_sg_gather<<<nb, kNodeBlock, 0, g->stream>>>(d); break;
-        case 3: k_fe_c<true, 128, 12><<<eb, kElemBlock, 0, g->stream>>>(d); break;
+        case 0:
+            if (octets(g, 0))
+                k_fn_a_small<<<ob, kSmallBlock, 0, g->stream>>>(d);
+            else
+                k_fn_a<<<nb, kNodeBlock, 0, g->stream>>>(d);
+            break;
+        case 2:
+            if (octets(g, 1))
+                k_sg_gather_small<<<ob, kSmallBlock, 0, g->stream>>>(d);
+            else
+                k_sg_gather<<<nb, kNodeBlock, 0, g->stream>>>(d);
+            break;
+        case 3:
+            if (quads_ec(g))
+                k_fe_c_quad<<<blocks(4LL * g->nelem, kSmallBlock), kSmallBlock, 0, g->stream>>>(d);
+            else
+                k_fe_c<true, 128, 12><<<eb, kElemBlock, 0, g->stream>>>(d);
+            break;
         default:
             if (g->hK.stress_bc_sides && d.bf.nbf > 0)
                 k_stress_bc_facets<<<blocks(d.bf.nbf, 128), 128, 0, g->stream>>>(d);
-            k_fn_c<<<nb, kNodeBlock, 0, g->stream>>>(d);
+            if (octets(g, 2))
+                k_fn_c_small<<<ob, kSmallBlock, 0, g->stream>>>(d);
+            else
+                k_fn_c<<<nb, kNodeBlock, 0, g->stream>>>(d);
             launch_surface(g);
             break;
         }
@@ -639,6 +689,11 @@ void launch_ea(des_gpu *g, int b0, int b1)
     else
 {
         const int n = b1 - b0, e0 = b0 * kElemBlock;
+        if (quads_ea(g)) {
+            constexpr int kQuads = kElemBlock * 4 / kSmallBlock;     // blocks of four lanes an element per block of one
+            k_ea_quad<<<n * kQuads, kSmallBlock, 0, g->stream>>>(g->d, e0, nb * kQuads);
+            return;
+        }
         k_ea_geometry<true, 128, 10><<<n, 128, 0, g->stream>>>(g->d, e0, nb);
         k_ea_rotate<true, 128, 7><<<n, 128, 0, g->stream>>>(g->d, e0);
         if (g->hK.thermal) k_ea_conduction<true, 128, 8><<<n, 128, 0, g->stream>>>(g->d, e0);
@@ -1164,7 +1219,7 @@ long long des_gpu_device_bytes(const des_gpu *g) { return g ? g->bytes : 0; }
 int des_gpu_kernels_per_step(const des_gpu *g)
 {
     if (!g) return 0;
-    int n = kStepKernels + (g->prec == DES_PREC_FP64 ? (g->hK.thermal ? 2 : 1) : 0) +   // FP64: E-A's three kernels
+    int n = kStepKernels + (g->prec == DES_PREC_FP64 && !quads_ea(g) ? (g->hK.thermal ? 2 : 1) : 0) +   // FP64: E-A's three kernels
             ((g->hK.stress_bc_sides && g->d.bf.nbf > 0) ? 1 : 0);
     if (g->P.surface_process_option == 1) n += g->d.bf.nbf > 0 ? 2 : 1;
     if (g->P.surface_process_option == 101) n += 1;
