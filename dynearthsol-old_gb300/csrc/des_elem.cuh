@@ -131,8 +131,16 @@ static __device__ __noinline__ void ea_gradients_exact(const Dev &d, int e, doub
 
 // volume, shape functions, mass contributions, dt minimum.  FP64 pipe 70 % and
 // integer ALU 70 % busy; 10 blocks of 128 per SM (8 or 12: the same within 1 %)
-template <bool SOFT, int BLK, int MINB>
-__global__ void __launch_bounds__(BLK, MINB) k_ea_geometry(Dev d, int e0, unsigned nblocks)
+//
+// PARTS: what the kernel does.  kStep is E-A's; the others are the reference's
+// functions: compute_volume (vol_old taken along with kSaveOld), compute_mass's
+// element half into tmp[0..2] (temperatures from Tsrc, NULL for 0),
+// compute_shape_fn.
+enum { kVolume = 1, kSaveOld = 2, kMass = 4, kShape = 8, kStep = 16 };
+constexpr int kStepGeometry = kStep | kVolume | kSaveOld | kShape;
+
+template <bool SOFT, int BLK, int MINB, int PARTS>
+__global__ void __launch_bounds__(BLK, MINB) k_ea_geometry(Dev d, int e0, unsigned nblocks, const double *Tsrc)
 {
     using N = Num<SOFT>;
     using Op = typename N::Op;
@@ -141,17 +149,16 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_geometry(Dev d, int e0, unsign
     const Consts &K = *d.K;
     const bool live = e < d.nelem;
     const int4 c = live ? d.conn[e] : int4{0, 0, 0, 0};
-    const bool dt_step = (K.fixed_dt == 0) && (d.clk->steps % 10 == 0);
-    if (e == 0) d.clk->mass_valid = 0;
+    const bool dt_step = (PARTS & kStep) && (K.fixed_dt == 0) && (d.clk->steps % 10 == 0);
+    if ((PARTS & kStep) && e == 0) d.clk->mass_valid = 0;
     double minh = 0;
     if (live) {
         const size_t E = d.nelem;
         double *se = s_edge + threadIdx.x;
-        double vol;
-        {
+        double e01[3], e12[3], e23[3];
+        if (PARTS & (kVolume | kShape)) {
             double X[4][3];
             load_xyz4(d, c, X);
-            double e01[3], e12[3], e23[3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 e01[k] = X[0][k] - X[1][k];
@@ -160,10 +167,15 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_geometry(Dev d, int e0, unsign
                 se[(kE01 + k) * BLK] = e01[k];
                 se[(kE12 + k) * BLK] = e12[k];
                 se[(kE23 + k) * BLK] = e23[k];
-                se[(kE02 + k) * BLK] = X[0][k] - X[2][k];
-                se[(kE03 + k) * BLK] = X[0][k] - X[3][k];
-                se[(kE13 + k) * BLK] = X[1][k] - X[3][k];
+                if (PARTS & kShape) {
+                    se[(kE02 + k) * BLK] = X[0][k] - X[2][k];
+                    se[(kE03 + k) * BLK] = X[0][k] - X[3][k];
+                    se[(kE13 + k) * BLK] = X[1][k] - X[3][k];
+                }
             }
+        }
+        double vol;
+        if (PARTS & kVolume) {
             // compute_volume (geometry.cxx:29-49)
             uint32_t far = 0;
             Op a[3], b[3], g[3];
@@ -178,43 +190,50 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_geometry(Dev d, int e0, unsign
             const double c2 = N::mul(b[1], a[2]) - N::mul(a[1], b[2]);
             vol = sf::div6(N::mul(a[0], N::op(c0, far)) + N::mul(b[0], N::op(c1, far)) + N::mul(g[0], N::op(c2, far)));
             if (SOFT && !sf::in_range(far)) vol = ea_volume_exact<BLK>(se);
+            if (PARTS & kSaveOld) d.vol_old[e] = d.vol[e];
+            d.vol[e] = vol;
+            if (not_positive(vol)) atomicOr(&d.clk->status, 0x4u);
+        } else {
+            vol = d.vol[e];
         }
-        d.vol_old[e] = d.vol[e];
-        d.vol[e] = vol;
-        if (not_positive(vol)) atomicOr(&d.clk->status, 0x4u);
         if (dt_step) minh = edge_min_height<BLK>(se, vol);
-        // compute_mass's element half (geometry.cxx:354-365)
-        {
+        if (PARTS & (kMass | kStep)) {
+            // compute_mass's element half (geometry.cxx:354-365)
             const Mix &x = K.M.mix[d.mix[e]];
-            double Tn[4];
-            load_nodal4(d.T, c, Tn);
+            const double *Ts = (PARTS & kStep) ? d.T : Tsrc;
+            double Tn[4] = {0, 0, 0, 0};
+            if ((PARTS & kStep) || Ts) load_nodal4(Ts, c, Tn);
             const double rT = mat_rho(K.M, x, elem_mean4(Tn[0], Tn[1], Tn[2], Tn[3]));
             const double rho = K.is_qs ? x.rho_qs : rT;
-            d.c_mass[e] = sf::quarter(sf::mul(rho, vol));
-            if (K.thermal) d.c_tmass[e] = sf::quarter(sf::mul(sf::mul(rT, x.cp), vol));
+            ((PARTS & kStep) ? d.c_mass : d.tmp + E)[e] = sf::quarter(sf::mul(rho, vol));
+            if (K.thermal)
+                ((PARTS & kStep) ? d.c_tmass : d.tmp + 2 * E)[e] = sf::quarter(sf::mul(sf::mul(rT, x.cp), vol));
+            if (!(PARTS & kStep)) d.tmp[e] = vol;
         }
-        // compute_shape_fn (geometry.cxx:410-452): node i's gradient is
-        // (a x b) / 6V with the edges (a, b) = (13, 12) (02, 23) (13, 03) (01, 02)
-        uint32_t far = 0;
-        const Op oiv = N::op(sf::div(1.0, sf::mul(6.0, vol)), far);
+        if (PARTS & kShape) {
+            // compute_shape_fn (geometry.cxx:410-452): node i's gradient is
+            // (a x b) / 6V with the edges (a, b) = (13, 12) (02, 23) (13, 03) (01, 02)
+            uint32_t far = 0;
+            const Op oiv = N::op(sf::div(1.0, sf::mul(6.0, vol)), far);
 #pragma unroll 1
-        for (int i = 0; i < 4; ++i) {
-            double ea[3], eb[3], g[3];
-            load_edge<BLK>(se, (0x0c3c >> (4 * i)) & 15, ea);
-            load_edge<BLK>(se, (0x36f9 >> (4 * i)) & 15, eb);
-            Op a[3], b[3];
+            for (int i = 0; i < 4; ++i) {
+                double ea[3], eb[3], g[3];
+                load_edge<BLK>(se, (0x0c3c >> (4 * i)) & 15, ea);
+                load_edge<BLK>(se, (0x36f9 >> (4 * i)) & 15, eb);
+                Op a[3], b[3];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                a[k] = N::op(ea[k], far);
-                b[k] = N::op(eb[k], far);
+                for (int k = 0; k < 3; ++k) {
+                    a[k] = N::op(ea[k], far);
+                    b[k] = N::op(eb[k], far);
+                }
+                g[0] = N::mul(a[1], b[2]) - N::mul(a[2], b[1]);
+                g[1] = N::mul(a[2], b[0]) - N::mul(a[0], b[2]);
+                g[2] = N::mul(a[0], b[1]) - N::mul(a[1], b[0]);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) d.shp[(size_t)(4 * k + i) * E + e] = N::mul(oiv, N::op(g[k], far));
             }
-            g[0] = N::mul(a[1], b[2]) - N::mul(a[2], b[1]);
-            g[1] = N::mul(a[2], b[0]) - N::mul(a[0], b[2]);
-            g[2] = N::mul(a[0], b[1]) - N::mul(a[1], b[0]);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) d.shp[(size_t)(4 * k + i) * E + e] = N::mul(oiv, N::op(g[k], far));
+            if (SOFT && !sf::in_range(far)) ea_gradients_exact(d, e, vol);
         }
-        if (SOFT && !sf::in_range(far)) ea_gradients_exact(d, e, vol);
     }
     if (dt_step) dt_reduce_and_finalize(d, minh, live, nblocks);
 }
@@ -230,19 +249,27 @@ static __device__ __noinline__ void ea_rates_exact(const Dev &d, int e, double *
     spin(V, dx, dy, dz, out[6], out[7], out[8]);
 }
 
-static __device__ __noinline__ void ea_rotate_exact(const Dev &d, int e, double *arr, double w3, double w4, double w5)
+static __device__ __noinline__ void ea_rotate_exact(const Dev &d, int e, double *arr, double dt, double w3, double w4,
+                                                    double w5)
 {
     double s[6];
     load6(arr, d.nelem, e, s);
-    jaumann(s, d.clk->step_dt, w3, w4, w5);
+    jaumann(s, dt, w3, w4, w5);
     store6(arr, d.nelem, e, s);
 }
 
 // the next strain rate, its dvoldt contribution, rotate_stress.  89 FP64
 // instructions per element at 82 % of the nominal rate, the pipe's measured peak;
 // 7 blocks of 128 per SM (6: 2 % slower, 8 and 9 the same)
-template <bool SOFT, int BLK, int MINB>
-__global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0)
+//
+// PARTS: kRates the strain rate into out, kDvoldt its dvoldt contribution,
+// kRotate the rotation with the current dt, kStepRotate the same with the
+// running step's, where the rheology has it.
+enum { kRates = 1, kDvoldt = 2, kRotate = 4, kStepRotate = 8 };
+constexpr int kStepRates = kRates | kDvoldt | kStepRotate;
+
+template <bool SOFT, int BLK, int MINB, int PARTS>
+__global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0, double *out)
 {
     using N = Num<SOFT>;
     using Op = typename N::Op;
@@ -306,17 +333,18 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0)
             for (int k = 0; k < 3; ++k) u[k] = 2 * r[6 + k];
         }
     }
-    store6(d.srate_next, E, e, D);
-    d.c_trdv[e] = sf::mul(tr3(D), d.vol[e]);
+    if (PARTS & kRates) store6(out, E, e, D);
+    if (PARTS & kDvoldt) d.c_trdv[e] = sf::mul(tr3(D), d.vol[e]);
     // rotate_stress (fields.cxx:419-433) with u = 2 w, twice the spin:
     // powers of two move through the products and sums exactly (the
     // operands are in range), so dt inc is dt (sum with u) for the normal
     // components, where the reference has 2 s_ab w, and (dt / 2) (sum
     // with u) for the others
-    if (!(d.K->rheol & 1)) return;
+    if (!(PARTS & (kRotate | kStepRotate)) || ((PARTS & kStepRotate) && !(d.K->rheol & 1))) return;
     uint32_t farw = 0;
     const Op w3 = N::op(u[0], farw), w4 = N::op(u[1], farw), w5 = N::op(u[2], farw);
-    const Op odt = N::op(d.clk->step_dt, farw), hdt = N::half(odt);
+    const double dt = (PARTS & kStepRotate) ? d.clk->step_dt : d.clk->dt;
+    const Op odt = N::op(dt, farw), hdt = N::half(odt);
 #pragma unroll 1
     for (int f = 0; f < 2; ++f) {
         double *arr = f ? d.strain : d.stress;
@@ -336,7 +364,7 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0)
         if (!SOFT || sf::in_range(far))
             store6(arr, E, e, s);
         else
-            ea_rotate_exact(d, e, arr, 0.5 * u[0], 0.5 * u[1], 0.5 * u[2]);
+            ea_rotate_exact(d, e, arr, dt, 0.5 * u[0], 0.5 * u[1], 0.5 * u[2]);
     }
 }
 
@@ -424,7 +452,8 @@ static __device__ __noinline__ void ec_force_exact(const Dev &d, int e)
 }
 
 // 12 blocks of 128 per SM (8: 349 us on 3.84M elements, 10: 332, 12: 330)
-template <bool SOFT, int BLK, int MINB>
+// NMD: E-C; without it the force vectors alone (update_force's element half)
+template <bool SOFT, int BLK, int MINB, bool NMD>
 __global__ void __launch_bounds__(BLK, MINB) k_fe_c(Dev d)
 {
     using N = Num<SOFT>;
@@ -436,14 +465,16 @@ __global__ void __launch_bounds__(BLK, MINB) k_fe_c(Dev d)
     const int4 c = d.conn[e];
     double s[6];
     load6(d.stress, E, e, s);
-    double a[4];
-    load_nodal4(d.ntmp, c, a);
-    double dpe = sf::add0(a[0]);                // 0 + a0, then the rest; / 4, / 3
-    for (int i = 1; i < 4; ++i) dpe += a[i];
-    const double ddp = sf::div3(-d.dp[e] + sf::quarter(dpe));
-    for (int i = 0; i < 3; ++i) {
-        s[i] += ddp;
-        d.stress[i * E + e] = s[i];
+    if (NMD) {
+        double a[4];
+        load_nodal4(d.ntmp, c, a);
+        double dpe = sf::add0(a[0]);            // 0 + a0, then the rest; / 4, / 3
+        for (int i = 1; i < 4; ++i) dpe += a[i];
+        const double ddp = sf::div3(-d.dp[e] + sf::quarter(dpe));
+        for (int i = 0; i < 3; ++i) {
+            s[i] += ddp;
+            d.stress[i * E + e] = s[i];
+        }
     }
     double buoy = 0;
     if (K.gravity != 0) {

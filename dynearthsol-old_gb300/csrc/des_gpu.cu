@@ -50,6 +50,7 @@ struct des_gpu {
     cudaGraphExec_t graph = nullptr;      // one step
     cudaGraphExec_t graph_many = nullptr; // kGraphSteps steps
     bool primed = false;
+    bool mass_valid = false;              // the clock's mass_valid, as the queued work leaves it
     int prec = DES_PREC_FP64;
     DevF f;
     ConstsF hF;
@@ -496,21 +497,27 @@ int read_clock(des_gpu *g, Clock &c)
     return DES_OK;
 }
 
+// nodal masses from the last E-A's contributions, before they are read
+int flush_masses(des_gpu *g)
+{
+    if (g->mass_valid) return DES_OK;
+    const int nb = blocks(g->nnode, kNodeBlock);
+    if (g->prec == DES_PREC_FP32)
+        kf_mass_flush<<<nb, kNodeBlock, 0, g->stream>>>(g->f);
+    else
+        k_mass_node<<<nb, kNodeBlock, 0, g->stream>>>(g->d, g->d.vol, g->d.c_mass, g->d.c_tmass);
+    DES_LAUNCH();
+    g->mass_valid = true;
+    return DES_OK;
+}
+
 // nodal masses current and fused-pass priming invalidated before a
-// per-function call
+// per-function call (the host follows the clock's mass_valid: reading it back
+// would wait for the stream in every call)
 int begin_fn(des_gpu *g)
 {
     if (!g) return DES_ERR_ARG;
-    Clock c;
-    int rc = read_clock(g, c);
-    if (rc) return rc;
-    if (!c.mass_valid) {
-        if (g->prec == DES_PREC_FP32)
-            kf_mass_flush<<<blocks(g->nnode, kNodeBlock), kNodeBlock, 0, g->stream>>>(g->f);
-        else
-            k_mass_flush<<<blocks(g->nnode, kNodeBlock), kNodeBlock, 0, g->stream>>>(g->d);
-        DES_LAUNCH();
-    }
+    if (int rc = flush_masses(g)) return rc;
     g->primed = false;
     return DES_OK;
 }
@@ -523,13 +530,33 @@ int begin_fn64(des_gpu *g)
     return begin_fn(g);
 }
 
+// the parts of the geometry kernel that the entry points ask for
+template <int PARTS>
+void launch_geometry(des_gpu *g, const double *Tsrc)
+{
+    k_ea_geometry<true, 128, 10, PARTS><<<blocks(g->nelem, 128), 128, 0, g->stream>>>(g->d, 0, 0, Tsrc);
+}
+
+// compute_mass's node half from the element kernel's tmp[0..2]
+void launch_masses(des_gpu *g)
+{
+    const size_t E = g->nelem;
+    k_mass_node<<<blocks(g->nnode, kNodeBlock), kNodeBlock, 0, g->stream>>>(g->d, g->d.tmp, g->d.tmp + E,
+                                                                            g->d.tmp + 2 * E);
+    g->mass_valid = true;
+}
+
 int prime(des_gpu *g)
 {
     if (g->primed) return DES_OK;
     if (g->prec == DES_PREC_FP32)
         kf_prime<<<blocks(g->nelem, kElemBlock), kElemBlock, 0, g->stream>>>(g->f);
     else
-        k_prime<<<blocks(g->nelem, kElemBlock), kElemBlock, 0, g->stream>>>(g->d);
+        {
+            const int eb = blocks(g->nelem, 128);
+            k_ea_rotate<true, 128, 7, kRates | kDvoldt><<<eb, 128, 0, g->stream>>>(g->d, 0, g->d.srate_next);
+            if (g->hK.thermal) k_ea_conduction<true, 128, 8><<<eb, 128, 0, g->stream>>>(g->d, 0);
+        }
     DES_LAUNCH();
     g->primed = true;
     return DES_OK;
@@ -656,7 +683,7 @@ void launch_pass(des_gpu *g, int k)
             if (quads_ec(g))
                 k_fe_c_quad<<<blocks(4LL * g->nelem, kSmallBlock), kSmallBlock, 0, g->stream>>>(d);
             else
-                k_fe_c<true, 128, 12><<<eb, kElemBlock, 0, g->stream>>>(d);
+                k_fe_c<true, 128, 12, true><<<eb, kElemBlock, 0, g->stream>>>(d);
             break;
         default:
             if (g->hK.stress_bc_sides && d.bf.nbf > 0)
@@ -683,6 +710,7 @@ void launch_head(des_gpu *g, cudaEvent_t *ev)
 // E-A over the element blocks [b0, b1) of its nblocks
 void launch_ea(des_gpu *g, int b0, int b1)
 {
+    g->mass_valid = false;
     const int nb = blocks(g->nelem, kElemBlock);
     if (g->prec == DES_PREC_FP32)
         kf_fe_a<<<b1 - b0, kElemBlock, 0, g->stream>>>(g->f, b0 * kElemBlock, nb);
@@ -694,8 +722,8 @@ void launch_ea(des_gpu *g, int b0, int b1)
             k_ea_quad<<<n * kQuads, kSmallBlock, 0, g->stream>>>(g->d, e0, nb * kQuads);
             return;
         }
-        k_ea_geometry<true, 128, 10><<<n, 128, 0, g->stream>>>(g->d, e0, nb);
-        k_ea_rotate<true, 128, 7><<<n, 128, 0, g->stream>>>(g->d, e0);
+        k_ea_geometry<true, 128, 10, kStepGeometry><<<n, 128, 0, g->stream>>>(g->d, e0, nb, nullptr);
+        k_ea_rotate<true, 128, 7, kStepRates><<<n, 128, 0, g->stream>>>(g->d, e0, g->d.srate_next);
         if (g->hK.thermal) k_ea_conduction<true, 128, 8><<<n, 128, 0, g->stream>>>(g->d, e0);
     }
 }
@@ -785,7 +813,9 @@ int capture_steps(des_gpu *g, int nsteps, cudaGraphExec_t *out)
 {
     cudaGraph_t graph;
     DES_CUDA(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
+    const bool masses = g->mass_valid;    // (nothing has run)
     for (int i = 0; i < nsteps; ++i) launch_step(g, nullptr);
+    g->mass_valid = masses;
     cudaError_t e = cudaStreamEndCapture(g->stream, &graph);
     if (e != cudaSuccess) return DES_ERR_CUDA;
     e = cudaGraphInstantiate(out, graph, 0);
@@ -814,6 +844,7 @@ int ensure_graphs(des_gpu *g, int nsteps)
 int launch_graphs(des_gpu *g, int nsteps)
 {
     int i = 0;
+    if (nsteps > 0) g->mass_valid = false;
     if (g->graph_many)
         for (; i + kGraphSteps <= nsteps; i += kGraphSteps) DES_CUDA(cudaGraphLaunch(g->graph_many, g->stream));
     for (; i < nsteps; ++i) DES_CUDA(cudaGraphLaunch(g->graph, g->stream));
@@ -1304,7 +1335,10 @@ int des_gpu_upload(des_gpu *g, const des_state_view *h, unsigned mask)
             c.dt = h->dt;
             c.steps = h->steps;
         }
-        if (mask & DES_F_MASS) c.mass_valid = 1;
+        if (mask & DES_F_MASS) {
+            c.mass_valid = 1;
+            g->mass_valid = true;
+        }
         k_clock_set<<<1, 32, 0, g->stream>>>(g->dclk, c.time, c.dt, c.steps, c.mass_valid);
         DES_LAUNCH();
     }
@@ -1432,18 +1466,6 @@ static int download_async(des_gpu *g, const std::vector<DownPart> &parts, long l
     return DES_OK;
 }
 
-// nodal masses from the last E-A's contributions, before they are read
-static int flush_masses(des_gpu *g, const Clock &c)
-{
-    if (c.mass_valid) return DES_OK;
-    if (g->prec == DES_PREC_FP32)
-        kf_mass_flush<<<blocks(g->nnode, kNodeBlock), kNodeBlock, 0, g->stream>>>(g->f);
-    else
-        k_mass_flush<<<blocks(g->nnode, kNodeBlock), kNodeBlock, 0, g->stream>>>(g->d);
-    DES_LAUNCH();
-    return DES_OK;
-}
-
 int des_gpu_download(des_gpu *g, des_state_view *h, unsigned mask)
 {
     if (!g || !h || h->nnode != g->nnode || h->nelem != g->nelem) return DES_ERR_ARG;
@@ -1451,7 +1473,7 @@ int des_gpu_download(des_gpu *g, des_state_view *h, unsigned mask)
     Clock c;
     int rc = read_clock(g, c);
     if (rc) return rc;
-    if ((mask & DES_F_MASS) && (rc = flush_masses(g, c))) return rc;
+    if ((mask & DES_F_MASS) && (rc = flush_masses(g))) return rc;
     if ((rc = download_fields(g, h, mask))) return rc;
     if (mask & DES_F_SCALARS) {
         h->time = c.time;
@@ -1963,24 +1985,17 @@ static int finish_elements_async(des_gpu *g, const des_state_view *h, unsigned l
 // and temperature, the values update_mesh (dynearthsol.cxx:237-261) leaves
 static int derive_geometry(des_gpu *g)
 {
-    const int eb = blocks(g->nelem, kElemBlock), nb = blocks(g->nnode, kNodeBlock);
-    cudaStream_t s = g->stream;
     if (g->prec == DES_PREC_FP32) {
-        kf_derive_geometry<<<eb, kElemBlock, 0, s>>>(g->f);
-        kf_mass_flush<<<nb, kNodeBlock, 0, s>>>(g->f);
+        kf_derive_geometry<<<blocks(g->nelem, kElemBlock), kElemBlock, 0, g->stream>>>(g->f);
+        kf_mass_flush<<<blocks(g->nnode, kNodeBlock), kNodeBlock, 0, g->stream>>>(g->f);
     } else {
-        k_volume<<<eb, kElemBlock, 0, s>>>(g->d, 0);
-        k_shape<<<eb, kElemBlock, 0, s>>>(g->d);
-        k_mass_elem<<<eb, kElemBlock, 0, s>>>(g->d, g->d.T);
-        k_mass_node<<<nb, kNodeBlock, 0, s>>>(g->d);
+        launch_geometry<kVolume | kShape | kMass>(g, g->d.T);
+        launch_masses(g);
     }
     DES_LAUNCH();
-    Clock c;
-    if (int rc = read_clock(g, c)) return rc;
-    k_clock_set<<<1, 32, 0, g->stream>>>(g->dclk, c.time, c.dt, c.steps, 1);
-    DES_LAUNCH();
+    g->mass_valid = true;
     g->primed = false;
-    return finish(g);
+    return DES_OK;
 }
 
 // the end of a host-buffer step once passes N-A .. N-C are queued and their
@@ -2018,7 +2033,7 @@ static int step_host_tail(des_gpu *g, des_state_view *host, unsigned mask, const
     if (!rc && report && (rc = des_gpu_report(g, report)) == DES_OK &&
         (report->status & (DES_STATUS_DT_NONPOSITIVE | DES_STATUS_NONFINITE)))
         rc = DES_ERR_DT;
-    if (!rc && (mask & DES_F_MASS)) rc = flush_masses(g, c);
+    if (!rc && (mask & DES_F_MASS)) rc = flush_masses(g);
     if (!rc) rc = download_async(g, late_node, &off);
     const cudaError_t ce = cudaStreamSynchronize(g->copy_stream);
     if (rc) return rc;
@@ -2246,7 +2261,7 @@ int des_gpu_update_temperature(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_temp_elem<<<ELEM_GRID(g)>>>(g->d);
+    k_ea_conduction<true, 128, 8><<<ELEM_GRID(g)>>>(g->d, 0);
     k_temp_node<<<NODE_GRID(g)>>>(g->d);
     return finish(g);
 }
@@ -2254,7 +2269,7 @@ int des_gpu_update_strain_rate(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_srate<<<ELEM_GRID(g)>>>(g->d, g->d.srate);
+    k_ea_rotate<true, 128, 7, kRates><<<ELEM_GRID(g)>>>(g->d, 0, g->d.srate);
     return finish(g);
 }
 int des_gpu_compute_dvoldt(des_gpu *g)
@@ -2276,7 +2291,11 @@ int des_gpu_update_stress(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_stress<<<ELEM_GRID(g)>>>(g->d);
+    switch (g->hK.rheol) {
+    case 5: k_stress<5><<<ELEM_GRID(g)>>>(g->d); break;
+    case 7: k_stress<7><<<ELEM_GRID(g)>>>(g->d); break;
+    default: k_stress<0><<<ELEM_GRID(g)>>>(g->d); break;
+    }
     return finish(g);
 }
 int des_gpu_NMD_stress(des_gpu *g)
@@ -2292,7 +2311,7 @@ int des_gpu_update_force(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_force_elem<<<ELEM_GRID(g)>>>(g->d);
+    k_fe_c<true, 128, 12, false><<<ELEM_GRID(g)>>>(g->d);
     if (g->hK.stress_bc_sides && g->d.bf.nbf > 0)
         k_stress_bc_facets<<<blocks(g->d.bf.nbf, 128), 128, 0, g->stream>>>(g->d);
     k_force_node<<<NODE_GRID(g)>>>(g->d, g->hK.is_qs);
@@ -2323,23 +2342,22 @@ int des_gpu_compute_volume(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_volume<<<ELEM_GRID(g)>>>(g->d, 0);
+    launch_geometry<kVolume>(g, nullptr);
     return finish(g);
 }
 int des_gpu_compute_mass(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_mass_elem<<<ELEM_GRID(g)>>>(g->d, g->d.T);
-    k_mass_node<<<NODE_GRID(g)>>>(g->d);
-    k_clock_mass_valid<<<1, 32, 0, g->stream>>>(g->dclk, 1);
+    launch_geometry<kMass>(g, g->d.T);
+    launch_masses(g);
     return finish(g);
 }
 int des_gpu_compute_shape_fn(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_shape<<<ELEM_GRID(g)>>>(g->d);
+    launch_geometry<kShape>(g, nullptr);
     return finish(g);
 }
 int des_gpu_update_mesh(des_gpu *g)
@@ -2348,18 +2366,15 @@ int des_gpu_update_mesh(des_gpu *g)
     if (rc) return rc;
     k_coord<<<NODE_GRID(g)>>>(g->d);
     launch_surface(g);
-    k_volume<<<ELEM_GRID(g)>>>(g->d, 1);
-    k_mass_elem<<<ELEM_GRID(g)>>>(g->d, g->d.T);
-    k_mass_node<<<NODE_GRID(g)>>>(g->d);
-    k_clock_mass_valid<<<1, 32, 0, g->stream>>>(g->dclk, 1);
-    k_shape<<<ELEM_GRID(g)>>>(g->d);
+    launch_geometry<kVolume | kSaveOld | kMass | kShape>(g, g->d.T);
+    launch_masses(g);
     return finish(g);
 }
 int des_gpu_rotate_stress(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_rotate<<<ELEM_GRID(g)>>>(g->d);
+    k_ea_rotate<true, 128, 7, kRotate><<<ELEM_GRID(g)>>>(g->d, 0, nullptr);
     return finish(g);
 }
 int des_gpu_compute_dt(des_gpu *g, double *dt_out)
@@ -2438,6 +2453,7 @@ static int init_fields_fp32(des_gpu *g)
     DES_CUDA(cudaMemcpyAsync(f.x0, f.x, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, s));
     kf_init_geometry<<<ELEM_GRID(g)>>>(f);
     kf_mass_flush<<<NODE_GRID(g)>>>(f);
+    g->mass_valid = true;
     k_clock_set<<<1, 32, 0, s>>>(g->dclk, 0.0, 0.0, 0, 1);
     kf_vbcs<<<NODE_GRID(g)>>>(f);
     if (g->P.gravity != 0) kf_init_stress<<<ELEM_GRID(g)>>>(f);
@@ -2470,12 +2486,10 @@ int des_gpu_init_fields(des_gpu *g)
     DES_CUDA(cudaMemsetAsync(d.strain, 0, sizeof(double) * 6 * E, s));
     DES_CUDA(cudaMemsetAsync(d.srate, 0, sizeof(double) * 6 * E, s));
     DES_CUDA(cudaMemcpyAsync(d.x0, d.x, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, s));
-    k_volume<<<ELEM_GRID(g)>>>(d, 0);
+    launch_geometry<kVolume | kMass | kShape>(g, nullptr);
     DES_CUDA(cudaMemcpyAsync(d.vol_old, d.vol, sizeof(double) * E, cudaMemcpyDeviceToDevice, s));
-    k_mass_elem<<<ELEM_GRID(g)>>>(d, nullptr);
-    k_mass_node<<<NODE_GRID(g)>>>(d);
+    launch_masses(g);
     k_clock_set<<<1, 32, 0, s>>>(g->dclk, 0.0, 0.0, 0, 1);
-    k_shape<<<ELEM_GRID(g)>>>(d);
     k_vbcs<<<NODE_GRID(g)>>>(d);
     if (g->P.gravity != 0) {
         k_init_stress<<<ELEM_GRID(g)>>>(d);

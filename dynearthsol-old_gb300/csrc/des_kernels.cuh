@@ -535,21 +535,6 @@ __device__ void dt_reduce_and_finalize(const Dev &d, double minh, bool active, u
 // per-function kernels
 // ===========================================================================
 
-// fields.cxx:119-144
-__global__ void k_temp_elem(Dev d)
-{
-    int e = gtid();
-    if (e >= d.nelem) return;
-    const size_t E = d.nelem;
-    int4 c = d.conn[e];
-    double dx[4], dy[4], dz[4], Tn[4], tr[4];
-    load_shp(d, e, dx, dy, dz);
-    load_nodal4(d.T, c, Tn);
-    double kv = d.K->M.mix[d.mix[e]].k * d.vol[e];
-    conduction(dx, dy, dz, Tn, kv, tr);
-    for (int i = 0; i < 4; ++i) d.tmp[i * E + e] = tr[i];
-}
-
 // fields.cxx:149-168
 __global__ void k_temp_node(Dev d)
 {
@@ -557,28 +542,15 @@ __global__ void k_temp_node(Dev d)
     if (n >= d.nnode) return;
     const size_t E = d.nelem;
     double tdot = 0;
-    for (int q = d.sup_off[n]; q < d.sup_off[n + 1]; ++q) {
-        unsigned p = __ldg(d.sup_ent + q);
-        tdot += d.tmp[(p & 3u) * E + (p >> 2)];
-    }
+    walk<4>(
+        d.sup_ent, d.sup_off[n], d.sup_off[n + 1], [&](unsigned p) { return d.tmp[(p & 3u) * E + (p >> 2)]; },
+        [&](double v) { tdot += v; });
     d.ntmp[n] = tdot;
     const Consts &K = *d.K;
     if (d.bcflag[n] & kBoundZ1)
         d.T[n] = K.surface_temperature;
     else
-        d.T[n] -= tdot * d.clk->dt / d.tmass[n];
-}
-
-// fields.cxx:184-243; out = srate or srate_next
-__global__ void k_srate(Dev d, double *out)
-{
-    int e = gtid();
-    if (e >= d.nelem) return;
-    double V[4][3], dx[4], dy[4], dz[4], s[6];
-    load_vel4(d, d.conn[e], V);
-    load_shp(d, e, dx, dy, dz);
-    strain_rate(V, dx, dy, dz, s);
-    store6(out, d.nelem, e, s);
+        d.T[n] -= sf::div(sf::mul(tdot, d.clk->dt), d.tmass[n]);
 }
 
 // geometry.cxx:128-134 (src = srate) and 200-204 (dp)
@@ -588,13 +560,13 @@ __global__ void k_dvoldt_elem(Dev d)
     if (e >= d.nelem) return;
     const size_t E = d.nelem;
     double dj = d.srate[e] + d.srate[E + e] + d.srate[2 * E + e];
-    d.tmp_sg[e] = dj * d.vol[e];
+    d.tmp_sg[e] = sf::mul(dj, d.vol[e]);
 }
 __global__ void k_dp_elem(Dev d)
 {
     int e = gtid();
     if (e >= d.nelem) return;
-    d.tmp_sg[e] = d.dp[e] * d.vol[e];
+    d.tmp_sg[e] = sf::mul(d.dp[e], d.vol[e]);
 }
 
 // geometry.cxx:138-143 and 208-213: ntmp[n] = sum(tmp_sg) / volume_n
@@ -622,7 +594,8 @@ __global__ void k_edvoldt(Dev d)
 }
 
 // rheology.cxx:525-650
-__global__ void k_stress(Dev d)
+template <int RHEOL>
+__global__ void __launch_bounds__(128, 8) k_stress(Dev d)
 {
     int e = gtid();
     bool live = e < d.nelem;
@@ -634,7 +607,7 @@ __global__ void k_stress(Dev d)
         load6(d.strain, E, e, es);
         load6(d.srate, E, e, edot);
         double pls = d.pls[e], dpls = d.dpls[e], dpress;
-        flags = stress_body<0>(d, e, d.conn[e], d.edvoldt[e], d.clk->dt, s, es, edot, pls, dpls, dpress);
+        flags = stress_body<RHEOL>(d, e, d.conn[e], d.edvoldt[e], d.clk->dt, s, es, edot, pls, dpls, dpress);
         store6(d.stress, E, e, s);
         store6(d.strain, E, e, es);
         store6(d.srate, E, e, edot);
@@ -660,7 +633,7 @@ __global__ void k_nmd_apply(Dev d)
     for (int i = 0; i < 3; ++i) d.stress[i * E + e] += ddp;
 }
 
-// fields.cxx:321-346: element force vectors into tmp[12][E]
+// fields.cxx:321-346: element force vectors into tmp[12][E], on the FP64 unit
 __device__ __forceinline__ void force_elem_body(const Dev &d, int e, int4 c, const double s[6])
 {
     const size_t E = d.nelem;
@@ -672,24 +645,13 @@ __device__ __forceinline__ void force_elem_body(const Dev &d, int e, int4 c, con
     if (K.gravity != 0) {
         double Tn[4];
         load_nodal4(d.T, c, Tn);
-        buoy = sf::quarter(mat_rho(K.M, K.M.mix[d.mix[e]], elem_mean4(Tn[0], Tn[1], Tn[2], Tn[3])) * K.gravity);
+        buoy = mat_rho(K.M, K.M.mix[d.mix[e]], elem_mean4(Tn[0], Tn[1], Tn[2], Tn[3])) * K.gravity / 4;
     }
-    // (products on the integer pipes, sf::mul)
     for (int i = 0; i < 4; ++i) {
-        d.tmp[(i)*E + e] = sf::mul(sf::mul(s[0], dx[i]) + sf::mul(s[3], dy[i]) + sf::mul(s[4], dz[i]), vol);
-        d.tmp[(i + 4) * E + e] =
-            sf::mul(sf::mul(s[3], dx[i]) + sf::mul(s[1], dy[i]) + sf::mul(s[5], dz[i]), vol);
-        d.tmp[(i + 8) * E + e] =
-            sf::mul(sf::mul(s[4], dx[i]) + sf::mul(s[5], dy[i]) + sf::mul(s[2], dz[i]) + buoy, vol);
+        d.tmp[(i)*E + e] = (s[0] * dx[i] + s[3] * dy[i] + s[4] * dz[i]) * vol;
+        d.tmp[(i + 4) * E + e] = (s[3] * dx[i] + s[1] * dy[i] + s[5] * dz[i]) * vol;
+        d.tmp[(i + 8) * E + e] = (s[4] * dx[i] + s[5] * dy[i] + s[2] * dz[i] + buoy) * vol;
     }
-}
-__global__ void k_force_elem(Dev d)
-{
-    int e = gtid();
-    if (e >= d.nelem) return;
-    double s[6];
-    load6(d.stress, d.nelem, e, s);
-    force_elem_body(d, e, d.conn[e], s);
 }
 
 // node j of facet f of a tetrahedron (constants.hpp:61-67: {1,2,3},
@@ -814,19 +776,40 @@ __device__ __forceinline__ void stress_bc_node(const Consts &K, const BdryFacets
     if (K.elastic_foundation && (flag & kBoundZ0)) f[2] -= K.elastic_foundation_constant * (z - z0);
 }
 
-// fields.cxx:351-365 + apply_damping (fields.cxx:250-309)
+// fields.cxx:351-365
 __device__ __forceinline__ void force_gather(const Dev &d, int n, double f[3])
 {
     const size_t E = d.nelem;
     f[0] = f[1] = f[2] = 0;
-    for (int q = d.sup_off[n]; q < d.sup_off[n + 1]; ++q) {
-        unsigned p = __ldg(d.sup_ent + q);
-        size_t e = p >> 2, i = p & 3u;
-        f[0] -= d.tmp[(i)*E + e];
-        f[1] -= d.tmp[(i + 4) * E + e];
-        f[2] -= d.tmp[(i + 8) * E + e];
+    walk<4>(
+        d.sup_ent, d.sup_off[n], d.sup_off[n + 1],
+        [&](unsigned p) {
+            const double *t = d.tmp + (size_t)(p & 3u) * E + (p >> 2);
+            return Three<double>{t[0], t[4 * E], t[8 * E]};
+        },
+        [&](const Three<double> &t) {
+            f[0] -= t.x;
+            f[1] -= t.y;
+            f[2] -= t.z;
+        });
+}
+
+// v += dt f / m (fields.cxx:386-389): one reciprocal of m on the integer pipes
+// for the three
+__device__ __forceinline__ void velocity_step(const double f[3], double dt, double m, double v[3])
+{
+    uint32_t far = 0;
+    const sf::Den dm = sf::denominator(m, far);
+    for (int j = 0; j < 3; ++j) {
+        const double a = sf::mul(dt, f[j]);
+        uint32_t fa = far;
+        double q = sf::quotient(a, dm, fa);
+        if (!sf::in_range(fa)) q = sf::div_slow(a, m);
+        v[j] += q;
     }
 }
+
+// the gather and apply_damping (fields.cxx:250-309)
 __global__ void k_force_node(Dev d, int damping)
 {
     int n = gtid();
@@ -850,10 +833,12 @@ __global__ void k_velocity(Dev d)
 {
     int n = gtid();
     if (n >= d.nnode) return;
-    double dt = d.clk->dt, m = d.mass[n];
-    d.vx[n] += dt * d.fx[n] / m;
-    d.vy[n] += dt * d.fy[n] / m;
-    d.vz[n] += dt * d.fz[n] / m;
+    const double f[3] = {d.fx[n], d.fy[n], d.fz[n]};
+    double v[3] = {d.vx[n], d.vy[n], d.vz[n]};
+    velocity_step(f, d.clk->dt, d.mass[n], v);
+    d.vx[n] = v[0];
+    d.vy[n] = v[1];
+    d.vz[n] = v[2];
 }
 
 // remeshing.cxx:2046-2054: the bottom nodes' coord0 back on z = -zlength
@@ -884,93 +869,11 @@ __global__ void k_coord(Dev d)
     int n = gtid();
     if (n >= d.nnode) return;
     double dt = d.clk->dt;
-    d.x[n] += d.vx[n] * dt;
-    d.y[n] += d.vy[n] * dt;
-    d.z[n] += d.vz[n] * dt;
+    d.x[n] += sf::mul(d.vx[n], dt);
+    d.y[n] += sf::mul(d.vy[n], dt);
+    d.z[n] += sf::mul(d.vz[n], dt);
     // output.cxx:195-208 stops on NaN/Inf coordinates
     if (not_finite(d.x[n]) || not_finite(d.y[n]) || not_finite(d.z[n])) atomicOr(&d.clk->status, 0x2u);
-}
-
-// geometry.cxx:94-110; save_old copies volume into volume_old first
-__global__ void k_volume(Dev d, int save_old)
-{
-    int e = gtid();
-    if (e >= d.nelem) return;
-    double X[4][3];
-    load_xyz4(d, d.conn[e], X);
-    double v = tet_volume(X[0], X[1], X[2], X[3]);
-    if (save_old) d.vol_old[e] = d.vol[e];
-    d.vol[e] = v;
-    if (!(v > 0)) atomicOr(&d.clk->status, 0x4u);
-}
-
-// geometry.cxx:354-365; Tsrc = NULL means T = 0 (the first compute_mass of init)
-__global__ void k_mass_elem(Dev d, const double *Tsrc)
-{
-    int e = gtid();
-    if (e >= d.nelem) return;
-    const size_t E = d.nelem;
-    const Consts &K = *d.K;
-    const Mix &x = K.M.mix[d.mix[e]];
-    double Tn[4] = {0, 0, 0, 0};
-    if (Tsrc) load_nodal4(Tsrc, d.conn[e], Tn);
-    double rT = mat_rho(K.M, x, elem_mean4(Tn[0], Tn[1], Tn[2], Tn[3]));
-    double vol = d.vol[e];
-    double rho = K.is_qs ? x.rho_qs : rT;
-    double m = rho * vol / 4;
-    double tm = rT * x.cp * vol / 4;
-    d.tmp[e] = vol;
-    d.tmp[E + e] = m;
-    if (K.thermal) d.tmp[2 * E + e] = tm;
-}
-
-// geometry.cxx:370-381 from tmp[0..2]
-__global__ void k_mass_node(Dev d)
-{
-    int n = gtid();
-    if (n >= d.nnode) return;
-    const size_t E = d.nelem;
-    const bool thermal = d.K->thermal;
-    double vn = 0, m = 0, tm = 0;
-    for (int q = d.sup_off[n]; q < d.sup_off[n + 1]; ++q) {
-        size_t e = __ldg(d.sup_ent + q) >> 2;
-        vn += d.tmp[e];
-        m += d.tmp[E + e];
-        if (thermal) tm += d.tmp[2 * E + e];
-    }
-    d.vol_n[n] = vn;
-    d.mass[n] = m;
-    d.tmass[n] = tm;
-}
-
-// geometry.cxx:400-466
-__global__ void k_shape(Dev d)
-{
-    int e = gtid();
-    if (e >= d.nelem) return;
-    double X[4][3], dx[4], dy[4], dz[4];
-    load_xyz4(d, d.conn[e], X);
-    shape_fn(X, d.vol[e], dx, dy, dz);
-    store_shp(d, e, dx, dy, dz);
-}
-
-// fields.cxx:478-529
-__global__ void k_rotate(Dev d)
-{
-    int e = gtid();
-    if (e >= d.nelem) return;
-    const size_t E = d.nelem;
-    double V[4][3], dx[4], dy[4], dz[4], w3, w4, w5, s[6];
-    load_vel4(d, d.conn[e], V);
-    load_shp(d, e, dx, dy, dz);
-    spin(V, dx, dy, dz, w3, w4, w5);
-    double dt = d.clk->dt;
-    load6(d.stress, E, e, s);
-    jaumann(s, dt, w3, w4, w5);
-    store6(d.stress, E, e, s);
-    load6(d.strain, E, e, s);
-    jaumann(s, dt, w3, w4, w5);
-    store6(d.strain, E, e, s);
 }
 
 // geometry.cxx:270-325
@@ -1010,89 +913,53 @@ __global__ void k_init_stress(Dev d)
 // fused passes
 // ===========================================================================
 
-// contributions for the next N-A pass from the current state: next strain
-// rate, tr(D) * volume, conduction vector
-// with the next step's strain rate D already formed
-__device__ __forceinline__ void next_step_contrib_d(const Dev &d, int e, int4 c, const double D[6],
-                                                    const double dx[4], const double dy[4],
-                                                    const double dz[4], double vol)
+// the nodal masses (geometry.cxx:370-381) from the element contributions
+// vol, m, t (E-A's, or compute_mass's in tmp[0..2]) on the FP64 unit: for a
+// node whose sums leave sf::PosSum's range
+static __device__ __noinline__ void node_masses_exact(const Dev &d, int q0, int q1, const double *vol, const double *m,
+                                                      const double *t, double out[3])
 {
-    const size_t E = d.nelem;
-    store6(d.srate_next, E, e, D);
-    d.c_trdv[e] = tr3(D) * vol;
-    if (d.K->thermal) {
-        double Tn[4], tr[4];
-        load_nodal4(d.T, c, Tn);
-        conduction(dx, dy, dz, Tn, d.K->M.mix[d.mix[e]].k * vol, tr);
-        for (int i = 0; i < 4; ++i) d.tmp[i * E + e] = tr[i];
-    }
-}
-
-__device__ __forceinline__ void next_step_contrib(const Dev &d, int e, int4 c, const double V[4][3],
-                                                  const double dx[4], const double dy[4],
-                                                  const double dz[4], double vol)
-{
-    double D[6];
-    strain_rate(V, dx, dy, dz, D);
-    next_step_contrib_d(d, e, c, D, dx, dy, dz, vol);
-}
-
-__global__ void k_prime(Dev d)
-{
-    int e = gtid();
-    if (e >= d.nelem) return;
-    int4 c = d.conn[e];
-    double V[4][3], dx[4], dy[4], dz[4];
-    load_vel4(d, c, V);
-    load_shp(d, e, dx, dy, dz);
-    next_step_contrib(d, e, c, V, dx, dy, dz, d.vol[e]);
-}
-
-// the nodal masses (geometry.cxx:370-381) from E-A's contributions on the FP64
-// unit: for a node whose sums leave sf::PosSum's range
-static __device__ __noinline__ void node_masses_exact(const Dev &d, int q0, int q1, double out[3])
-{
-    double vn = 0, m = 0, tm = 0;
+    double vn = 0, mn = 0, tn = 0;
     for (int q = q0; q < q1; ++q) {
         const size_t e = __ldg(d.sup_ent + q) >> 2;
-        vn += d.vol[e];
-        m += d.c_mass[e];
-        if (d.K->thermal) tm += d.c_tmass[e];
+        vn += vol[e];
+        mn += m[e];
+        if (d.K->thermal) tn += t[e];
     }
     out[0] = vn;
-    out[1] = m;
-    out[2] = tm;
+    out[1] = mn;
+    out[2] = tn;
 }
 
 // the same as sums of positive numbers on the integer pipes
-__device__ __forceinline__ void node_masses(const Dev &d, int q0, int q1, double &vn, double &m, double &tm)
+__device__ __forceinline__ void node_masses(const Dev &d, int q0, int q1, const double *vol, const double *m,
+                                            const double *t, double out[3])
 {
     const bool thermal = d.K->thermal;
-    vn = m = tm = 0;
+    out[0] = out[1] = out[2] = 0;
     if (q0 == q1) return;
     const size_t e0 = __ldg(d.sup_ent + q0) >> 2;
-    sf::PosSum sv = sf::pos_first(d.vol[e0]), sm = sf::pos_first(d.c_mass[e0]),
-               st = sf::pos_first(thermal ? d.c_tmass[e0] : 1.0);
+    sf::PosSum sv = sf::pos_first(vol[e0]), sm = sf::pos_first(m[e0]), st = sf::pos_first(thermal ? t[e0] : 1.0);
     walk<4>(
         d.sup_ent, q0 + 1, q1,
         [&](unsigned p) {
             const size_t e = p >> 2;
-            return Three<double>{d.vol[e], d.c_mass[e], thermal ? d.c_tmass[e] : 1.0};
+            return Three<double>{vol[e], m[e], thermal ? t[e] : 1.0};
         },
-        [&](const Three<double> &t) {
-            sf::pos_add(sv, t.x);
-            sf::pos_add(sm, t.y);
-            sf::pos_add(st, t.z);
+        [&](const Three<double> &w) {
+            sf::pos_add(sv, w.x);
+            sf::pos_add(sm, w.y);
+            sf::pos_add(st, w.z);
         });
-    vn = sf::value(sv);
-    m = sf::value(sm);
-    tm = thermal ? sf::value(st) : 0.0;
+    out[0] = sf::value(sv);
+    out[1] = sf::value(sm);
+    out[2] = thermal ? sf::value(st) : 0.0;
     if (!(sf::exact(sv) && sf::exact(sm) && sf::exact(st))) {
         double r[3];
-        node_masses_exact(d, q0, q1, r);
-        vn = r[0];
-        m = r[1];
-        tm = r[2];
+        node_masses_exact(d, q0, q1, vol, m, t, r);
+        out[0] = r[0];
+        out[1] = r[1];
+        out[2] = r[2];
     }
 }
 
@@ -1121,11 +988,11 @@ __global__ void __launch_bounds__(256, 4) k_fn_a(Dev d)
         vn = d.vol_n[n];
         tm = d.tmass[n];
     } else {
-        double m;
-        node_masses(d, q0, q1, vn, m, tm);
-        d.vol_n[n] = vn;
-        d.mass[n] = m;
-        d.tmass[n] = tm;
+        double w[3];
+        node_masses(d, q0, q1, d.vol, d.c_mass, d.c_tmass, w);
+        d.vol_n[n] = vn = w[0];
+        d.mass[n] = w[1];
+        d.tmass[n] = tm = w[2];
     }
     if (K.thermal) {
         double tdot = 0;
@@ -1236,21 +1103,9 @@ __global__ void k_fn_c(Dev d)
     int n = gtid();
     if (n >= d.nnode) return;
     const Consts &K = *d.K;
-    const int q0 = d.sup_off[n], q1 = d.sup_off[n + 1];
     const double dt = d.clk->dt;
-    double f[3] = {0, 0, 0};
-    const size_t E = d.nelem;
-    walk<4>(
-        d.sup_ent, q0, q1,
-        [&](unsigned p) {
-            const double *t = d.tmp + (size_t)(p & 3u) * E + (p >> 2);
-            return Three<double>{t[0], t[4 * E], t[8 * E]};
-        },
-        [&](const Three<double> &t) {
-            f[0] -= t.x;
-            f[1] -= t.y;
-            f[2] -= t.z;
-        });
+    double f[3];
+    force_gather(d, n, f);
     stress_bc_node(K, d.bf, n, d.bcflag[n], d.z[n], d.z0[n], f);
     double v[3] = {d.vx[n], d.vy[n], d.vz[n]};
     if (K.is_qs) {
@@ -1261,17 +1116,7 @@ __global__ void k_fn_c(Dev d)
     d.fx[n] = f[0];
     d.fy[n] = f[1];
     d.fz[n] = f[2];
-    // v += dt f / m: one reciprocal of m on the integer pipes for the three
-    const double m = d.mass[n];
-    uint32_t far = 0;
-    const sf::Den dm = sf::denominator(m, far);
-    for (int j = 0; j < 3; ++j) {
-        const double a = sf::mul(dt, f[j]);
-        uint32_t fa = far;
-        double q = sf::quotient(a, dm, fa);
-        if (!sf::in_range(fa)) q = sf::div_slow(a, m);
-        v[j] += q;
-    }
+    velocity_step(f, dt, d.mass[n], v);
     vbc_node(K, d.bcflag[n], v);
     d.vx[n] = v[0];
     d.vy[n] = v[1];
@@ -1284,23 +1129,18 @@ __global__ void k_fn_c(Dev d)
     if (not_finite(x) || not_finite(y) || not_finite(z)) atomicOr(&d.clk->status, 0x2u);
 }
 
-// nodal masses from the fused-pass contributions (used before a download)
-__global__ void k_mass_flush(Dev d)
+// compute_mass's node half, from E-A's contributions (before the masses are
+// read) or from tmp[0..2]
+__global__ void __launch_bounds__(256, 4) k_mass_node(Dev d, const double *vol, const double *m, const double *t)
 {
     int n = gtid();
     if (n == 0) d.clk->mass_valid = 1;
     if (n >= d.nnode) return;
-    const bool thermal = d.K->thermal;
-    double vn = 0, m = 0, tm = 0;
-    for (int q = d.sup_off[n]; q < d.sup_off[n + 1]; ++q) {
-        size_t e = __ldg(d.sup_ent + q) >> 2;
-        vn += d.vol[e];
-        m += d.c_mass[e];
-        if (thermal) tm += d.c_tmass[e];
-    }
-    d.vol_n[n] = vn;
-    d.mass[n] = m;
-    d.tmass[n] = tm;
+    double w[3];
+    node_masses(d, d.sup_off[n], d.sup_off[n + 1], vol, m, t, w);
+    d.vol_n[n] = w[0];
+    d.mass[n] = w[1];
+    d.tmass[n] = w[2];
 }
 
 // ---- layout conversion ----------------------------------------------------
@@ -1413,10 +1253,6 @@ __global__ void k_clock_set(Clock *clk, double time, double dt, int steps, int m
         clk->steps = steps;
         clk->mass_valid = mass_valid;
     }
-}
-__global__ void k_clock_mass_valid(Clock *clk, int v)
-{
-    if (threadIdx.x == 0 && blockIdx.x == 0) clk->mass_valid = v;
 }
 __global__ void k_clock_dt(Clock *clk, double dt)
 {

@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(kSmallBlock) k_ea_quad(Dev d, int e0, unsigned
             const unsigned bad = __ballot_sync(0xffffffffu, !sf::in_range(far));
             if (!live) continue;
             if ((bad >> (base & 31)) & 15u) {
-                if (i == 0) ea_rotate_exact(d, e, arr, 0.5 * u[0], 0.5 * u[1], 0.5 * u[2]);
+                if (i == 0) ea_rotate_exact(d, e, arr, step_dt, 0.5 * u[0], 0.5 * u[1], 0.5 * u[2]);
             } else if (i < 3) {
                 arr[kk * E + e] = sn;
                 arr[(3 + kk) * E + e] = so;
