@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(kNnListBlock) kf_nn_list(DevF d, const MlpDev 
 
 // E-B3: the exact FP64 return map over a list
 template <int RHEOL>
-__global__ void kf_exact_list(DevF d, int from_pending)
+__global__ void __launch_bounds__(128, 5) kf_exact_list(DevF d, int from_pending)
 {
     const unsigned n = from_pending ? d.clk->npend : d.clk->nexact;
     const int *list = from_pending ? d.pend : d.exact;

@@ -65,8 +65,8 @@ struct MatTable {
     Mix    mix[kMaxMix];
 };
 
-__device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
-__device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
+__device__ __forceinline__ double smin(double a, double b) { return sf::less(b, a) ? b : a; }
+__device__ __forceinline__ double smax(double a, double b) { return sf::less(a, b) ? b : a; }
 // The templated helpers below are instantiated with double for the FP64 form
 // (identical operation order to the reference) and with float for the FP32
 // form; literals are cast to R so that a float instantiation stays in FP32.
@@ -166,7 +166,7 @@ __device__ __forceinline__ double mat_visc(const MatTable &M, const Mix &x, doub
 {
     if (const int c = visc_clipped(M, x, T, srate))
         return c > 0 ? smin(smax(M.visc_max, M.visc_min), M.visc_max) : smin(M.visc_min, M.visc_max);
-    double edot = sqrt(second_invariant2(srate));
+    double edot = sf::root(second_invariant2(srate));
     edot = smax(edot, 1e-30);
     const bool skip = x.single >= 0 || (M.visc_plain && T > 0 && edot <= 1e30);
     const int terms = skip ? x.npresent : M.nmat;
@@ -194,16 +194,16 @@ __device__ __forceinline__ void plastic_props(const MatTable &M, const Mix &x, d
     if (x.single >= 0) {
         // one material, power-of-two count: (v * k) / k == v
         int m = x.single;
-        if (pls < M.pls0[m]) {
+        if (sf::less(pls, M.pls0[m])) {
             cohesion = M.c0[m];
             phi = M.f0[m];
             psi = M.d0[m];
             hardn = 0;
-        } else if (pls < M.pls1[m]) {
-            double p = (pls - M.pls0[m]) / (M.pls1[m] - M.pls0[m]);
-            cohesion = M.c0[m] + p * (M.c1[m] - M.c0[m]);
-            phi = M.f0[m] + p * (M.f1[m] - M.f0[m]);
-            psi = M.d0[m] + p * (M.d1[m] - M.d0[m]);
+        } else if (sf::less(pls, M.pls1[m])) {
+            double p = sf::div(pls - M.pls0[m], M.pls1[m] - M.pls0[m]);
+            cohesion = M.c0[m] + sf::mul(p, M.c1[m] - M.c0[m]);
+            phi = M.f0[m] + sf::mul(p, M.f1[m] - M.f0[m]);
+            psi = M.d0[m] + sf::mul(p, M.d1[m] - M.d0[m]);
             hardn = M.hslope[m];
         } else {
             cohesion = M.c1[m];
@@ -218,13 +218,13 @@ __device__ __forceinline__ void plastic_props(const MatTable &M, const Mix &x, d
             int k = x.count[m];
             if (k == 0) continue;
             n += k;
-            if (pls < M.pls0[m]) {
+            if (sf::less(pls, M.pls0[m])) {
                 c += M.c0[m] * k;
                 f += M.f0[m] * k;
                 d += M.d0[m] * k;
                 h += 0;
-            } else if (pls < M.pls1[m]) {
-                double p = (pls - M.pls0[m]) / (M.pls1[m] - M.pls0[m]);
+            } else if (sf::less(pls, M.pls1[m])) {
+                double p = sf::div(pls - M.pls0[m], M.pls1[m] - M.pls0[m]);
                 c += (M.c0[m] + p * (M.c1[m] - M.c0[m])) * k;
                 f += (M.f0[m] + p * (M.f1[m] - M.f0[m])) * k;
                 d += (M.d0[m] + p * (M.d1[m] - M.d0[m])) * k;
@@ -251,21 +251,22 @@ __device__ __forceinline__ void plastic_props(const MatTable &M, const Mix &x, d
         sqanphi = M.sqanphi_w;
         tphi = M.tphi_w;
     } else {
-        double sphi = sin(phi * kDeg2Rad);
-        anphi = (1 + sphi) / (1 - sphi);
-        sqanphi = sqrt(anphi);
-        tphi = tan(phi * kDeg2Rad);
+        const double a = sf::mul(phi, kDeg2Rad);
+        double sphi = sin(a);
+        anphi = sf::div(1 + sphi, 1 - sphi);
+        sqanphi = sf::root(anphi);
+        tphi = tan(a);
     }
     if (psi == M.psi_c) {
         anpsi = M.anpsi_c;
     } else if (psi == M.psi_w) {
         anpsi = M.anpsi_w;
     } else {
-        double spsi = sin(psi * kDeg2Rad);
-        anpsi = (1 + spsi) / (1 - spsi);
+        double spsi = sin(sf::mul(psi, kDeg2Rad));
+        anpsi = sf::div(1 + spsi, 1 - spsi);
     }
-    amc = 2 * cohesion * sqanphi;
-    ten_max = (phi == 0) ? M.tension_max : smin(M.tension_max, cohesion / tphi);
+    amc = sf::mul(sf::twice(cohesion), sqanphi);
+    ten_max = (phi == 0) ? M.tension_max : smin(M.tension_max, sf::div(cohesion, tphi));
 }
 
 // ---- 3x3 symmetric eigen-solver -------------------------------------------
@@ -290,9 +291,9 @@ __device__ __forceinline__ void eig_cardano(const double *A, double w[3])
     double c0 = mul(a22, dd) + mul(a00, ee) + mul(a11, ff) - mul(mul(a00, a11), a22) - mul(mul(2.0, a02), de);
     double p = mul(m, m) - mul(3.0, c1);
     double q = mul(m, p - mul(3.0 / 2.0, c1)) - mul(27.0 / 2.0, c0);
-    double sqrt_p = sqrt(fabs(p));
+    double sqrt_p = sf::root(fabs(p));
     double phi = mul(27.0, mul(mul(0.25, mul(c1, c1)), p - c1) + mul(c0, q + mul(27.0 / 4.0, c0)));
-    phi = mul(1.0 / 3.0, atan2(sqrt(fabs(phi)), q));
+    phi = mul(1.0 / 3.0, atan2(sf::root(fabs(phi)), q));
     double sp, cp;
     sincos(phi, &sp, &cp);
     double c = mul(sqrt_p, cp);
@@ -412,9 +413,9 @@ __device__ __forceinline__ int eig_hybrid(const double *A, double Q[3][3], doubl
     using sf::mul;
     eig_cardano(A, w);
     t = fabs(w[0]);
-    if ((u = fabs(w[1])) > t) t = u;
-    if ((u = fabs(w[2])) > t) t = u;
-    if (t < 1.0)
+    if (sf::less(t, u = fabs(w[1]))) t = u;
+    if (sf::less(t, u = fabs(w[2]))) t = u;
+    if (sf::less(t, 1.0))
         u = t;
     else
         u = mul(t, t);
@@ -426,15 +427,15 @@ __device__ __forceinline__ int eig_hybrid(const double *A, double Q[3][3], doubl
     Q[1][0] = q11 + mul(a12, w[0]);
     Q[2][0] = mul(a00 - w[0], a11 - w[0]) - q21;
     norm = mul(Q[0][0], Q[0][0]) + mul(Q[1][0], Q[1][0]) + mul(Q[2][0], Q[2][0]);
-    if (norm <= error) return eig_ql(A, Q, w) == 0 ? 1 : -1;
-    norm = sqrt(1.0 / norm);
+    if (sf::less(norm, error) || norm == error) return eig_ql(A, Q, w) == 0 ? 1 : -1;
+    norm = sf::root(sf::div(1.0, norm));
     for (int j = 0; j < 3; j++) Q[j][0] = mul(Q[j][0], norm);
     Q[0][1] = q01 + mul(a02, w[1]);
     Q[1][1] = q11 + mul(a12, w[1]);
     Q[2][1] = mul(a00 - w[1], a11 - w[1]) - q21;
     norm = mul(Q[0][1], Q[0][1]) + mul(Q[1][1], Q[1][1]) + mul(Q[2][1], Q[2][1]);
-    if (norm <= error) return eig_ql(A, Q, w) == 0 ? 1 : -1;
-    norm = sqrt(1.0 / norm);
+    if (sf::less(norm, error) || norm == error) return eig_ql(A, Q, w) == 0 ? 1 : -1;
+    norm = sf::root(sf::div(1.0, norm));
     for (int j = 0; j < 3; j++) Q[j][1] = mul(Q[j][1], norm);
     Q[0][2] = mul(Q[1][0], Q[2][1]) - mul(Q[2][0], Q[1][1]);
     Q[1][2] = mul(Q[2][0], Q[0][1]) - mul(Q[0][0], Q[2][1]);
@@ -457,9 +458,9 @@ __device__ __forceinline__ int principal3(const double *s, double p[3], double v
             v[r][j] = bb;                                    \
         }                                                    \
     }
-    if (p[0] > p[1]) DES_SWAP_COL(0, 1)
-    if (p[1] > p[2]) DES_SWAP_COL(1, 2)
-    if (p[0] > p[1]) DES_SWAP_COL(0, 1)
+    if (sf::less(p[1], p[0])) DES_SWAP_COL(0, 1)
+    if (sf::less(p[2], p[1])) DES_SWAP_COL(1, 2)
+    if (sf::less(p[1], p[0])) DES_SWAP_COL(0, 1)
 #undef DES_SWAP_COL
     return rc;
 }
@@ -519,15 +520,17 @@ __device__ __forceinline__ void viscous(R bulkm, R viscosity, R total_dv, const 
 __device__ __forceinline__ bool surely_elastic(const double *s, double anphi, double amc,
                                                double ten_max)
 {
-    double m = (s[0] + s[1] + s[2]) * (1.0 / 3.0);
-    double a = s[0] - m, b = s[1] - m, c = s[2] - m;
-    double dev2 = a * a + b * b + c * c + 2.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5]);
-    double R = sqrt(dev2 * (2.0 / 3.0)) * (1.0 + 1e-12);
-    double scale = fabs(m) + R;
-    double margin = 1e-6 * scale * (1.0 + anphi) + 1e-300;
-    double fs_lo = (m - R) - anphi * (m + R) + amc;
-    double ft_hi = (m + R) - ten_max;
-    return fs_lo > margin && ft_hi < -margin;
+    using sf::mul;
+    const double m = mul(s[0] + s[1] + s[2], 1.0 / 3.0);
+    const double a = s[0] - m, b = s[1] - m, c = s[2] - m;
+    const double dev2 = mul(a, a) + mul(b, b) + mul(c, c) +
+                        sf::twice(mul(s[3], s[3]) + mul(s[4], s[4]) + mul(s[5], s[5]));
+    const double R = mul(sf::root(mul(dev2, 2.0 / 3.0)), 1.0 + 1e-12);
+    const double hi = m + R;
+    const double margin = mul(mul(1e-6, fabs(m) + R), 1.0 + anphi) + 1e-300;
+    const double fs_lo = (m - R) - mul(anphi, hi) + amc;
+    const double ft_hi = hi - ten_max;
+    return sf::less(margin, fs_lo) && sf::less(ft_hi, -margin);
 }
 
 // The same bound in FP32 from FP32 plastic properties, before any FP64 work on
@@ -600,32 +603,35 @@ __device__ __forceinline__ int plastic_return(double bulkm, double shearm, doubl
     double v[3][3];
     int rc = principal3(s, p, v);
     int flags = 1 | (rc == 1 ? 2 : 0) | (rc < 0 ? 6 : 0);
-    double fs = p[0] - p[2] * anphi + amc;
+    // (products, quotients, roots and comparisons on the integer pipes)
+    using sf::mul;
+    const double zero = 0;
+    double fs = p[0] - mul(p[2], anphi) + amc;
     double ft = p[2] - ten_max;
-    if (fs > 0 && ft < 0) return flags;
-    double pa = sqrt(1 + anphi * anphi) + anphi;
-    double ps = ten_max * anphi - amc;
-    double h = p[2] - ten_max + pa * (p[0] - ps);
-    double a1 = bulkm + 4. / 3 * shearm;
-    double a2 = bulkm - 2. / 3 * shearm;
+    if (sf::less(zero, fs) && sf::less(ft, zero)) return flags;
+    double pa = sf::root(1 + mul(anphi, anphi)) + anphi;
+    double ps = mul(ten_max, anphi) - amc;
+    double h = p[2] - ten_max + mul(pa, p[0] - ps);
+    double a1 = bulkm + mul(4. / 3, shearm);
+    double a2 = bulkm - mul(2. / 3, shearm);
     double alam;
-    if (h < 0) {
+    if (sf::less(h, zero)) {
         flags |= 16;
-        alam = fs / (a1 - a2 * anpsi + a1 * anphi * anpsi - a2 * anphi + 2 * sqrt(anphi) * hardn);
-        p[0] -= alam * (a1 - a2 * anpsi);
-        p[1] -= alam * (a2 - a2 * anpsi);
-        p[2] -= alam * (a2 - a1 * anpsi);
-        depls = fabs(alam) * sqrt((7 + 4 * anpsi + 7 * anpsi * anpsi) / 18);
+        const double a1psi = mul(a1, anpsi), a2psi = mul(a2, anpsi);
+        alam = sf::div(fs, a1 - a2psi + mul(mul(a1, anphi), anpsi) - mul(a2, anphi) +
+                               mul(sf::twice(sf::root(anphi)), hardn));
+        p[0] -= mul(alam, a1 - a2psi);
+        p[1] -= mul(alam, a2 - a2psi);
+        p[2] -= mul(alam, a2 - a1psi);
+        depls = mul(fabs(alam), sf::root(sf::div(7 + mul(4.0, anpsi) + mul(mul(7.0, anpsi), anpsi), 18.0)));
     } else {
         flags |= 32;
-        alam = ft / a1;
-        p[0] -= alam * a2;
-        p[1] -= alam * a2;
-        p[2] -= alam * a1;
-        depls = fabs(alam) * sqrt(7. / 18);
+        alam = sf::div(ft, a1);
+        p[0] -= mul(alam, a2);
+        p[1] -= mul(alam, a2);
+        p[2] -= mul(alam, a1);
+        depls = mul(fabs(alam), sqrt(7. / 18));
     }
-    // (the reconstruction's products on the integer pipes, sf::mul)
-    using sf::mul;
     double ss00 = 0, ss11 = 0, ss22 = 0, ss01 = 0, ss02 = 0, ss12 = 0;
     for (int k = 0; k < 3; k++) {
         ss00 += mul(mul(v[0][k], v[0][k]), p[k]);

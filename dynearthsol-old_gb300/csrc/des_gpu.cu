@@ -859,7 +859,7 @@ __device__ __forceinline__ unsigned long long check_mix(unsigned long long z)
     return z ^ (z >> 31);
 }
 
-// sf::mul, sf::div, sf::to_float, sf::add0, sf::twice, sf::half, sf::div6, sf::div3
+// sf::mul, sf::div, sf::root, sf::to_float, sf::add0, sf::twice, sf::half, sf::div6, sf::div3
 // and sf::quarter against the FP64 unit's multiply, conversion, addition and
 // division
 __global__ void k_softf64_check(unsigned long long *bad, long long n, unsigned long long seed)
@@ -883,6 +883,10 @@ __global__ void k_softf64_check(unsigned long long *bad, long long n, unsigned l
         g = sf::mul(x1, y1);
         nb[1] += sf::bits(h) != sf::bits(g);
         h = __ddiv_rn(x1, y1), g = sf::div(x1, y1);
+        nb[1] += sf::bits(h) != sf::bits(g);
+        h = __dsqrt_rn(x), g = sf::root(x);
+        nb[0] += sf::bits(h) != sf::bits(g) && !(h != h && g != g);
+        h = __dsqrt_rn(fabs(x1)), g = sf::root(fabs(x1));
         nb[1] += sf::bits(h) != sf::bits(g);
         float hf = __double2float_rn(x), gf = sf::to_float(x);
         nb[2] += __float_as_uint(hf) != __float_as_uint(gf) && !(hf != hf && gf != gf);

@@ -17,6 +17,7 @@
 // The header compiles as plain C++ too, so that the host can check it
 // against its own IEEE arithmetic.
 #pragma once
+#include <math.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -264,6 +265,15 @@ DES_SF_HD double mul(double x, double y)
     return from_bits(mul_slow(bits(x), bits(y)));
 }
 
+// a < b (an FP64 comparison occupies the FP64 pipe like an addition)
+DES_SF_HD bool less(double a, double b)
+{
+    const uint64_t x = bits(a), y = bits(b), mx = x & kAbs, my = y & kAbs;
+    // a zero's sign does not count; NaN compares false
+    const int64_t kx = (x >> 63) ? -(int64_t)mx : (int64_t)mx, ky = (y >> 63) ? -(int64_t)my : (int64_t)my;
+    return kx < ky && mx <= kInf && my <= kInf;
+}
+
 // ---- quotients ----------------------------------------------------------------
 // The FP64 unit's division takes about nine FP64 instructions; on the integer
 // pipes the reciprocal of the denominator's significand comes from an FP32
@@ -350,6 +360,56 @@ DES_SF_HD double div(double x, double y)
     const Den d = denominator(y, far);
     const double q = quotient(x, d, far);
     return in_range(far) ? q : div_slow(x, y);
+}
+
+// ---- square root -----------------------------------------------------------------
+
+#if defined(__CUDACC__)
+static __host__ __device__ __noinline__
+#else
+static
+#endif
+double root_slow(double x) { return ::sqrt(x); }
+
+// about 2^32 / sqrt(a) for a in [1, 4) given as an FP32 number, in (2^31, 2^32)
+DES_SF_HD uint32_t rsqrt_seed(uint32_t fbits)
+{
+#if defined(__CUDA_ARCH__)
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(float_from_bits(fbits)));
+    uint32_t b = __float_as_uint(r);
+#else
+    const float r = 1.0f / ::sqrtf(float_from_bits(fbits));
+    uint32_t b;
+    memcpy(&b, &r, 4);
+#endif
+    b = b > 0x3f000000u ? b : 0x3f000000u;
+    return b >= 0x3f800000u ? 0xffffffffu : ((b & 0x7fffffu) | 0x800000u) << 8;
+}
+
+// sqrt(x) as the FP64 unit rounds it (about 18 FP64 instructions there): with
+// a in [1, 4) and an even exponent, an FP32 reciprocal root and two steps of
+// g += (a - g g) / (2 sqrt(a)) in 62-bit fixed point, then the exact remainder
+// of the nearest 53-bit candidate, which is at most one off.  A root is never
+// half way between two 53-bit numbers.
+DES_SF_HD double root(double x)
+{
+    const uint64_t v = bits(x);
+    const uint32_t h = (uint32_t)(v >> 32);
+    if (!(h - (1u << 20) < (2046u << 20))) return root_slow(x);      // zero, subnormal, negative, infinity, NaN
+    const uint32_t e = h >> 20, odd = (e & 1) ^ 1;                   // biased 1023 is even in effect
+    const uint64_t A = ((v & kFrac) | kHidden) << (10 + odd);        // a 2^62
+    const uint32_t y = rsqrt_seed((0x3f800000u + (odd << 23)) | ((uint32_t)(v >> 29) & 0x7fffffu));
+    uint64_t g = wide_mad((uint32_t)(A >> 32), y, wide_mul((uint32_t)A, y) >> 32);
+    const int32_t r0 = (int32_t)((int64_t)((A >> 2) - mulhi64(g, g)) >> 12);
+    g += (uint64_t)(((int64_t)r0 * (int64_t)y) >> 19);
+    const int32_t r1 = (int32_t)((A >> 2) - mulhi64(g, g));
+    g += (uint64_t)(((int64_t)r1 * (int64_t)y) >> 31);
+    uint64_t s = (g + 512) >> 10;
+    const int64_t r = (int64_t)((A << 42) - s * s);
+    s += (uint64_t)(r > (int64_t)s) - (uint64_t)(r <= -(int64_t)s);
+    const uint64_t ex = (uint64_t)((e + 1023 - odd) >> 1) - 1;
+    return from_bits((ex << 52) + s);
 }
 
 // ---- sums of positive numbers ---------------------------------------------------

@@ -524,9 +524,9 @@ int         des_gpu_kernels_per_step(const des_gpu *g);
 /* Self-check of the integer-pipe FP64 arithmetic that the step kernels use
  * in place of FP64 unit instructions (no reference counterpart): n seeded
  * pseudo-random operands per kind on `device`, compared bit for bit with the
- * device's own FP64 instructions.  mismatches[0..9]: multiply and divide on any
- * bit patterns, multiply and divide on operands near 1, conversion to FP32 on any bit
- * patterns, conversion within the FP32 range, 0 + x, 2 x, x / 2, x / 6,
+ * device's own FP64 instructions.  mismatches[0..9]: multiply, divide and
+ * square root on any bit patterns, the same on operands near 1, conversion to
+ * FP32 on any bit patterns, conversion within the FP32 range, 0 + x, 2 x, x / 2, x / 6,
  * x / 3, x / 4 (the last six on any bit patterns and on exponents 0-8). */
 int         des_gpu_softf64_check(int device, long long n, unsigned long long seed,
                                   unsigned long long mismatches[10]);

@@ -1,5 +1,6 @@
 // Host check of the grouped integer-pipe product (unpack, prod, in_range), the
-// quotient (div), the running
+// quotient (div), the square
+// root (root), the comparison (less), the running
 // sum of positive numbers (PosSum) and the FP32 -> FP64 conversion (widen) of dynearthsol-old_gb300/csrc/des_softf64.cuh against the
 // host's IEEE arithmetic, bit for bit.
 //   softf64_ops_check <pairs per kind>  -> one line per kind; exit 1 on a mismatch
@@ -73,6 +74,9 @@ int main(int argc, char **argv)
                 bad += bits(m) != bits(prod(a, b));
             }
             bad += !same(q, div(x, y));
+            const double sq = std::sqrt(vx);
+            bad += !same(sq, root(x));
+            bad += less(x, y) != (vx < vy);
         }
         // the range itself: kinds 0 and 4 lie inside it, kind 3's infinities never do
         if ((kind == 0 || kind == 4) && grouped != per) ++bad;
