@@ -384,8 +384,10 @@ static __device__ __noinline__ void ea_conduction_exact(const Dev &d, int e, dou
 // (gradNi.gradNj) T_j.  gradNi.gradNj and gradNj.gradNi round
 // identically (the products commute and are summed in the same
 // order), so the 10 distinct dot products are formed once: those of
-// pairs go through shared memory, a node's own stays in its row.  Integer ALU
-// 74 %, FP64 pipe 65 % busy.
+// pairs go through shared memory, a node's own stays in its row.  The rows
+// are unrolled (190 -> 174 us for 2.4M elements; the pairs too: 175; the other
+// kernels' loops over nodes unrolled: geometry 229 -> 289, E-C 212 -> 259, for
+// the spills and the longer code).
 template <bool SOFT, int BLK, int MINB>
 __global__ void __launch_bounds__(BLK, MINB) k_ea_conduction(Dev d, int e0)
 {
@@ -419,7 +421,7 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_conduction(Dev d, int e0)
     Op oT[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) oT[j] = N::op(Tn[j], far);
-#pragma unroll 1
+#pragma unroll
     for (int i = 0; i < 4; ++i) {
         // the pair number of (i, j), j = 0..3 (the diagonal's nibble unused)
         const unsigned pairs = i == 0 ? 0x2100u : i == 1 ? 0x4300u : i == 2 ? 0x5031u : 0x0542u;
