@@ -132,6 +132,66 @@ int read_err(const int *derr)
     return e ? DES_ERR_CUDA : DES_OK;
 }
 
+// Rows of the caller's as a kernel reads or writes them: in place where the
+// GPU reaches any host memory through the host's page tables (GB300 over
+// NVLink-C2C) and the rows are 16-byte aligned, else through a device copy.
+// In place, 250k samples' rows cross the link under the kernel, where a device
+// copy had its own allocation, transfer and release (with one kept Call, below:
+// forward 700 -> 355 us, 135 of it the caller's fresh output pages; loss and
+// gradient 700 -> 238 us; both 200 -> 57 us on 256 samples).
+struct Rows {
+    DevBuf buf;
+    float *p = nullptr;
+    bool host = false;
+    int open(const float *rows, size_t bytes, bool copy_in)
+    {
+        int dev = 0, ats = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&ats, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev);
+        host = ats && reinterpret_cast<uintptr_t>(rows) % 16 == 0;
+        if (host) {
+            p = const_cast<float *>(rows);
+            return DES_OK;
+        }
+        if (buf.alloc(bytes)) return DES_ERR_NOMEM;
+        p = buf.as<float>();
+        if (copy_in && cudaMemcpy(p, rows, bytes, cudaMemcpyHostToDevice) != cudaSuccess) return DES_ERR_CUDA;
+        return DES_OK;
+    }
+};
+
+// The small device data of one call, one allocation and one copy each way:
+// parameters, gradient, loss, the kernels' time-out flag (the last three zero)
+struct Call {
+    float params[kNParams], grad[kNParams];
+    double loss;
+    int err;
+};
+
+// A thread's Call on the current device, kept between its calls (48 KB; a
+// cudaMalloc and cudaFree of a small block map and unmap 2 MB each time, about
+// 100 us a call) and released when the thread ends.  Every call waits for its
+// work, so the thread's next one finds it free; one that a device reset took
+// away is allocated anew.
+struct CallBuf {
+    Call *p = nullptr;
+    ~CallBuf() { if (p) cudaFree(p); }
+    Call *get()
+    {
+        int dev = 0;
+        cudaPointerAttributes a;
+        if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+        if (p && cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeDevice) {
+            if (a.device == dev) return p;
+            cudaFree(p);
+        }
+        cudaGetLastError();
+        p = nullptr;
+        return cudaMalloc(&p, sizeof(Call)) == cudaSuccess ? p : p = nullptr;
+    }
+};
+thread_local CallBuf call_buf;
+
 }  // namespace
 
 extern "C" {
@@ -139,55 +199,51 @@ extern "C" {
 int des_mlp_forward(const des_mlp *net, const float *x, long long n, float *y)
 {
     if (!net || !x || !y || n < 1) return DES_ERR_ARG;
+    std::vector<Call> h(1);
     std::vector<float> P;
     pack(*net, P);
-    DevBuf dP, dx, dy, de;
-    if (dP.alloc(sizeof(float) * kNParams) || dx.alloc(sizeof(float) * n * kMlpIn) ||
-        dy.alloc(sizeof(float) * n * kMlpOut) || de.alloc(sizeof(int)))
-        return DES_ERR_NOMEM;
+    std::memcpy(h[0].params, P.data(), sizeof(h[0].params));
+    Rows rx, ry;
+    int rc;
+    Call *c = call_buf.get();
+    if (!c) return DES_ERR_NOMEM;
+    if ((rc = rx.open(x, sizeof(float) * n * kMlpIn, true)) || (rc = ry.open(y, sizeof(float) * n * kMlpOut, false)))
+        return rc;
     if (smem_setup((const void *)k_mlp_forward)) return DES_ERR_CUDA;
-    if (cudaMemcpy(dP.p, P.data(), sizeof(float) * kNParams, cudaMemcpyHostToDevice) ||
-        cudaMemcpy(dx.p, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice) ||
-        cudaMemset(de.p, 0, sizeof(int)))
-        return DES_ERR_CUDA;
+    if (cudaMemcpy(c, h.data(), sizeof(Call), cudaMemcpyHostToDevice)) return DES_ERR_CUDA;
     const int grid = tile_grid((n + kTile - 1) / kTile);
-    k_mlp_forward<<<grid, kTcRows, kMlpTcSmemBytes>>>(dP.as<float>(), dx.as<float>(), n, dy.as<float>(),
-                                                      de.as<int>());
+    k_mlp_forward<<<grid, kTcRows, kMlpTcSmemBytes>>>(c->params, rx.p, n, ry.p, &c->err);
     if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) return DES_ERR_CUDA;
-    if (int rc = read_err(de.as<int>())) return rc;
-    return cudaMemcpy(y, dy.p, sizeof(float) * n * kMlpOut, cudaMemcpyDeviceToHost) == cudaSuccess ? DES_OK
-                                                                                                    : DES_ERR_CUDA;
+    if ((rc = read_err(&c->err)) || ry.host) return rc;
+    return cudaMemcpy(y, ry.p, sizeof(float) * n * kMlpOut, cudaMemcpyDeviceToHost) == cudaSuccess ? DES_OK
+                                                                                                   : DES_ERR_CUDA;
 }
 
 int des_mlp_loss_grad(const des_mlp *net, const float *x, const float *y, long long n, double *loss,
                       des_mlp *grad)
 {
     if (!net || !x || !y || n < 1 || !loss || !grad) return DES_ERR_ARG;
+    std::vector<Call> h(1);
     std::vector<float> P;
     pack(*net, P);
-    DevBuf dP, dx, dy, dg, dl, de;
-    if (dP.alloc(sizeof(float) * kNParams) || dx.alloc(sizeof(float) * n * kMlpIn) ||
-        dy.alloc(sizeof(float) * n * kMlpOut) || dg.alloc(sizeof(float) * kNParams) || dl.alloc(sizeof(double)) ||
-        de.alloc(sizeof(int)))
-        return DES_ERR_NOMEM;
+    std::memcpy(h[0].params, P.data(), sizeof(h[0].params));
+    Rows rx, ry;
+    int rc;
+    Call *c = call_buf.get();
+    if (!c) return DES_ERR_NOMEM;
+    if ((rc = rx.open(x, sizeof(float) * n * kMlpIn, true)) || (rc = ry.open(y, sizeof(float) * n * kMlpOut, true)))
+        return rc;
     if (smem_setup((const void *)k_mlp_grad)) return DES_ERR_CUDA;
-    if (cudaMemcpy(dP.p, P.data(), sizeof(float) * kNParams, cudaMemcpyHostToDevice) ||
-        cudaMemcpy(dx.p, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice) ||
-        cudaMemcpy(dy.p, y, sizeof(float) * n * kMlpOut, cudaMemcpyHostToDevice) ||
-        cudaMemset(dg.p, 0, sizeof(float) * kNParams) || cudaMemset(dl.p, 0, sizeof(double)) ||
-        cudaMemset(de.p, 0, sizeof(int)))
-        return DES_ERR_CUDA;
+    if (cudaMemcpy(c, h.data(), sizeof(Call), cudaMemcpyHostToDevice)) return DES_ERR_CUDA;
     const long long ntiles = (n + kTile - 1) / kTile;
-    k_mlp_grad<<<tile_grid(ntiles), kTcRows, kMlpTcSmemBytes>>>(dP.as<float>(), dx.as<float>(), dy.as<float>(),
-                                                                n, 0, ntiles, 1.f / (float)n, dg.as<float>(), dl.as<double>(), de.as<int>());
-    if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) return DES_ERR_CUDA;
-    if (int rc = read_err(de.as<int>())) return rc;
-    std::vector<float> G(kNParams);
-    if (cudaMemcpy(G.data(), dg.p, sizeof(float) * kNParams, cudaMemcpyDeviceToHost) ||
-        cudaMemcpy(loss, dl.p, sizeof(double), cudaMemcpyDeviceToHost))
-        return DES_ERR_CUDA;
+    k_mlp_grad<<<tile_grid(ntiles), kTcRows, kMlpTcSmemBytes>>>(c->params, rx.p, ry.p, n, 0, ntiles, 1.f / (float)n,
+                                                                c->grad, &c->loss, &c->err);
+    if (cudaGetLastError() != cudaSuccess) return DES_ERR_CUDA;
+    if (cudaMemcpy(h.data(), c, sizeof(Call), cudaMemcpyDeviceToHost)) return DES_ERR_CUDA;
+    if (h[0].err) return DES_ERR_CUDA;
+    *loss = h[0].loss;
     std::memset(grad, 0, sizeof(*grad));
-    unpack(G, *grad);
+    unpack(std::vector<float>(h[0].grad, h[0].grad + kNParams), *grad);
     return DES_OK;
 }
 
