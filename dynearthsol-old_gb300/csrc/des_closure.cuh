@@ -164,7 +164,7 @@ __device__ __forceinline__ void f_trial_from_state(const DevF &d, int e, FTrial 
     f_load6(d.srate, E, e, edot);
     q.pls = d.pls[e];
     q.s0 = d.s0[e];
-    q.dt = (float)d.clk->dt;
+    q.dt = sf::to_float(d.clk->dt);
     for (int i = 0; i < 6; ++i) {
         q.de[i] = edot[i] * q.dt;
         q.s[i] = q.so[i];
@@ -218,10 +218,28 @@ __device__ __forceinline__ void list_append(unsigned *count, int *list, bool tak
     if (take) list[base + __popc(m & ((1u << lane) - 1u))] = e;
 }
 
+// the exact FP64 return map for one element after E-B1 has left its trial's
+// parts (strain and corrected strain rate new, stress old); returns eigen flags
+template <int RHEOL>
+static __device__ __noinline__ int f_exact_element(const DevF &d, int e)
+{
+    FTrial q;
+    f_trial_from_state<RHEOL>(d, e, q);
+    const Consts &K = *d.K;
+    float sp[6];
+    double depls;
+    const int flags = ep_fp64(K, K.M.mix[q.mix], q.pls, q.s0, q.so, q.de, sp, depls);
+    f_finish<RHEOL>(d, e, q, sp, depls, false);
+    return flags;
+}
+
 // E-B1, over the elements from e0 (a multiple of the block size); registers
 // bounded for 12 blocks of 128 per SM (E-B1 0.331 -> 0.317 ms on config 2)
-template <int RHEOL>
-__global__ void __launch_bounds__(128, 12) kf_fe_b_ep(DevF d, int e0)
+// (DIRECT: an undecided element takes its exact return here instead of
+// joining the list: on small meshes the list's kernel costs more, launch and
+// all, than the lanes that wait for it)
+template <int RHEOL, bool DIRECT>
+__global__ void __launch_bounds__(128, DIRECT ? 4 : 12) kf_fe_b_ep(DevF d, int e0)
 {
     const int e = e0 + gtid();
     const bool live = e < d.nelem;
@@ -285,7 +303,18 @@ __global__ void __launch_bounds__(128, 12) kf_fe_b_ep(DevF d, int e0)
             pending = true;
         }
     }
-    list_append(&d.clk->npend, d.pend, pending, e);
+    if (!DIRECT) {
+        list_append(&d.clk->npend, d.pend, pending, e);
+        return;
+    }
+    const int flags = pending ? f_exact_element<RHEOL>(d, e) : 0;
+    const unsigned solved = __ballot_sync(0xffffffffu, flags & 1), ql = __ballot_sync(0xffffffffu, flags & 2),
+                   ret = __ballot_sync(0xffffffffu, pending);
+    if ((threadIdx.x & 31) == 0) {
+        if (solved) atomicAdd(&d.clk->eig, (unsigned long long)__popc(solved));
+        if (ql) atomicAdd(&d.clk->ql, (unsigned long long)__popc(ql));
+        if (ret) atomicAdd(&d.clk->fp64_returns, (unsigned long long)__popc(ret));
+    }
 }
 
 constexpr int kNnListBlock = 128;
@@ -443,14 +472,7 @@ __global__ void __launch_bounds__(128, 5) kf_exact_list(DevF d, int from_pending
     const int *list = from_pending ? d.pend : d.exact;
     unsigned nsolved = 0, nql = 0, nret = 0;
     for (unsigned j = gtid(); j < n; j += gridDim.x * blockDim.x) {
-        const int e = list[j];
-        FTrial q;
-        f_trial_from_state<RHEOL>(d, e, q);
-        const Consts &K = *d.K;
-        float sp[6];
-        double depls;
-        const int flags = ep_fp64(K, K.M.mix[q.mix], q.pls, q.s0, q.so, q.de, sp, depls);
-        f_finish<RHEOL>(d, e, q, sp, depls, false);
+        const int flags = f_exact_element<RHEOL>(d, list[j]);
         nsolved += (flags & 1) ? 1u : 0u;
         nql += (flags & 2) ? 1u : 0u;
         ++nret;

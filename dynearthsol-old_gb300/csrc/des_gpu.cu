@@ -582,11 +582,15 @@ void launch_surface(des_gpu *g)
 // 27.6k, 46.2 / 42.2 at 54k; E-C 8.2 / 10.3, 12.3 / 12.3, 16.4 / 13.9.
 const int kOctetNodes[2][3] = {{128, 32, 90}, {200, 300, 96}};   // [FP64, FP32][N-A, N-B, N-C]
 const int kQuadElemsEa = 280, kQuadElemsEc = 180;
+// FP32 E-B with the exact returns in place / over the list: 9.6 / 13.4 at 27.7k elements, on yielding boxes 54.9 / 61.8 at
+// 14.4k, 61.9 / 64.4 at 54k, 119 / 80 at 240k
+const int kDirectReturns = 300;
 bool octets(const des_gpu *g, int pass)
 {
     return g->nnode <= kOctetNodes[g->prec == DES_PREC_FP32][pass] * g->sms;
 }
 bool quads_ea(const des_gpu *g) { return g->nelem <= kQuadElemsEa * g->sms; }
+bool direct_returns(const des_gpu *g) { return !g->closure && g->nelem <= kDirectReturns * g->sms; }
 bool quads_ec(const des_gpu *g) { return g->nelem <= kQuadElemsEc * g->sms; }
 
 // the first kernel of pass E-B over the element blocks [b0, b1)
@@ -594,10 +598,15 @@ void launch_eb_first(des_gpu *g, int b0, int b1)
 {
     const int n = b1 - b0, e0 = b0 * kElemBlock;
     if (g->prec == DES_PREC_FP32) {
-        if (g->hF.rheol == 7)
-            kf_fe_b_ep<7><<<n, kElemBlock, 0, g->stream>>>(g->f, e0);
+        const bool direct = direct_returns(g);
+        if (g->hF.rheol == 7 && direct)
+            kf_fe_b_ep<7, true><<<n, kElemBlock, 0, g->stream>>>(g->f, e0);
+        else if (g->hF.rheol == 7)
+            kf_fe_b_ep<7, false><<<n, kElemBlock, 0, g->stream>>>(g->f, e0);
+        else if (g->hF.rheol == 5 && direct)
+            kf_fe_b_ep<5, true><<<n, kElemBlock, 0, g->stream>>>(g->f, e0);
         else if (g->hF.rheol == 5)
-            kf_fe_b_ep<5><<<n, kElemBlock, 0, g->stream>>>(g->f, e0);
+            kf_fe_b_ep<5, false><<<n, kElemBlock, 0, g->stream>>>(g->f, e0);
         else
             kf_fe_b<<<n, kElemBlock, 0, g->stream>>>(g->f, e0);
     } else if (g->d.ret_log) {
@@ -616,7 +625,7 @@ void launch_eb_first(des_gpu *g, int b0, int b1)
 // exact return map, each over the dense list the first kernel left
 void launch_eb_rest(des_gpu *g)
 {
-    if (g->prec != DES_PREC_FP32 || (g->hF.rheol != 5 && g->hF.rheol != 7)) return;
+    if (g->prec != DES_PREC_FP32 || (g->hF.rheol != 5 && g->hF.rheol != 7) || direct_returns(g)) return;
     const DevF &f = g->f;
     const int nn_grid = 4 * g->sms, exact_grid = std::min(8 * g->sms, blocks(g->nelem, 128));
     if (g->hF.rheol == 7) {
@@ -1259,7 +1268,7 @@ int des_gpu_kernels_per_step(const des_gpu *g)
     if (g->P.surface_process_option == 1) n += g->d.bf.nbf > 0 ? 2 : 1;
     if (g->P.surface_process_option == 101) n += 1;
     // the FP32 form's elasto-plastic stress pass: the exact list, the network
-    if (g->prec == DES_PREC_FP32 && (g->hF.rheol == 5 || g->hF.rheol == 7)) n += g->closure ? 2 : 1;
+    if (g->prec == DES_PREC_FP32 && (g->hF.rheol == 5 || g->hF.rheol == 7)) n += g->closure ? 2 : direct_returns(g) ? 0 : 1;
     return n + (g->avg_interval > 0 ? 1 : 0);
 }
 
