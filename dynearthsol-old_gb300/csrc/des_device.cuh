@@ -87,7 +87,10 @@ __device__ __forceinline__ double pdiv3(double x) { return sf::div3(x); }
 __device__ __forceinline__ float pdiv3(float x) { return x / 3; }
 __device__ __forceinline__ double pmul(double a, double b) { return sf::mul(a, b); }
 __device__ __forceinline__ float pmul(float a, float b) { return a * b; }
-__device__ __forceinline__ double pdiv(double a, double b) { return sf::div(a, b); }
+// (the quotient as a call: inlined six times it made E-B of rh_evp wait for
+// instructions)
+static __device__ __noinline__ double div_call(double a, double b) { return sf::div(a, b); }
+__device__ __forceinline__ double pdiv(double a, double b) { return div_call(a, b); }
 __device__ __forceinline__ float pdiv(float a, float b) { return a / b; }
 
 // utils.hpp:78-87
@@ -121,13 +124,13 @@ __device__ __forceinline__ double mat_rho(const MatTable &M, const Mix &x, doubl
         int m = x.single;
         return sf::mul(M.rho0[m], 1 - sf::mul(M.alpha[m], TinCelsius));
     }
+    // (absent materials add +0)
     double result = 0;
-    int n = 0;
-    for (int m = 0; m < M.nmat; m++) {
-        result += M.rho0[m] * (1 - M.alpha[m] * TinCelsius) * x.count[m];
-        n += x.count[m];
+    for (int k = 0; k < x.npresent; k++) {
+        const int m = x.present[k];
+        result += sf::mul(sf::mul(M.rho0[m], 1 - sf::mul(M.alpha[m], TinCelsius)), (double)x.count[m]);
     }
-    return result / n;
+    return sf::div(result, (double)x.n);
 }
 
 // Whether mat_visc's value is certainly clipped: +1 at visc_max, -1 at

@@ -262,7 +262,7 @@ __device__ __forceinline__ int stress_body(const Dev &d, int e, int4 c, double e
         double Tn[4];
         load_nodal4(d.T, c, Tn);
         double viscosity = mat_visc(M, x, elem_mean4(Tn[0], Tn[1], Tn[2], Tn[3]), edot);
-        double dv = sf::div(d.vol[e], d.vol_old[e]) - 1;
+        double dv = pdiv(d.vol[e], d.vol_old[e]) - 1;
         maxwell(x.bulkm, x.shearm, viscosity, dt, dv, de, s);
     } break;
     case 5: { // elasto-plastic
@@ -281,7 +281,7 @@ __device__ __forceinline__ int stress_body(const Dev &d, int e, int4 c, double e
         double Tn[4];
         load_nodal4(d.T, c, Tn);
         double viscosity = mat_visc(M, x, elem_mean4(Tn[0], Tn[1], Tn[2], Tn[3]), edot);
-        double dv = sf::div(d.vol[e], d.vol_old[e]) - 1;
+        double dv = pdiv(d.vol[e], d.vol_old[e]) - 1;
         double sv[6];
         for (int i = 0; i < 6; ++i) sv[i] = s[i];
         maxwell(x.bulkm, x.shearm, viscosity, dt, dv, de, sv);
