@@ -39,6 +39,10 @@ struct Num<true> {
     using Op = sf::Op;
     __device__ __forceinline__ static Op op(double x, uint32_t &far) { return sf::unpack(x, far); }
     __device__ __forceinline__ static double mul(const Op &a, const Op &b) { return sf::prod(a, b); }
+    __device__ __forceinline__ static void sum_diff(double x, double y, double &s, double &d, bool &rare)
+    {
+        sf::sum_diff(x, y, s, d, rare);
+    }
     // a / 2 (an operand in range)
     __device__ __forceinline__ static Op half(Op a)
     {
@@ -66,6 +70,11 @@ struct Num<false> {
     using Op = double;
     __device__ __forceinline__ static Op op(double x, uint32_t &) { return x; }
     __device__ __forceinline__ static double mul(double a, double b) { return a * b; }
+    __device__ __forceinline__ static void sum_diff(double x, double y, double &s, double &d, bool &)
+    {
+        s = x + y;
+        d = x - y;
+    }
     __device__ __forceinline__ static double half(double a) { return 0.5 * a; }
     __device__ __forceinline__ static void put(double *w, uint32_t *, double a) { *w = a; }
     __device__ __forceinline__ static double get(const double *w, const uint32_t *) { return *w; }
@@ -258,9 +267,9 @@ static __device__ __noinline__ void ea_rotate_exact(const Dev &d, int e, double 
     store6(arr, d.nelem, e, s);
 }
 
-// the next strain rate, its dvoldt contribution, rotate_stress.  89 FP64
-// instructions per element at 82 % of the nominal rate, the pipe's measured peak;
-// 7 blocks of 128 per SM (6: 2 % slower, 8 and 9 the same)
+// the next strain rate, its dvoldt contribution, rotate_stress.  81 FP64
+// instructions per element, the pipe near its measured peak; 8 blocks of 128
+// per SM
 //
 // PARTS: kRates the strain rate into out, kDvoldt its dvoldt contribution,
 // kRotate the rotation with the current dt, kStepRotate the same with the
@@ -287,6 +296,7 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0, double *
     double D[6], u[3];
     {
         uint32_t far = 0;
+        bool rare = false;
         double t[3];
 #pragma unroll 1
         for (int i = 0; i < 4; ++i) {
@@ -297,34 +307,35 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0, double *
 #pragma unroll
             for (int k = 0; k < 3; ++k) g[k] = N::op(gp[4 * k * E], far);
             const double xx = N::mul(v0, g[0]), yy = N::mul(v1, g[1]), zz = N::mul(v2, g[2]);
-            const double xy = N::mul(v0, g[1]), yx = N::mul(v1, g[0]);
-            const double xz = N::mul(v0, g[2]), zx = N::mul(v2, g[0]);
-            const double yz = N::mul(v1, g[2]), zy = N::mul(v2, g[1]);
+            double tp[3], um[3];
+            // (one pair of the three on the integer pipes: E-A takes 861 us on
+            // 2.4M elements with none, 830 with one, 833 with two, 858 with all)
+            Num<false>::sum_diff(N::mul(v0, g[1]), N::mul(v1, g[0]), tp[0], um[0], rare);
+            Num<false>::sum_diff(N::mul(v0, g[2]), N::mul(v2, g[0]), tp[1], um[1], rare);
+            N::sum_diff(N::mul(v1, g[2]), N::mul(v2, g[1]), tp[2], um[2], rare);
             if (i == 0) {
                 D[0] = sf::add0(xx);
                 D[1] = sf::add0(yy);
                 D[2] = sf::add0(zz);
-                t[0] = sf::add0(xy + yx);
-                t[1] = sf::add0(xz + zx);
-                t[2] = sf::add0(yz + zy);
-                u[0] = sf::add0(xy - yx);
-                u[1] = sf::add0(xz - zx);
-                u[2] = sf::add0(yz - zy);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    t[k] = sf::add0(tp[k]);
+                    u[k] = sf::add0(um[k]);
+                }
             } else {
                 D[0] += xx;
                 D[1] += yy;
                 D[2] += zz;
-                t[0] += xy + yx;
-                t[1] += xz + zx;
-                t[2] += yz + zy;
-                u[0] += xy - yx;
-                u[1] += xz - zx;
-                u[2] += yz - zy;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    t[k] += tp[k];
+                    u[k] += um[k];
+                }
             }
         }
 #pragma unroll
         for (int k = 0; k < 3; ++k) D[3 + k] = sf::half(t[k]);
-        if (SOFT && !sf::in_range(far)) {
+        if (SOFT && (rare || !sf::in_range(far))) {
             double r[9];
             ea_rates_exact(d, e, r);
 #pragma unroll

@@ -554,7 +554,7 @@ int prime(des_gpu *g)
     else
         {
             const int eb = blocks(g->nelem, 128);
-            k_ea_rotate<true, 128, 7, kRates | kDvoldt><<<eb, 128, 0, g->stream>>>(g->d, 0, g->d.srate_next);
+            k_ea_rotate<true, 128, 8, kRates | kDvoldt><<<eb, 128, 0, g->stream>>>(g->d, 0, g->d.srate_next);
             if (g->hK.thermal) k_ea_conduction<true, 128, 8><<<eb, 128, 0, g->stream>>>(g->d, 0);
         }
     DES_LAUNCH();
@@ -732,7 +732,7 @@ void launch_ea(des_gpu *g, int b0, int b1)
             return;
         }
         k_ea_geometry<true, 128, 10, kStepGeometry><<<n, 128, 0, g->stream>>>(g->d, e0, nb, nullptr);
-        k_ea_rotate<true, 128, 7, kStepRates><<<n, 128, 0, g->stream>>>(g->d, e0, g->d.srate_next);
+        k_ea_rotate<true, 128, 8, kStepRates><<<n, 128, 0, g->stream>>>(g->d, e0, g->d.srate_next);
         if (g->hK.thermal) k_ea_conduction<true, 128, 8><<<n, 128, 0, g->stream>>>(g->d, e0);
     }
 }
@@ -2282,7 +2282,7 @@ int des_gpu_update_strain_rate(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_ea_rotate<true, 128, 7, kRates><<<ELEM_GRID(g)>>>(g->d, 0, g->d.srate);
+    k_ea_rotate<true, 128, 8, kRates><<<ELEM_GRID(g)>>>(g->d, 0, g->d.srate);
     return finish(g);
 }
 int des_gpu_compute_dvoldt(des_gpu *g)
@@ -2387,7 +2387,7 @@ int des_gpu_rotate_stress(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_ea_rotate<true, 128, 7, kRotate><<<ELEM_GRID(g)>>>(g->d, 0, nullptr);
+    k_ea_rotate<true, 128, 8, kRotate><<<ELEM_GRID(g)>>>(g->d, 0, nullptr);
     return finish(g);
 }
 int des_gpu_compute_dt(des_gpu *g, double *dt_out)

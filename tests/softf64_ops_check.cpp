@@ -1,6 +1,6 @@
 // Host check of the grouped integer-pipe product (unpack, prod, in_range), the
 // quotient (div), the square
-// root (root), the comparison (less), the running
+// root (root), the comparison (less), the sum and difference (sum_diff), the running
 // sum of positive numbers (PosSum) and the FP32 -> FP64 conversion (widen) of dynearthsol-old_gb300/csrc/des_softf64.cuh against the
 // host's IEEE arithmetic, bit for bit.
 //   softf64_ops_check <pairs per kind>  -> one line per kind; exit 1 on a mismatch
@@ -72,6 +72,15 @@ int main(int argc, char **argv)
             if (in_range(far)) {
                 ++grouped;
                 bad += bits(m) != bits(prod(a, b));
+                // two products of such operands; a pair that falls outside
+                // sum_diff's range says so
+                double p, d;
+                bool rare = false;
+                const double other = kind == 4 ? from_bits(bits(m) ^ (i & 1 ? kSign : 0) ^ (uint64_t)(i % 3)) : vx;
+                volatile double vo = other, vm = m;
+                const double hs = vm + vo, hd = vm - vo;
+                sum_diff(m, other, p, d, rare);
+                bad += !rare && (bits(hs) != bits(p) || bits(hd) != bits(d));
             }
             bad += !same(q, div(x, y));
             const double sq = std::sqrt(vx);
