@@ -776,22 +776,41 @@ __device__ __forceinline__ void stress_bc_node(const Consts &K, const BdryFacets
     if (K.elastic_foundation && (flag & kBoundZ0)) f[2] -= K.elastic_foundation_constant * (z - z0);
 }
 
-// fields.cxx:351-365
+// -x
+__device__ __forceinline__ double minus(double x) { return sf::from_bits(sf::bits(x) ^ sf::kSign); }
+
+// minus the sum of a component array over a node's entries on the FP64 unit
+static __device__ __noinline__ double gather_exact(const unsigned *ent, int q0, int q1, const double *t, size_t E)
+{
+    double f = 0;
+    for (int q = q0; q < q1; ++q) {
+        const unsigned p = __ldg(ent + q);
+        f -= t[(size_t)(p & 3u) * E + (p >> 2)];
+    }
+    return f;
+}
+
+// minus the sums of the three force components over a node's entries
+// (fields.cxx:351-365), x on the integer pipes (sf::sum), beside y and z on
+// the FP64 unit
 __device__ __forceinline__ void force_gather(const Dev &d, int n, double f[3])
 {
     const size_t E = d.nelem;
+    const int q0 = d.sup_off[n], q1 = d.sup_off[n + 1];
     f[0] = f[1] = f[2] = 0;
+    bool rare = false;
     walk<4>(
-        d.sup_ent, d.sup_off[n], d.sup_off[n + 1],
+        d.sup_ent, q0, q1,
         [&](unsigned p) {
             const double *t = d.tmp + (size_t)(p & 3u) * E + (p >> 2);
             return Three<double>{t[0], t[4 * E], t[8 * E]};
         },
         [&](const Three<double> &t) {
-            f[0] -= t.x;
+            f[0] = sf::sum(f[0], minus(t.x), rare);
             f[1] -= t.y;
             f[2] -= t.z;
         });
+    if (rare) f[0] = gather_exact(d.sup_ent, q0, q1, d.tmp, E);
 }
 
 // v += dt f / m (fields.cxx:386-389): one reciprocal of m on the integer pipes
@@ -1094,10 +1113,10 @@ __global__ void __launch_bounds__(128, 8) k_fe_b_t(Dev d, int e0)
 }
 
 // N-C: force gather, damping, velocity, velocity BCs, coordinates.  Its
-// products and its three divisions by one mass are on the integer pipes (20.6
-// -> 17.0 FP64 instructions per element, at the pipe's peak: 108 -> 91 us for
-// 2.4M elements); its 12 signed additions are not: one on the integer pipes
-// takes about as long as on the FP64 unit.
+// products, its three divisions by one mass and a third of its additions are
+// on the integer pipes: 20.6 -> 13 FP64 instructions per element, 118 -> 89 us
+// for 2.4M elements (101 with the additions on the FP64 unit, which then is at
+// its peak).  The FP32 form's N-C lost by the same move (106 -> 128 us).
 __global__ void k_fn_c(Dev d)
 {
     int n = gtid();

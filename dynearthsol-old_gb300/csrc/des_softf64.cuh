@@ -320,6 +320,33 @@ DES_SF_HD void sum_diff(double x, double y, double &sum, double &diff, bool &rar
     diff = from_bits(same ? D : S);
 }
 
+// x + y alone, for zeros and numbers of 2^-900 and more (rare as above).
+DES_SF_HD double sum(double x, double y, bool &rare)
+{
+    const uint64_t bx = bits(x), by = bits(y);
+    const bool swap = (bx & kAbs) < (by & kAbs);
+    const uint64_t big = swap ? by : bx, small = swap ? bx : by;
+    const uint32_t hb = (uint32_t)(big >> 32), hs = (uint32_t)(small >> 32);
+    const uint32_t eb = hb & 0x7ff00000u, es = hs & 0x7ff00000u;
+    uint32_t d = (eb - es) >> 20;
+    d = d < 63u ? d : 63u;
+    // significands at bit 61, 9 zero bits below; a zero has none
+    const uint64_t mb = ((big << 9) & 0x1fffffffffffffffull) | (eb ? 0x2000000000000000ull : 0);
+    const uint64_t ms = ((small << 9) & 0x1fffffffffffffffull) | (es ? 0x2000000000000000ull : 0);
+    uint64_t a = ms >> d;
+    a |= (uint64_t)((a << d) != ms);                      // sticky
+    const uint64_t minus = (uint64_t)((int64_t)(bx ^ by) >> 63);
+    uint64_t f = mb + (a ^ minus) - minus;
+    const uint32_t k = (uint32_t)clz32((uint32_t)(f >> 32)) - 1;
+    const bool none = f == 0;
+    rare = rare || (!none && k > 30u) || eb - (123u << 20) > (1900u << 20) - (123u << 20);
+    f <<= k & 63;
+    f += 0x1ff + ((uint32_t)(f >> 10) & 1);
+    const uint64_t w = (f >> 10) + ((uint64_t)(eb - (k << 20)) << 32);
+    const uint64_t sign = none && minus ? 0 : big & kSign;
+    return from_bits((none ? 0 : w) | sign);
+}
+
 // ---- quotients ----------------------------------------------------------------
 // The FP64 unit's division takes about nine FP64 instructions; on the integer
 // pipes the reciprocal of the denominator's significand comes from an FP32

@@ -1,6 +1,7 @@
 // Host check of the grouped integer-pipe product (unpack, prod, in_range), the
 // quotient (div), the square
-// root (root), the comparison (less), the sum and difference (sum_diff), the running
+// root (root), the comparison (less), the sum and
+// difference (sum_diff, sum), the running
 // sum of positive numbers (PosSum) and the FP32 -> FP64 conversion (widen) of dynearthsol-old_gb300/csrc/des_softf64.cuh against the
 // host's IEEE arithmetic, bit for bit.
 //   softf64_ops_check <pairs per kind>  -> one line per kind; exit 1 on a mismatch
@@ -81,6 +82,9 @@ int main(int argc, char **argv)
                 const double hs = vm + vo, hd = vm - vo;
                 sum_diff(m, other, p, d, rare);
                 bad += !rare && (bits(hs) != bits(p) || bits(hd) != bits(d));
+                rare = false;
+                p = sum(m, other, rare);
+                bad += !rare && bits(hs) != bits(p);
             }
             bad += !same(q, div(x, y));
             const double sq = std::sqrt(vx);
