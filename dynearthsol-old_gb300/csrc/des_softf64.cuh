@@ -666,12 +666,11 @@ DES_SF_HD float to_float(double x)
 {
     const uint64_t a = bits(x);
     const uint32_t hi = (uint32_t)(a >> 32), lo = (uint32_t)a;
-    const int ef = (int)((hi >> 20) & 0x7ff) - 896;
-    if ((uint32_t)(ef - 1) < 254u) {
-        const uint32_t m = ((hi & 0xfffffu) << 3) | (lo >> 29);
-        const uint32_t rem = lo & 0x1fffffffu;
-        const uint32_t up = (uint32_t)((rem > 0x10000000u) | ((rem == 0x10000000u) & m));
-        return float_from_bits((hi & 0x80000000u) | ((((uint32_t)ef) << 23) + m + up));
+    if ((hi & 0x7fffffffu) - (897u << 20) < (254u << 20)) {
+        // half a unit less a bit, plus the unit's parity, added below the 24
+        // bits that stay; the exponent's upper bits leave with the shift
+        const uint64_t r = a + (0x0fffffffu + ((lo >> 29) & 1));
+        return float_from_bits((hi & 0x80000000u) | (((uint32_t)(r >> 29) - (896u << 23)) & 0x7fffffffu));
     }
     return float_from_bits(to_float_slow(a));
 }
