@@ -579,9 +579,11 @@ void launch_surface(des_gpu *g)
 // 10.3 / 16.3, 14.3 / 16.4, 20.5 / 17.4.  FP32: N-A 9.3 / 14.2 at 5.6k, 12.8 /
 // 14.1 at 21.9k, 19.8 / 17.1 at 48k; N-B 5.8 / 8.2, 6.5 / 8.1, 8.2 / 8.4; N-C
 // 12.3 / 18.4, 20.5 / 18.4.  E-A 15.6 / 31.3 at 9.6k elements, 28.1 / 35.8 at
-// 27.6k, 46.2 / 42.2 at 54k; E-C 8.2 / 10.3, 12.3 / 12.3, 16.4 / 13.9.
+// 27.6k, 46.2 / 42.2 at 54k; E-C 8.2 / 10.3, 12.3 / 12.3, 16.4 / 13.9.  FP32 E-A
+// 10.6 / 12.7 at 192 elements, 10.9 / 12.9 at 9.6k, 13.3 / 15.0 at 27.6k, 17.4 /
+// 14.7 at 38.9k (the step 23.0 / 26.4, 27.0 / 29.3, 32.4 / 32.6, 37.9 / 34.8).
 const int kOctetNodes[2][3] = {{128, 32, 90}, {200, 300, 96}};   // [FP64, FP32][N-A, N-B, N-C]
-const int kQuadElemsEa = 280, kQuadElemsEc = 180;
+const int kQuadElemsEa[2] = {280, 170}, kQuadElemsEc = 180;      // E-A: [FP64, FP32]
 // FP32 E-B with the exact returns in place / over the list: 9.6 / 13.4 at 27.7k elements, on yielding boxes 54.9 / 61.8 at
 // 14.4k, 61.9 / 64.4 at 54k, 119 / 80 at 240k
 const int kDirectReturns = 300;
@@ -589,7 +591,7 @@ bool octets(const des_gpu *g, int pass)
 {
     return g->nnode <= kOctetNodes[g->prec == DES_PREC_FP32][pass] * g->sms;
 }
-bool quads_ea(const des_gpu *g) { return g->nelem <= kQuadElemsEa * g->sms; }
+bool quads_ea(const des_gpu *g) { return g->nelem <= kQuadElemsEa[g->prec == DES_PREC_FP32] * g->sms; }
 bool direct_returns(const des_gpu *g) { return !g->closure && g->nelem <= kDirectReturns * g->sms; }
 bool quads_ec(const des_gpu *g) { return g->nelem <= kQuadElemsEc * g->sms; }
 
@@ -720,17 +722,16 @@ void launch_head(des_gpu *g, cudaEvent_t *ev)
 void launch_ea(des_gpu *g, int b0, int b1)
 {
     g->mass_valid = false;
-    const int nb = blocks(g->nelem, kElemBlock);
-    if (g->prec == DES_PREC_FP32)
-        kf_fe_a<<<b1 - b0, kElemBlock, 0, g->stream>>>(g->f, b0 * kElemBlock, nb);
-    else
-{
-        const int n = b1 - b0, e0 = b0 * kElemBlock;
-        if (quads_ea(g)) {
-            constexpr int kQuads = kElemBlock * 4 / kSmallBlock;     // blocks of four lanes an element per block of one
-            k_ea_quad<<<n * kQuads, kSmallBlock, 0, g->stream>>>(g->d, e0, nb * kQuads);
-            return;
-        }
+    const int nb = blocks(g->nelem, kElemBlock), n = b1 - b0, e0 = b0 * kElemBlock;
+    constexpr int kQuads = kElemBlock * 4 / kSmallBlock;     // blocks of four lanes an element per block of one
+    const bool f32 = g->prec == DES_PREC_FP32;
+    if (f32 && quads_ea(g)) {
+        kf_ea_quad<<<n * kQuads, kSmallBlock, 0, g->stream>>>(g->f, e0, nb * kQuads);
+    } else if (f32) {
+        kf_fe_a<<<n, kElemBlock, 0, g->stream>>>(g->f, e0, nb);
+    } else if (quads_ea(g)) {
+        k_ea_quad<<<n * kQuads, kSmallBlock, 0, g->stream>>>(g->d, e0, nb * kQuads);
+    } else {
         k_ea_geometry<true, 128, 10, kStepGeometry><<<n, 128, 0, g->stream>>>(g->d, e0, nb, nullptr);
         k_ea_rotate<true, 128, 8, kStepRates><<<n, 128, 0, g->stream>>>(g->d, e0, g->d.srate_next);
         if (g->hK.thermal) k_ea_conduction<true, 128, 8><<<n, 128, 0, g->stream>>>(g->d, e0);

@@ -337,6 +337,170 @@ __device__ __forceinline__ double signed_by(double x, bool minus)
     return sf::from_bits(sf::bits(x) ^ (minus ? sf::kSign : 0ull));
 }
 
+// The FP32 form's E-A (kf_fe_a) with lane i at node i: its cofactor, gradient,
+// reference force and row of the conduction; lanes 0 and 1 rotate the stress
+// and the strain, 2 and 3 store the strain rate and its trace.  The FP32 sums
+// over the nodes are formed by every lane, in kf_fe_a's order.
+// A small mesh's pass is one thread's chain of about 2,000 instructions, 37 of
+// them on the FP64 unit: a lane's is a third of it, 12 on the FP64 unit (9.6k
+// elements 12.9 -> 10.9 us).  Four lanes take 1.3 times the FP64 instructions
+// of one thread, so beyond a few warps a scheduler the pass is slower.
+__global__ void __launch_bounds__(kSmallBlock) kf_ea_quad(DevF d, int e0, unsigned nblocks)
+{
+    __shared__ double s_x[3][kSmallBlock];
+    __shared__ float s_f[6][kSmallBlock];
+    const int i = threadIdx.x & 3, base = threadIdx.x & ~3;
+    const int e_ = e0 + (int)(blockIdx.x * kSmallBlock + threadIdx.x) / 4;
+    const Consts &K = *d.K;
+    const ConstsF &F = *d.F;
+    const bool live = e_ < d.nelem;
+    const int e = live ? e_ : d.nelem - 1;
+    const bool dt_step = (K.fixed_dt == 0) && (d.clk->steps % 10 == 0);
+    if (e_ == 0 && i == 0) d.clk->mass_valid = 0;
+    const size_t E = d.nelem;
+    const int n = reinterpret_cast<const int *>(d.conn)[4 * (size_t)e + i];
+    const MixF &xf = F.mix[d.mix[e]];
+    const bool rotate = F.rheol & 1;
+    const float dt = sf::to_float(d.clk->dt);
+    float *field = i == 0 ? d.stress : d.strain, s[6];
+    if (rotate && i < 2) f_load6(field, E, e, s);
+    const double T = d.T[n], vol_was = d.vol[e], s0 = d.s0[e];
+    const double x[3] = {d.x[n], d.y[n], d.z[n]};
+    s_f[0][threadIdx.x] = d.vx[n];
+    s_f[1][threadIdx.x] = d.vy[n];
+    s_f[2][threadIdx.x] = d.vz[n];
+    // f_cofactors: the edge to each lane's node; lanes 1-3 the cross products of
+    // the two others' (b, q) (q, a) (a, b); lane k < 3 the three products' k-th
+    // components' sum, which is minus lane 0's cofactor
+    double cf[3], det;
+    {
+        const int iu = two(0x7a, i), iv = two(0x9f, i), kk = i < 3 ? i : 2;     // - 2 3 1 | - 3 1 2
+        double u[3], v[3], a[3], c1[3];
+        uint32_t far = 0;
+        sf::Op ou[3], ov[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s_x[k][threadIdx.x] = x[k] - quad_get(x[k], 0);
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            u[k] = s_x[k][base + iu];
+            v[k] = s_x[k][base + iv];
+            a[k] = s_x[k][base + 1];
+            ou[k] = sf::unpack(u[k], far);
+            ov[k] = sf::unpack(v[k], far);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int p = (k + 1) % 3, q = (k + 2) % 3;
+            cf[k] = fma(u[p], v[q], -sf::prod(ou[q], ov[p]));
+            s_x[k][threadIdx.x] = cf[k];
+        }
+        __syncwarp();
+        const double sum = s_x[kk][base + 1] + s_x[kk][base + 2] + s_x[kk][base + 3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            c1[k] = s_x[k][base + 1];
+            const double c0 = signed_by(quad_get(sum, k), true);
+            if (i == 0) cf[k] = c0;
+        }
+        det = fma(a[0], c1[0], fma(a[1], c1[1], sf::prod(sf::unpack(a[2], far), sf::unpack(c1[2], far))));
+        far = max(far, __shfl_xor_sync(0xffffffffu, far, 1, 4));
+        far = max(far, __shfl_xor_sync(0xffffffffu, far, 2, 4));
+        if (!sf::in_range(far)) {
+            double r[12];
+            det = f_cofactors_exact(d, d.conn[e], r);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) cf[k] = r[3 * i + k];
+        }
+    }
+    const double vol = sf::mul(det, 1.0 / 6.0);
+    const float volf = sf::to_float(vol);
+    if (live && i == 0) {
+        d.vol_old[e] = vol_was;
+        d.vol[e] = vol;
+        d.c_vol[e] = volf;
+        if (not_positive(vol)) atomicOr(&d.clk->status, 0x4u);
+    }
+    // f_reference_force, node i
+    {
+        const double s6 = sf::mul(s0, 1.0 / 6.0), buoy = F.gravity != 0.f ? sf::mul(xf.rho_g4, vol) : 0.0;
+        uint32_t far = 0;
+        const sf::Op o6 = sf::unpack(s6, far);
+        double fx = sf::prod(o6, sf::unpack(cf[0], far)), fy = sf::prod(o6, sf::unpack(cf[1], far));
+        if (!sf::in_range(far)) {
+            fx = sf::from_bits(sf::mul_slow(sf::bits(s6), sf::bits(cf[0])));
+            fy = sf::from_bits(sf::mul_slow(sf::bits(s6), sf::bits(cf[1])));
+        }
+        if (live) {
+            d.f0[i * E + e] = fx;
+            d.f0[(i + 4) * E + e] = fy;
+            d.f0[(i + 8) * E + e] = fma(s6, cf[2], buoy);
+        }
+    }
+    double minh = 0;
+    if (dt_step) {
+        const double m = fma(cf[0], cf[0], fma(cf[1], cf[1], cf[2] * cf[2]));
+        minh = 6 * vol / sqrt(fmax(fmax(quad_get(m, 0), quad_get(m, 1)), fmax(quad_get(m, 2), quad_get(m, 3))));
+    }
+    const float iv = 1.f / sf::to_float(det);
+    float g[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        g[k] = sf::to_float(cf[k]) * iv;
+        s_f[3 + k][threadIdx.x] = g[k];
+        if (live) d.shp[(size_t)(4 * k + i) * E + e] = g[k];
+    }
+    __syncwarp();
+    float V[4][3], dx[4], dy[4], dz[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) V[j][k] = s_f[k][base + j];
+        dx[j] = s_f[3][base + j];
+        dy[j] = s_f[4][base + j];
+        dz[j] = s_f[5][base + j];
+    }
+    {
+        const float t = sf::to_float(T);
+        const float rT = f_rho(F, xf, elem_mean4(quad_get(t, 0), quad_get(t, 1), quad_get(t, 2), quad_get(t, 3)));
+        if (live && i == 2) d.c_mass[e] = (F.is_qs ? xf.rho_qs : rT) * volf * 0.25f;
+        if (live && i == 3 && F.thermal) d.c_tmass[e] = rT * xf.cp * volf * 0.25f;
+    }
+    if (rotate && i < 2) {
+        float w3, w4, w5;
+        spin(V, dx, dy, dz, w3, w4, w5);
+        jaumann(s, dt, w3, w4, w5);
+        if (live) f_store6(field, E, e, s);
+    }
+    // f_next_contrib
+    if (i >= 2) {
+        float D[6];
+        strain_rate(V, dx, dy, dz, D);
+        if (live && i == 2) f_store6(d.srate_next, E, e, D);
+        if (live && i == 3) d.c_trdv[e] = tr3(D) * volf;
+    }
+    if (F.thermal) {
+        const double T0 = quad_get(T, 0);
+        const float t = sf::to_float(T - T0);
+        const float t1 = quad_get(t, 1), t2 = quad_get(t, 2), t3 = quad_get(t, 3);
+        const float gx = dx[1] * t1 + dx[2] * t2 + dx[3] * t3;
+        const float gy = dy[1] * t1 + dy[2] * t2 + dy[3] * t3;
+        const float gz = dz[1] * t1 + dz[2] * t2 + dz[3] * t3;
+        const float kv = xf.k * volf;
+        if (live) d.tmp[i * E + e] = kv * (g[0] * gx + g[1] * gy + g[2] * gz);
+    }
+    if (dt_step) {
+        Dev dd;
+        dd.conn = d.conn;
+        dd.T = d.T;
+        dd.mix = d.mix;
+        dd.K = d.K;
+        dd.clk = d.clk;
+        dt_reduce_and_finalize(dd, minh, live, nblocks);
+    }
+}
+
 // E-A (k_ea_geometry, k_ea_rotate, k_ea_conduction in one): lane i has node i
 // of the element: its gradient, its products with the velocity, its row of
 // the conduction matrix; lanes 0-2 sum the rates' components and rotate one

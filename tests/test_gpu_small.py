@@ -8,6 +8,7 @@ import pytest
 
 import des_gb300 as D
 from des_gb300 import abi, workload as W
+from helpers import rel_l2
 from oracle.oracle import PortOracle
 
 FIELDS = ["coord", "vel", "force", "temperature", "mass", "tmass", "volume_n", "ntmp", "volume", "volume_old",
@@ -61,4 +62,33 @@ def test_operands_out_of_range_take_the_exact_path(gpu, box):
     got = dev.download(abi.State(mesh.nnode, mesh.nelem), abi.F_STEP_STATE)
     for f in FIELDS:
         assert np.array_equal(getattr(got, f), getattr(ref, f)), f
+    dev.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("box", BOXES)
+def test_small_meshes_fp32(gpu, box):
+    """The FP32 form's shared-lane kernels: one step from the oracle's state to
+    the one-step bars of test_gpu_fp32.py, and the temperature (1e-12 there)
+    after a second step, which is the first to read the pass's conduction."""
+    cfg = W.scaled(W.CONFIGS["tiny"], *box)
+    mesh, p, T, pls, _ = D.setup_case(cfg)
+    ref = W.new_state(mesh, T, pls)
+    o = PortOracle(mesh, p)
+    o.init_fields(ref)
+    o.step(ref, 9)                         # the step after it forms dt
+    p32 = abi.Params.from_buffer_copy(p)
+    p32.precision = abi.PREC_FP32
+    dev = D.Device(mesh, p32, device=0)
+    dev.upload(ref, abi.F_ALL)
+    o.step(ref, 1)
+    dev.step(1)
+    got = dev.download(abi.State(mesh.nnode, mesh.nelem), abi.F_STEP_STATE)
+    for f in ["vel", "force", "stress", "strain", "mass", "tmass", "volume_n", "volume", "shpdx", "shpdy", "shpdz"]:
+        assert rel_l2(getattr(got, f), getattr(ref, f)) <= 1e-6, f
+    assert got.dt == pytest.approx(ref.dt, rel=1e-6) and got.steps == ref.steps
+    o.step(ref, 1)
+    dev.step(1)
+    dev.download(got, abi.F_STEP_STATE)
+    assert rel_l2(got.temperature, ref.temperature) <= 1e-12
     dev.close()
