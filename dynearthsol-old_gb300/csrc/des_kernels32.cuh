@@ -890,12 +890,13 @@ __global__ void k_stress_split(const double *src, double *s0, float *dst, long l
     for (int c = 0; c < 6; ++c) dst[c * ld + row0 + r] = (float)(a[c] - (c < 3 ? m : 0.0));
 }
 __global__ void k_stress_join(const double *s0, const float *src, double *dst, long long rows,
-                              long long row0, long long ld)
+                              long long row0, long long ld, int skip)
 {
-    long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    double m = s0[row0 + r];
-    for (int c = 0; c < 6; ++c) dst[6 * r + c] = (double)src[c * ld + row0 + r] + (c < 3 ? m : 0.0);
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x - skip;
+    if (i < 0 || i >= rows * 6) return;
+    const long long r = i / 6;
+    const int c = (int)(i - r * 6);
+    dst[i] = (double)src[c * ld + row0 + r] + (c < 3 ? s0[row0 + r] : 0.0);
 }
 
 // the same split for page-locked host rows read in place: a block moves 256
@@ -976,10 +977,10 @@ __global__ void k_aos_to_soa_f(const double *src, float *dst, int ncomp, long lo
     dst[c * ld + row0 + r] = (float)src[i];
 }
 __global__ void k_soa_to_aos_f(const float *src, double *dst, int ncomp, long long rows, long long row0,
-                               long long ld)
+                               long long ld, int skip)
 {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * ncomp) return;
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x - skip;
+    if (i < 0 || i >= rows * ncomp) return;
     long long r = i / ncomp;
     int c = (int)(i - r * ncomp);
     dst[i] = (double)src[c * ld + row0 + r];
