@@ -41,7 +41,7 @@ B_NODE = 3 * 8 * 2 * 2 + 8 * 2 + 4
 
 # DRAM bytes (read + written) per element of each FP64 pass from one ncu
 # capture of the pass alone on a 100x100x40 box of config 2's physics
-TRAFFIC_PER_ELEM = {"N-A": 95.0, "E-B": 438.9, "N-B": 26.3, "E-C": 310.6, "N-C": 136.7, "E-A": 607.2}
+TRAFFIC_PER_ELEM = {"N-A": 88.2, "E-B": 416.7, "N-B": 26.3, "E-C": 317.5, "N-C": 135.5, "E-A": 638.6}
 
 
 def peaks():
@@ -719,11 +719,12 @@ def run_ours(args):
     # FP64 pipe: thread instructions on the FP64 pipe per element of each pass
     # in a step without the dt reduction (ncu instruction counters of the same
     # passes on a 100x100x40 box of this physics), against GB300's 2 FP64
-    # instructions per clock per SM.  Part of each pass's multiplies run as
-    # exactly rounded integer-pipe products (sf::mul) instead, which is what
+    # instructions per clock per SM (a loop of independent FMAs reaches 79 % of
+    # that).  Products, quotients, roots and some sums run as exactly rounded
+    # integer-pipe arithmetic (des_softf64.cuh) instead, which is what
     # lets the step beat this pipe's bound for the reference's arithmetic
     # (604 FP64 instructions per element-step when every product is on it).
-    fp64_ops = {"N-A": 23.1, "E-B": 44.0, "N-B": 5.4, "E-C": 44.1, "N-C": 19.7, "E-A": 260.0}
+    fp64_ops = {"N-A": 8.2, "E-B": 31.0, "N-B": 4.0, "E-C": 41.0, "N-C": 10.5, "E-A": 154.0}
     fp64_ops_all_on_pipe = 604.2
     import torch
     sms = torch.cuda.get_device_properties(local).multi_processor_count
