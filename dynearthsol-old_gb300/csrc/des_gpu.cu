@@ -808,12 +808,17 @@ void launch_step(des_gpu *g, cudaEvent_t *ev)
     launch_tail(g, ev);
 }
 
-int finish(des_gpu *g)
+// the end of a call that has queued work on the caller's host rows, which the
+// kernels read and write in place: it waits for the stream where the call has
+// failed (rc), too, since the caller may release the rows when it returns
+int settle(des_gpu *g, int rc)
 {
-    DES_CUDA(cudaGetLastError());
-    DES_CUDA(cudaStreamSynchronize(g->stream));
-    return DES_OK;
+    const cudaError_t launched = cudaGetLastError(), done = cudaStreamSynchronize(g->stream);
+    if (rc) return rc;
+    return launched == cudaSuccess && done == cudaSuccess ? DES_OK : DES_ERR_CUDA;
 }
+
+int finish(des_gpu *g) { return settle(g, DES_OK); }
 
 // the second stream (output copies, downloads overlapping E-A) and its events
 int ensure_copy_stream(des_gpu *g)
@@ -1298,10 +1303,32 @@ int des_gpu_kernels_per_step(const des_gpu *g)
     return n + (g->avg_interval > 0 ? 1 : 0);
 }
 
-int des_gpu_upload(des_gpu *g, const des_state_view *h, unsigned mask)
+// whether every array that the mask asks for is there
+static bool has_arrays(const des_state_view *h, unsigned mask)
 {
-    if (!g || !h || h->nnode != g->nnode || h->nelem != g->nelem) return DES_ERR_ARG;
-    if (mask & ~(unsigned)DES_F_ALL) return DES_ERR_ARG;
+    const struct {
+        unsigned flag;
+        const double *rows;
+    } need[] = {{DES_F_COORD, h->coord},           {DES_F_COORD0, h->coord0},
+                {DES_F_VEL, h->vel},               {DES_F_FORCE, h->force},
+                {DES_F_TEMPERATURE, h->temperature}, {DES_F_MASS, h->mass},
+                {DES_F_MASS, h->tmass},            {DES_F_MASS, h->volume_n},
+                {DES_F_NTMP, h->ntmp},             {DES_F_VOLUME, h->volume},
+                {DES_F_VOLUME, h->volume_old},     {DES_F_STRESS, h->stress},
+                {DES_F_STRAIN, h->strain},         {DES_F_STRAIN_RATE, h->strain_rate},
+                {DES_F_PLSTRAIN, h->plstrain},     {DES_F_PLSTRAIN, h->delta_plstrain},
+                {DES_F_DPRESSURE, h->dpressure},   {DES_F_EDVOLDT, h->edvoldt},
+                {DES_F_SHAPE, h->shpdx},           {DES_F_SHAPE, h->shpdy},
+                {DES_F_SHAPE, h->shpdz},           {DES_F_TMP_RESULT, h->tmp_result},
+                {DES_F_TMP_RESULT, h->tmp_result_sg}};
+    for (const auto &n : need)
+        if ((mask & n.flag) && !n.rows) return false;
+    return true;
+}
+
+// the mask fields of h, all of them there, into the device's arrays
+static int upload_fields(des_gpu *g, const des_state_view *h, unsigned mask)
+{
     const long long N = g->nnode, E = g->nelem;
     Dev &d = g->d;
     int rc = DES_OK;
@@ -1329,7 +1356,6 @@ int des_gpu_upload(des_gpu *g, const des_state_view *h, unsigned mask)
     UP(DES_F_VOLUME, volume_old, d.vol_old, 1, E)
     if (mask & DES_F_STRESS) {
         if (f32) {
-            if (!h->stress) return DES_ERR_ARG;
             if (const double *m = static_cast<const double *>(mapped(h->stress))) {
                 k_stress_split_tiled<<<blocks(E, 256), 256, 0, g->stream>>>(m, f.s0, f.stress, E);
                 DES_LAUNCH();
@@ -1382,7 +1408,16 @@ int des_gpu_upload(des_gpu *g, const des_state_view *h, unsigned mask)
         DES_LAUNCH();
     }
     g->primed = false;
-    return finish(g);
+    return DES_OK;
+}
+
+int des_gpu_upload(des_gpu *g, const des_state_view *h, unsigned mask)
+{
+    if (!g || !h || h->nnode != g->nnode || h->nelem != g->nelem) return DES_ERR_ARG;
+    if (mask & ~(unsigned)DES_F_ALL) return DES_ERR_ARG;
+    // (before anything is queued: a refused call has read nothing)
+    if (!has_arrays(h, mask)) return DES_ERR_ARG;
+    return settle(g, upload_fields(g, h, mask));
 }
 
 // One field of a download: its host rows and its device source (FP64 or
@@ -1518,13 +1553,13 @@ int des_gpu_download(des_gpu *g, des_state_view *h, unsigned mask)
     int rc = read_clock(g, c);
     if (rc) return rc;
     if ((mask & DES_F_MASS) && (rc = flush_masses(g))) return rc;
-    if ((rc = download_fields(g, h, mask))) return rc;
+    if ((rc = settle(g, download_fields(g, h, mask)))) return rc;
     if (mask & DES_F_SCALARS) {
         h->time = c.time;
         h->dt = c.dt;
         h->steps = c.steps;
     }
-    return finish(g);
+    return DES_OK;
 }
 
 int des_gpu_report(des_gpu *g, des_step_report *r)
@@ -1773,11 +1808,9 @@ int des_gpu_set_averaging(des_gpu *g, int interval)
     return DES_OK;
 }
 
-int des_gpu_download_averages(des_gpu *g, double *coord0, double *strain0, double *stress_sum,
-                              double *dpls_sum, double *time0)
+static int download_averages(des_gpu *g, double *coord0, double *strain0, double *stress_sum, double *dpls_sum,
+                             double *time0)
 {
-    if (!g) return DES_ERR_ARG;
-    if (!g->avg_c0) return DES_ERR_UNSUPPORTED;
     int rc;
     if (coord0 && (rc = download_field(g, coord0, g->avg_c0, 3, g->nnode, g->stream, g->staging))) return rc;
     if (strain0 && (rc = download_field(g, strain0, g->avg_strain0, 6, g->nelem, g->stream, g->staging))) return rc;
@@ -1785,7 +1818,15 @@ int des_gpu_download_averages(des_gpu *g, double *coord0, double *strain0, doubl
                                                  g->staging))) return rc;
     if (dpls_sum && (rc = download_field(g, dpls_sum, g->avg_dpls, 1, g->nelem, g->stream, g->staging))) return rc;
     if (time0) DES_CUDA(cudaMemcpyAsync(time0, g->avg_time0, sizeof(double), cudaMemcpyDeviceToHost, g->stream));
-    return finish(g);
+    return DES_OK;
+}
+
+int des_gpu_download_averages(des_gpu *g, double *coord0, double *strain0, double *stress_sum,
+                              double *dpls_sum, double *time0)
+{
+    if (!g) return DES_ERR_ARG;
+    if (!g->avg_c0) return DES_ERR_UNSUPPORTED;
+    return settle(g, download_averages(g, coord0, strain0, stress_sum, dpls_sum, time0));
 }
 
 int des_gpu_set_closure(des_gpu *g, const des_mlp *net)

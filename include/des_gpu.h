@@ -259,7 +259,9 @@ int  des_gpu_remesh(des_gpu *g, const des_mesh_view *mesh, const des_state_view 
                     int reset_bottom_coord0);
 
 /* Host Variables -> device (fields in mask).  Marks nodal masses as current,
- * so the next step uses them as the reference does after update_mesh. */
+ * so the next step uses them as the reference does after update_mesh.
+ * DES_ERR_ARG, with nothing uploaded, where an array that mask names is NULL.
+ * The rows are the caller's again when the call returns, whatever it returns. */
 int  des_gpu_upload(des_gpu *g, const des_state_view *host, unsigned mask);
 /* device -> host Variables (fields in mask); synchronises. */
 int  des_gpu_download(des_gpu *g, des_state_view *host, unsigned mask);
