@@ -134,7 +134,8 @@ int read_err(const int *derr)
 
 // Rows of the caller's as a kernel reads or writes them: in place where the
 // GPU reaches any host memory through the host's page tables (GB300 over
-// NVLink-C2C) and the rows are 16-byte aligned, else through a device copy.
+// NVLink-C2C), the rows are 16-byte aligned and the caller allows it, else
+// through a device copy.
 // In place, 250k samples' rows cross the link under the kernel, where a device
 // copy had its own allocation, transfer and release (with one kept Call, below:
 // forward 700 -> 355 us, 135 of it the caller's fresh output pages; loss and
@@ -143,12 +144,12 @@ struct Rows {
     DevBuf buf;
     float *p = nullptr;
     bool host = false;
-    int open(const float *rows, size_t bytes, bool copy_in)
+    int open(const float *rows, size_t bytes, bool copy_in, bool in_place = true)
     {
         int dev = 0, ats = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&ats, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev);
-        host = ats && reinterpret_cast<uintptr_t>(rows) % 16 == 0;
+        host = in_place && ats && reinterpret_cast<uintptr_t>(rows) % 16 == 0;
         if (host) {
             p = const_cast<float *>(rows);
             return DES_OK;
@@ -159,6 +160,12 @@ struct Rows {
         return DES_OK;
     }
 };
+
+bool overlap(const void *a, size_t na, const void *b, size_t nb)
+{
+    const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+    return p < q + nb && q < p + na;
+}
 
 // The small device data of one call, one allocation and one copy each way:
 // parameters, gradient, loss, the kernels' time-out flag (the last three zero)
@@ -207,8 +214,10 @@ int des_mlp_forward(const des_mlp *net, const float *x, long long n, float *y)
     int rc;
     Call *c = call_buf.get();
     if (!c) return DES_ERR_NOMEM;
-    if ((rc = rx.open(x, sizeof(float) * n * kMlpIn, true)) || (rc = ry.open(y, sizeof(float) * n * kMlpOut, false)))
-        return rc;
+    // (outputs over the inputs: a tile's would be written over rows that other
+    // tiles have yet to read)
+    const size_t nx = sizeof(float) * n * kMlpIn, ny = sizeof(float) * n * kMlpOut;
+    if ((rc = rx.open(x, nx, true, !overlap(x, nx, y, ny))) || (rc = ry.open(y, ny, false))) return rc;
     if (smem_setup((const void *)k_mlp_forward)) return DES_ERR_CUDA;
     if (cudaMemcpy(c, h.data(), sizeof(Call), cudaMemcpyHostToDevice)) return DES_ERR_CUDA;
     const int grid = tile_grid((n + kTile - 1) / kTile);

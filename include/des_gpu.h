@@ -352,7 +352,7 @@ typedef struct des_mlp {
     float tol;                                      /* relative yield-residual tolerance */
 } des_mlp;
 
-/* y[n][8] = net(x[n][16]) on the tensor cores (host arrays). */
+/* y[n][8] = net(x[n][16]) on the tensor cores (host arrays; y may lie over x). */
 int  des_mlp_forward(const des_mlp *net, const float *x, long long n, float *y);
 /* loss = mean over the n samples of the summed squared error of the 7
  * outputs, and its gradient with respect to every weight and bias. */
