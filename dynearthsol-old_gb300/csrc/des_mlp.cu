@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 #include <numeric>
@@ -137,7 +138,7 @@ int read_err(const int *derr)
 // NVLink-C2C), the rows are 16-byte aligned and the caller allows it, else
 // through a device copy.
 // In place, 250k samples' rows cross the link under the kernel, where a device
-// copy had its own allocation, transfer and release (with one kept Call, below:
+// copy had its own allocation, transfer and release (with the kept Call, below:
 // forward 700 -> 355 us, 135 of it the caller's fresh output pages; loss and
 // gradient 700 -> 238 us; both 200 -> 57 us on 256 samples).
 struct Rows {
@@ -175,29 +176,33 @@ struct Call {
     int err;
 };
 
-// A thread's Call on the current device, kept between its calls (48 KB; a
-// cudaMalloc and cudaFree of a small block map and unmap 2 MB each time, about
-// 100 us a call) and released when the thread ends.  Every call waits for its
-// work, so the thread's next one finds it free; one that a device reset took
-// away is allocated anew.
-struct CallBuf {
-    Call *p = nullptr;
-    ~CallBuf() { if (p) cudaFree(p); }
+// A call's Call on the current device: one of kCallSlots in the library's own
+// module (their addresses looked up by every call, so they follow the module
+// through a device reset), taken for the duration of the call, which waits for
+// its work; a call beyond kCallSlots at a time allocates one.  (A cudaMalloc
+// and cudaFree of a small block map and unmap 2 MB each time, about 100 us a
+// call.)
+constexpr int kCallSlots = 8;
+__device__ Call g_calls[kCallSlots];
+std::atomic<unsigned> g_calls_taken{0};      // a bit per slot
+
+struct CallSlot {
+    int slot = -1;
+    DevBuf own;
+    ~CallSlot() { if (slot >= 0) g_calls_taken.fetch_and(~(1u << slot)); }
     Call *get()
     {
-        int dev = 0;
-        cudaPointerAttributes a;
-        if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-        if (p && cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeDevice) {
-            if (a.device == dev) return p;
-            cudaFree(p);
+        unsigned taken = g_calls_taken.load();
+        while (slot < 0 && ~taken & ((1u << kCallSlots) - 1)) {
+            int k = 0;
+            while (taken >> k & 1) ++k;
+            if (g_calls_taken.compare_exchange_weak(taken, taken | 1u << k)) slot = k;
         }
-        cudaGetLastError();
-        p = nullptr;
-        return cudaMalloc(&p, sizeof(Call)) == cudaSuccess ? p : p = nullptr;
+        if (slot < 0) return own.alloc(sizeof(Call)) ? nullptr : own.as<Call>();
+        void *p = nullptr;
+        return cudaGetSymbolAddress(&p, g_calls) == cudaSuccess ? static_cast<Call *>(p) + slot : nullptr;
     }
 };
-thread_local CallBuf call_buf;
 
 }  // namespace
 
@@ -212,7 +217,8 @@ int des_mlp_forward(const des_mlp *net, const float *x, long long n, float *y)
     std::memcpy(h[0].params, P.data(), sizeof(h[0].params));
     Rows rx, ry;
     int rc;
-    Call *c = call_buf.get();
+    CallSlot slot;
+    Call *c = slot.get();
     if (!c) return DES_ERR_NOMEM;
     // (outputs over the inputs: a tile's would be written over rows that other
     // tiles have yet to read)
@@ -238,7 +244,8 @@ int des_mlp_loss_grad(const des_mlp *net, const float *x, const float *y, long l
     std::memcpy(h[0].params, P.data(), sizeof(h[0].params));
     Rows rx, ry;
     int rc;
-    Call *c = call_buf.get();
+    CallSlot slot;
+    Call *c = slot.get();
     if (!c) return DES_ERR_NOMEM;
     if ((rc = rx.open(x, sizeof(float) * n * kMlpIn, true)) || (rc = ry.open(y, sizeof(float) * n * kMlpOut, true)))
         return rc;
