@@ -696,17 +696,22 @@ __global__ void __launch_bounds__(kSmallBlock) k_fe_c_quad(Dev d)
     const int e = live ? e_ : d.nelem - 1;
     const size_t E = d.nelem;
     const int n = reinterpret_cast<const int *>(d.conn)[4 * (size_t)e + i];
+    // lane k < 3 has the k-th normal stress to itself: it is corrected in place,
+    // so no other lane may read it from memory (lanes of a warp run in any order
+    // between barriers); the shear stresses are not written
+    const bool mine = live && i < 3;
+    double sn = mine ? d.stress[i * E + e] : 0.0;
     double s[6];
-    load6(d.stress, E, e, s);
+#pragma unroll
+    for (int k = 3; k < 6; ++k) s[k] = d.stress[k * E + e];
     const double g[3] = {d.shp[(size_t)i * E + e], d.shp[(size_t)(4 + i) * E + e], d.shp[(size_t)(8 + i) * E + e]};
     const double vol = d.vol[e], dp = d.dp[e], a = d.ntmp[n], T = d.T[n];
     const double dpe = sf::add0(quad_get(a, 0)) + quad_get(a, 1) + quad_get(a, 2) + quad_get(a, 3);
     const double ddp = sf::div3(-dp + sf::quarter(dpe));
+    sn += ddp;
+    if (mine) d.stress[i * E + e] = sn;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        s[k] += ddp;
-        if (live && i == k) d.stress[k * E + e] = s[k];
-    }
+    for (int k = 0; k < 3; ++k) s[k] = quad_get(sn, k);
     const double Tm = elem_mean4(quad_get(T, 0), quad_get(T, 1), quad_get(T, 2), quad_get(T, 3));
     double buoy = 0;
     if (K.gravity != 0) buoy = sf::quarter(sf::mul(mat_rho(K.M, K.M.mix[d.mix[e]], Tm), K.gravity));
