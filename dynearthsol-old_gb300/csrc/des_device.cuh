@@ -167,7 +167,9 @@ __device__ __forceinline__ int visc_clipped(const MatTable &M, const Mix &x, dou
 __device__ __forceinline__ double mat_visc(const MatTable &M, const Mix &x, double T,
                                            const double *srate)
 {
-    if (const int c = visc_clipped(M, x, T, srate))
+    // (the clip's test only where every material's viscosity is a positive
+    // number: it does not look at absent ones, whose term can be 0 / 0)
+    if (const int c = M.visc_plain ? visc_clipped(M, x, T, srate) : 0)
         return c > 0 ? smin(smax(M.visc_max, M.visc_min), M.visc_max) : smin(M.visc_min, M.visc_max);
     double edot = sf::root(second_invariant2(srate));
     edot = smax(edot, 1e-30);
