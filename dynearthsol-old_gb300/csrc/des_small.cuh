@@ -607,19 +607,30 @@ __global__ void __launch_bounds__(kSmallBlock) k_ea_quad(Dev d, int e0, unsigned
         if (live && i == 0) d.c_mass[e] = sf::quarter(sf::mul(K.is_qs ? x.rho_qs : rT, vol));
         if (live && i == 1 && K.thermal) d.c_tmass[e] = sf::quarter(sf::mul(sf::mul(rT, x.cp), vol));
     }
-    // spin and next strain rate
+    // spin and next strain rate (as k_ea_rotate forms them: half the brackets'
+    // sum, exact while every operand of the element is in sf::unpack's range)
     double D[3], u[3];
     {
-        double p[9];
-        products<9>({v[0], v[1], v[2], v[0], v[1], v[0], v[2], v[1], v[2]},
-                    {g[0], g[1], g[2], g[1], g[0], g[2], g[0], g[2], g[1]}, p);
-        __syncwarp();                    // (the coordinates have been read)
+        uint32_t far = 0;
+        sf::Op ov[3], og[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            s_x[k][threadIdx.x] = p[k];
-            s_x[3 + k][threadIdx.x] = p[3 + 2 * k] + p[4 + 2 * k];
-            s_x[6 + k][threadIdx.x] = p[3 + 2 * k] - p[4 + 2 * k];
+            ov[k] = sf::unpack(v[k], far);
+            og[k] = sf::unpack(g[k], far);
         }
+        far = max(far, __shfl_xor_sync(0xffffffffu, far, 1, 4));
+        far = max(far, __shfl_xor_sync(0xffffffffu, far, 2, 4));
+        const double xy = sf::prod(ov[0], og[1]), yx = sf::prod(ov[1], og[0]), xz = sf::prod(ov[0], og[2]),
+                     zx = sf::prod(ov[2], og[0]), yz = sf::prod(ov[1], og[2]), zy = sf::prod(ov[2], og[1]);
+        __syncwarp();                    // (the coordinates have been read)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s_x[k][threadIdx.x] = sf::prod(ov[k], og[k]);
+        s_x[3][threadIdx.x] = xy + yx;
+        s_x[4][threadIdx.x] = xz + zx;
+        s_x[5][threadIdx.x] = yz + zy;
+        s_x[6][threadIdx.x] = xy - yx;
+        s_x[7][threadIdx.x] = xz - zx;
+        s_x[8][threadIdx.x] = yz - zy;
         __syncwarp();
         double Dk = sf::add0(s_x[kk][base]), tk = sf::add0(s_x[3 + kk][base]), uk = sf::add0(s_x[6 + kk][base]);
 #pragma unroll
@@ -628,9 +639,17 @@ __global__ void __launch_bounds__(kSmallBlock) k_ea_quad(Dev d, int e0, unsigned
             tk += s_x[3 + kk][base + j];
             uk += s_x[6 + kk][base + j];
         }
+        tk = sf::half(tk);
+        if (live && !sf::in_range(far)) {
+            double r[9];
+            ea_rates_exact(d, e, r);
+            Dk = kk == 0 ? r[0] : kk == 1 ? r[1] : r[2];
+            tk = kk == 0 ? r[3] : kk == 1 ? r[4] : r[5];
+            uk = 2 * (kk == 0 ? r[6] : kk == 1 ? r[7] : r[8]);
+        }
         if (live && i < 3) {
             d.srate_next[kk * E + e] = Dk;
-            d.srate_next[(3 + kk) * E + e] = sf::half(tk);
+            d.srate_next[(3 + kk) * E + e] = tk;
         }
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
