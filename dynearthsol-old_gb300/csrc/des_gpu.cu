@@ -51,6 +51,7 @@ struct des_gpu {
     cudaGraphExec_t graph_many = nullptr; // kGraphSteps steps
     bool primed = false;
     bool mass_valid = false;              // the clock's mass_valid, as the queued work leaves it
+    int lanes = DES_LANES_BY_SIZE;        // which form of the passes runs
     int prec = DES_PREC_FP64;
     DevF f;
     ConstsF hF;
@@ -612,13 +613,15 @@ const int kQuadElemsEa[2] = {280, 170}, kQuadElemsEc = 180;      // E-A: [FP64, 
 // FP32 E-B with the exact returns in place / over the list: 9.6 / 13.4 at 27.7k elements, on yielding boxes 54.9 / 61.8 at
 // 14.4k, 61.9 / 64.4 at 54k, 119 / 80 at 240k
 const int kDirectReturns = 300;
-bool octets(const des_gpu *g, int pass)
+// n nodes (elements) within per_sm per multiprocessor, or as the handle is told
+bool small_mesh(const des_gpu *g, long long n, int per_sm)
 {
-    return g->nnode <= kOctetNodes[g->prec == DES_PREC_FP32][pass] * g->sms;
+    return g->lanes == DES_LANES_BY_SIZE ? n <= (long long)per_sm * g->sms : g->lanes == DES_LANES_SHARED;
 }
-bool quads_ea(const des_gpu *g) { return g->nelem <= kQuadElemsEa[g->prec == DES_PREC_FP32] * g->sms; }
-bool direct_returns(const des_gpu *g) { return !g->closure && g->nelem <= kDirectReturns * g->sms; }
-bool quads_ec(const des_gpu *g) { return g->nelem <= kQuadElemsEc * g->sms; }
+bool octets(const des_gpu *g, int pass) { return small_mesh(g, g->nnode, kOctetNodes[g->prec == DES_PREC_FP32][pass]); }
+bool quads_ea(const des_gpu *g) { return small_mesh(g, g->nelem, kQuadElemsEa[g->prec == DES_PREC_FP32]); }
+bool direct_returns(const des_gpu *g) { return !g->closure && small_mesh(g, g->nelem, kDirectReturns); }
+bool quads_ec(const des_gpu *g) { return small_mesh(g, g->nelem, kQuadElemsEc); }
 
 // the first kernel of pass E-B over the element blocks [b0, b1)
 void launch_eb_first(des_gpu *g, int b0, int b1)
@@ -1408,6 +1411,14 @@ static int upload_fields(des_gpu *g, const des_state_view *h, unsigned mask)
         DES_LAUNCH();
     }
     g->primed = false;
+    return DES_OK;
+}
+
+int des_gpu_set_lanes(des_gpu *g, int lanes)
+{
+    if (!g || lanes < DES_LANES_BY_SIZE || lanes > DES_LANES_SHARED) return DES_ERR_ARG;
+    drop_graphs(g);
+    g->lanes = lanes;
     return DES_OK;
 }
 
@@ -2313,6 +2324,7 @@ int des_gpu_remesh(des_gpu *g, const des_mesh_view *mesh, const des_state_view *
             return fail(DES_ERR_CUDA);
         ng->closure = true;
     }
+    ng->lanes = g->lanes;
     // averaging restarts with the next step (remeshing falls on an
     // interval's last step, output.cxx:229-233)
     if (g->avg_interval > 0 && (rc = des_gpu_set_averaging(ng, g->avg_interval))) return fail(rc);

@@ -65,6 +65,7 @@ def lib():
     L.des_gpu_device_bytes.argtypes = [C.c_void_p]
     L.des_gpu_device_bytes.restype = C.c_longlong
     L.des_gpu_kernels_per_step.argtypes = [C.c_void_p]
+    L.des_gpu_set_lanes.argtypes = [C.c_void_p, C.c_int]
     L.des_gpu_softf64_check.argtypes = [C.c_int, C.c_longlong, C.c_ulonglong, P(C.c_ulonglong)]
     L.des_gpu_time_steps.argtypes = [C.c_void_p, C.c_int, P(C.c_double)]
     L.des_gpu_profile_steps.argtypes = [C.c_void_p, C.c_int, P(C.c_double)]
@@ -298,6 +299,10 @@ class Device:
         """Installs an abi.Mlp as the learned closure (None removes it)."""
         _ck(lib().des_gpu_set_closure(self.h, C.byref(net) if net is not None else None),
             "des_gpu_set_closure")
+
+    def set_lanes(self, lanes):
+        """Which form of the step's kernels runs (abi.LANES_*)."""
+        _ck(self.L.des_gpu_set_lanes(self.h, lanes), "des_gpu_set_lanes")
 
     @property
     def kernels_per_step(self):

@@ -29,6 +29,7 @@ RH_ELASTIC, RH_VISCOUS, RH_PLASTIC = 1, 2, 4
 RH_MAXWELL, RH_EP, RH_EVP = 3, 5, 7
 
 PREC_FP64, PREC_FP32 = 0, 1
+LANES_BY_SIZE, LANES_ALONE, LANES_SHARED = 0, 1, 2
 
 F_COORD = 1 << 0
 F_VEL = 1 << 1

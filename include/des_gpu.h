@@ -523,6 +523,11 @@ const char *des_gpu_error_string(int code);
 long long   des_gpu_device_bytes(const des_gpu *g);
 /* number of kernels one des_gpu_step launches per step */
 int         des_gpu_kernels_per_step(const des_gpu *g);
+/* Which form of the step's kernels runs, for checks and timing: one thread per
+ * node and element, or lanes that share one (made for small meshes, right on
+ * any), by default as the mesh's size asks.  The results are the same bits. */
+enum { DES_LANES_BY_SIZE = 0, DES_LANES_ALONE = 1, DES_LANES_SHARED = 2 };
+int         des_gpu_set_lanes(des_gpu *g, int lanes);
 /* Self-check of the integer-pipe FP64 arithmetic that the step kernels use
  * in place of FP64 unit instructions (no reference counterpart): n seeded
  * pseudo-random operands per kind on `device`, compared bit for bit with the
