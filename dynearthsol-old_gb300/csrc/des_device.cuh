@@ -41,6 +41,7 @@ struct Mix {
 struct MatTable {
     int    nmat, nmix;
     double rho0[kMaxMat], alpha[kMaxMat];
+    int    rho_plain;              // for |T| < 2^600 every density is finite
     double vexp_pw[kMaxMat], vexp_pw1[kMaxMat], vcoef_pow[kMaxMat], vQ[kMaxMat], vnR[kMaxMat];
     int    visc_law[kMaxMat];      // the first material with the same four viscosity constants
     int    visc_plain;             // for 1e-30 <= edot <= 1e30 and T > 0 every viscosity is a positive number
@@ -124,10 +125,13 @@ __device__ __forceinline__ double mat_rho(const MatTable &M, const Mix &x, doubl
         int m = x.single;
         return sf::mul(M.rho0[m], 1 - sf::mul(M.alpha[m], TinCelsius));
     }
-    // (absent materials add +0)
+    // absent materials add a zero while their density is finite (an infinite
+    // one's term is inf * 0 in the reference)
+    const bool skip = M.rho_plain && ((uint32_t)(sf::bits(TinCelsius) >> 32) & 0x7fffffffu) < (1023u + 600u) << 20;
+    const int terms = skip ? x.npresent : M.nmat;
     double result = 0;
-    for (int k = 0; k < x.npresent; k++) {
-        const int m = x.present[k];
+    for (int k = 0; k < terms; k++) {
+        const int m = skip ? x.present[k] : k;
         result += sf::mul(sf::mul(M.rho0[m], 1 - sf::mul(M.alpha[m], TinCelsius)), (double)x.count[m]);
     }
     return sf::div(result, (double)x.n);

@@ -240,8 +240,9 @@ int build_consts(des_gpu *g)
     }
     M.vlog_min = (float)std::log2(p.visc_min);
     M.vlog_max = (float)std::log2(p.visc_max);
-    M.visc_plain = 1;
+    M.visc_plain = M.rho_plain = 1;
     for (int m = 0; m < g->nmat; ++m) {
+        if (!(std::fabs(M.rho0[m]) < 1e60 && std::fabs(M.alpha[m]) < 1e60)) M.rho_plain = 0;
         const double span = 30 * std::fabs(M.vexp_pw[m]), base = std::log10(0.25e6 * M.vcoef_pow[m]);
         if (!(base - span > -280 && base + span < 280 && span < 280 && M.vQ[m] / M.vnR[m] >= 0)) M.visc_plain = 0;
     }
