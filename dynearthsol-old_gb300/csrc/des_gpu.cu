@@ -904,9 +904,9 @@ __device__ __forceinline__ unsigned long long check_mix(unsigned long long z)
     return z ^ (z >> 31);
 }
 
-// sf::mul, sf::div, sf::root, sf::to_float, sf::add0, sf::twice, sf::half, sf::div6, sf::div3
-// and sf::quarter against the FP64 unit's multiply, conversion, addition and
-// division
+// every routine of des_softf64.cuh that the kernels call against the FP64
+// unit's own multiplication, division, root, addition, comparison and
+// conversion
 __global__ void k_softf64_check(unsigned long long *bad, long long n, unsigned long long seed)
 {
     unsigned long long nb[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -933,6 +933,30 @@ __global__ void k_softf64_check(unsigned long long *bad, long long n, unsigned l
         nb[0] += sf::bits(h) != sf::bits(g) && !(h != h && g != g);
         h = __dsqrt_rn(fabs(x1)), g = sf::root(fabs(x1));
         nb[1] += sf::bits(h) != sf::bits(g);
+        // sums of operands near 1, of a number and its neighbour or opposite (the
+        // cancellations sum_diff and sum leave to the FP64 unit are rare), and of
+        // positive numbers
+        const double z = (i & 3) ? y1 : sf::from_bits((sf::bits(x1) + r2 % 5 - 2) ^ (r2 & sf::kSign));
+        bool rare = false;
+        double sum, diff;
+        sf::sum_diff(x1, z, sum, diff, rare);
+        nb[1] += !rare && (sf::bits(sum) != sf::bits(__dadd_rn(x1, z)) || sf::bits(diff) != sf::bits(__dsub_rn(x1, z)));
+        rare = false;
+        sum = sf::sum(x1, z, rare);
+        nb[1] += !rare && sf::bits(sum) != sf::bits(__dadd_rn(x1, z));
+        sf::PosSum pos = sf::pos_first(fabs(x1));
+        double acc = fabs(x1);
+        for (int k = 1; k < 6; ++k) {
+            const unsigned long long r = check_mix(r1 + k);
+            const double term = sf::from_bits((r & 0x000fffffffffffffull) | (((sf::bits(x1) >> 52 & 0x7ff) - 3 + r % 7) << 52));
+            sf::pos_add(pos, term);
+            acc = __dadd_rn(acc, term);
+        }
+        nb[1] += sf::exact(pos) && sf::bits(sf::value(pos)) != sf::bits(acc);
+        nb[0] += sf::less(x, y) != (x < y);
+        nb[1] += sf::less(x1, z) != (x1 < z);
+        const float w = __uint_as_float((unsigned)(r1 >> 32));
+        nb[3] += sf::bits((double)w) != sf::bits(sf::widen(w)) && w == w;
         float hf = __double2float_rn(x), gf = sf::to_float(x);
         nb[2] += __float_as_uint(hf) != __float_as_uint(gf) && !(hf != hf && gf != gf);
         hf = __double2float_rn(xf);

@@ -531,10 +531,12 @@ int         des_gpu_set_lanes(des_gpu *g, int lanes);
 /* Self-check of the integer-pipe FP64 arithmetic that the step kernels use
  * in place of FP64 unit instructions (no reference counterpart): n seeded
  * pseudo-random operands per kind on `device`, compared bit for bit with the
- * device's own FP64 instructions.  mismatches[0..9]: multiply, divide and
- * square root on any bit patterns, the same on operands near 1, conversion to
- * FP32 on any bit patterns, conversion within the FP32 range, 0 + x, 2 x, x / 2, x / 6,
- * x / 3, x / 4 (the last six on any bit patterns and on exponents 0-8). */
+ * device's own FP64 instructions.  mismatches[0..9]: multiply, divide, square
+ * root and compare on any bit patterns; the same, sums and differences (with
+ * cancellation, and of positive numbers) on operands near 1; conversion to
+ * FP32 on any bit patterns; conversion within the FP32 range and from any FP32
+ * number; 0 + x, 2 x, x / 2, x / 6, x / 3, x / 4 (the last six on any bit
+ * patterns and on exponents 0-8). */
 int         des_gpu_softf64_check(int device, long long n, unsigned long long seed,
                                   unsigned long long mismatches[10]);
 
