@@ -27,58 +27,33 @@
 
 namespace des {
 
-// Operands and products of the pass: on the integer pipes (SOFT: sf::prod,
-// exact while the stage's operands are in sf::unpack's range) or on the
-// FP64 unit.  The results are the same bits.  put / get keep an operand in
-// shared memory, in an 8-byte column and (SOFT) a 4-byte column per thread.
-template <bool SOFT>
-struct Num;
+constexpr int kEaBlock = 128;     // threads of a block, in E-A's kernels and E-C
 
-template <>
-struct Num<true> {
-    using Op = sf::Op;
-    __device__ __forceinline__ static Op op(double x, uint32_t &far) { return sf::unpack(x, far); }
-    __device__ __forceinline__ static double mul(const Op &a, const Op &b) { return sf::prod(a, b); }
-    __device__ __forceinline__ static void sum_diff(double x, double y, double &s, double &d, bool &rare)
-    {
-        sf::sum_diff(x, y, s, d, rare);
-    }
-    // a / 2 (an operand in range)
-    __device__ __forceinline__ static Op half(Op a)
-    {
-        a.ex -= a.hi ? 1u << 20 : 0u;
-        return a;
-    }
-    __device__ __forceinline__ static void put(double *w, uint32_t *x, const Op &a)
-    {
-        *w = __hiloint2double((int)a.hi, (int)a.lo);
-        *x = a.ex;
-    }
-    __device__ __forceinline__ static Op get(const double *w, const uint32_t *x)
-    {
-        const double v = *w;
-        Op a;
-        a.lo = (uint32_t)__double2loint(v);
-        a.hi = (uint32_t)__double2hiint(v);
-        a.ex = *x;
-        return a;
-    }
-};
+// Products are on the integer pipes (sf::prod), exact while the stage's
+// operands are in sf::unpack's range; an element with one outside is formed
+// again on the FP64 unit, out of line.
 
-template <>
-struct Num<false> {
-    using Op = double;
-    __device__ __forceinline__ static Op op(double x, uint32_t &) { return x; }
-    __device__ __forceinline__ static double mul(double a, double b) { return a * b; }
-    __device__ __forceinline__ static void sum_diff(double x, double y, double &s, double &d, bool &)
-    {
-        s = x + y;
-        d = x - y;
-    }
-    __device__ __forceinline__ static double half(double a) { return 0.5 * a; }
-    __device__ __forceinline__ static void put(double *w, uint32_t *, double a) { *w = a; }
-    __device__ __forceinline__ static double get(const double *w, const uint32_t *) { return *w; }
-};
+// an operand in shared memory: an 8-byte column and a 4-byte column per thread
+__device__ __forceinline__ void put_op(double *w, uint32_t *x, const sf::Op &a)
+{
+    *w = __hiloint2double((int)a.hi, (int)a.lo);
+    *x = a.ex;
+}
+__device__ __forceinline__ sf::Op get_op(const double *w, const uint32_t *x)
+{
+    const double v = *w;
+    sf::Op a;
+    a.lo = (uint32_t)__double2loint(v);
+    a.hi = (uint32_t)__double2hiint(v);
+    a.ex = *x;
+    return a;
+}
+// a / 2 (an operand in range)
+__device__ __forceinline__ sf::Op half_op(sf::Op a)
+{
+    a.ex -= a.hi ? 1u << 20 : 0u;
+    return a;
+}
 
 // ---- geometry ---------------------------------------------------------------
 
@@ -86,21 +61,19 @@ struct Num<false> {
 // memory, three components each, a column per thread.
 constexpr int kE01 = 0, kE02 = 3, kE03 = 6, kE12 = 9, kE13 = 12, kE23 = 15, kEdgeCols = 18;
 
-template <int BLK>
 __device__ __forceinline__ void load_edge(const double *se, int c, double a[3])
 {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) a[k] = se[(c + k) * BLK];
+    for (int k = 0; k < 3; ++k) a[k] = se[(c + k) * kEaBlock];
 }
 
 // the squared norm of a x b (tri_area2's terms: the facet's cross product up
 // to the sign of both factors or of the whole, which the squares do not see)
-template <int BLK>
 __device__ __forceinline__ double edge_norm2(const double *se, int ca, int cb)
 {
     double a[3], b[3];
-    load_edge<BLK>(se, ca, a);
-    load_edge<BLK>(se, cb, b);
+    load_edge(se, ca, a);
+    load_edge(se, cb, b);
     const double d0 = a[1] * b[2] - a[2] * b[1], d1 = a[2] * b[0] - a[0] * b[2], d2 = a[0] * b[1] - a[1] * b[0];
     return d0 * d0 + d1 * d1 + d2 * d2;
 }
@@ -108,24 +81,22 @@ __device__ __forceinline__ double edge_norm2(const double *se, int ca, int cb)
 // min_height (geometry.cxx:280-293) from the edges: facets (0,1,2): e01 x e02,
 // (0,1,3): e01 x e03, (2,3,0): e02 x e23, (2,3,1): e12 x e23.  Out of line:
 // every tenth step calls it, and its registers stay out of the pass's own.
-template <int BLK>
 static __device__ __noinline__ double edge_min_height(const double *se, double vol)
 {
-    const double m2 = smax(smax(edge_norm2<BLK>(se, kE01, kE02), edge_norm2<BLK>(se, kE01, kE03)),
-                           smax(edge_norm2<BLK>(se, kE02, kE23), edge_norm2<BLK>(se, kE12, kE23)));
+    const double m2 = smax(smax(edge_norm2(se, kE01, kE02), edge_norm2(se, kE01, kE03)),
+                           smax(edge_norm2(se, kE02, kE23), edge_norm2(se, kE12, kE23)));
     return 3 * vol / (sqrt(m2) / 2);
 }
 
 // The stages on the FP64 unit, for an element with an operand outside
 // sf::unpack's range (a subnormal or huge number, an infinity, NaN); out of
 // line, each from what the stage started from.
-template <int BLK>
 static __device__ __noinline__ double ea_volume_exact(const double *se)
 {
     double a[3], b[3], c[3];                 // e01, e12, e23
-    load_edge<BLK>(se, kE01, a);
-    load_edge<BLK>(se, kE12, b);
-    load_edge<BLK>(se, kE23, c);
+    load_edge(se, kE01, a);
+    load_edge(se, kE12, b);
+    load_edge(se, kE23, c);
     return sf::div6(a[0] * (c[1] * b[2] - b[1] * c[2]) + b[0] * (a[1] * c[2] - c[1] * a[2]) +
                     c[0] * (b[1] * a[2] - a[1] * b[2]));
 }
@@ -148,13 +119,14 @@ static __device__ __noinline__ void ea_gradients_exact(const Dev &d, int e, doub
 enum { kVolume = 1, kSaveOld = 2, kMass = 4, kShape = 8, kStep = 16 };
 constexpr int kStepGeometry = kStep | kVolume | kSaveOld | kShape;
 
-template <bool SOFT, int BLK, int MINB, int PARTS>
-__global__ void __launch_bounds__(BLK, MINB) k_ea_geometry(Dev d, int e0, unsigned nblocks, const double *Tsrc)
+template <int PARTS>
+__global__ void __launch_bounds__(kEaBlock, 10) k_ea_geometry(Dev d, int e0, unsigned nblocks, const double *Tsrc)
 {
-    using N = Num<SOFT>;
-    using Op = typename N::Op;
-    __shared__ double s_edge[kEdgeCols * BLK];
-    const int e = e0 + blockIdx.x * BLK + threadIdx.x;
+    using sf::Op;
+    using sf::prod;
+    using sf::unpack;
+    __shared__ double s_edge[kEdgeCols * kEaBlock];
+    const int e = e0 + blockIdx.x * kEaBlock + threadIdx.x;
     const Consts &K = *d.K;
     const bool live = e < d.nelem;
     const int4 c = live ? d.conn[e] : int4{0, 0, 0, 0};
@@ -173,13 +145,13 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_geometry(Dev d, int e0, unsign
                 e01[k] = X[0][k] - X[1][k];
                 e12[k] = X[1][k] - X[2][k];
                 e23[k] = X[2][k] - X[3][k];
-                se[(kE01 + k) * BLK] = e01[k];
-                se[(kE12 + k) * BLK] = e12[k];
-                se[(kE23 + k) * BLK] = e23[k];
+                se[(kE01 + k) * kEaBlock] = e01[k];
+                se[(kE12 + k) * kEaBlock] = e12[k];
+                se[(kE23 + k) * kEaBlock] = e23[k];
                 if (PARTS & kShape) {
-                    se[(kE02 + k) * BLK] = X[0][k] - X[2][k];
-                    se[(kE03 + k) * BLK] = X[0][k] - X[3][k];
-                    se[(kE13 + k) * BLK] = X[1][k] - X[3][k];
+                    se[(kE02 + k) * kEaBlock] = X[0][k] - X[2][k];
+                    se[(kE03 + k) * kEaBlock] = X[0][k] - X[3][k];
+                    se[(kE13 + k) * kEaBlock] = X[1][k] - X[3][k];
                 }
             }
         }
@@ -190,22 +162,22 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_geometry(Dev d, int e0, unsign
             Op a[3], b[3], g[3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                a[k] = N::op(e01[k], far);
-                b[k] = N::op(e12[k], far);
-                g[k] = N::op(e23[k], far);
+                a[k] = unpack(e01[k], far);
+                b[k] = unpack(e12[k], far);
+                g[k] = unpack(e23[k], far);
             }
-            const double c0 = N::mul(g[1], b[2]) - N::mul(b[1], g[2]);
-            const double c1 = N::mul(a[1], g[2]) - N::mul(g[1], a[2]);
-            const double c2 = N::mul(b[1], a[2]) - N::mul(a[1], b[2]);
-            vol = sf::div6(N::mul(a[0], N::op(c0, far)) + N::mul(b[0], N::op(c1, far)) + N::mul(g[0], N::op(c2, far)));
-            if (SOFT && !sf::in_range(far)) vol = ea_volume_exact<BLK>(se);
+            const double c0 = prod(g[1], b[2]) - prod(b[1], g[2]);
+            const double c1 = prod(a[1], g[2]) - prod(g[1], a[2]);
+            const double c2 = prod(b[1], a[2]) - prod(a[1], b[2]);
+            vol = sf::div6(prod(a[0], unpack(c0, far)) + prod(b[0], unpack(c1, far)) + prod(g[0], unpack(c2, far)));
+            if (!sf::in_range(far)) vol = ea_volume_exact(se);
             if (PARTS & kSaveOld) d.vol_old[e] = d.vol[e];
             d.vol[e] = vol;
             if (not_positive(vol)) atomicOr(&d.clk->status, 0x4u);
         } else {
             vol = d.vol[e];
         }
-        if (dt_step) minh = edge_min_height<BLK>(se, vol);
+        if (dt_step) minh = edge_min_height(se, vol);
         if (PARTS & (kMass | kStep)) {
             // compute_mass's element half (geometry.cxx:354-365)
             const Mix &x = K.M.mix[d.mix[e]];
@@ -223,25 +195,25 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_geometry(Dev d, int e0, unsign
             // compute_shape_fn (geometry.cxx:410-452): node i's gradient is
             // (a x b) / 6V with the edges (a, b) = (13, 12) (02, 23) (13, 03) (01, 02)
             uint32_t far = 0;
-            const Op oiv = N::op(sf::div(1.0, sf::mul(6.0, vol)), far);
+            const Op oiv = unpack(sf::div(1.0, sf::mul(6.0, vol)), far);
 #pragma unroll 1
             for (int i = 0; i < 4; ++i) {
                 double ea[3], eb[3], g[3];
-                load_edge<BLK>(se, (0x0c3c >> (4 * i)) & 15, ea);
-                load_edge<BLK>(se, (0x36f9 >> (4 * i)) & 15, eb);
+                load_edge(se, (0x0c3c >> (4 * i)) & 15, ea);
+                load_edge(se, (0x36f9 >> (4 * i)) & 15, eb);
                 Op a[3], b[3];
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    a[k] = N::op(ea[k], far);
-                    b[k] = N::op(eb[k], far);
+                    a[k] = unpack(ea[k], far);
+                    b[k] = unpack(eb[k], far);
                 }
-                g[0] = N::mul(a[1], b[2]) - N::mul(a[2], b[1]);
-                g[1] = N::mul(a[2], b[0]) - N::mul(a[0], b[2]);
-                g[2] = N::mul(a[0], b[1]) - N::mul(a[1], b[0]);
+                g[0] = prod(a[1], b[2]) - prod(a[2], b[1]);
+                g[1] = prod(a[2], b[0]) - prod(a[0], b[2]);
+                g[2] = prod(a[0], b[1]) - prod(a[1], b[0]);
 #pragma unroll
-                for (int k = 0; k < 3; ++k) d.shp[(size_t)(4 * k + i) * E + e] = N::mul(oiv, N::op(g[k], far));
+                for (int k = 0; k < 3; ++k) d.shp[(size_t)(4 * k + i) * E + e] = prod(oiv, unpack(g[k], far));
             }
-            if (SOFT && !sf::in_range(far)) ea_gradients_exact(d, e, vol);
+            if (!sf::in_range(far)) ea_gradients_exact(d, e, vol);
         }
     }
     if (dt_step) dt_reduce_and_finalize(d, minh, live, nblocks);
@@ -277,12 +249,13 @@ static __device__ __noinline__ void ea_rotate_exact(const Dev &d, int e, double 
 enum { kRates = 1, kDvoldt = 2, kRotate = 4, kStepRotate = 8 };
 constexpr int kStepRates = kRates | kDvoldt | kStepRotate;
 
-template <bool SOFT, int BLK, int MINB, int PARTS>
-__global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0, double *out)
+template <int PARTS>
+__global__ void __launch_bounds__(kEaBlock, 8) k_ea_rotate(Dev d, int e0, double *out)
 {
-    using N = Num<SOFT>;
-    using Op = typename N::Op;
-    const int e = e0 + blockIdx.x * BLK + threadIdx.x;
+    using sf::Op;
+    using sf::prod;
+    using sf::unpack;
+    const int e = e0 + blockIdx.x * kEaBlock + threadIdx.x;
     if (e >= d.nelem) return;
     const size_t E = d.nelem;
     const int4 c = d.conn[e];
@@ -302,17 +275,20 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0, double *
         for (int i = 0; i < 4; ++i) {
             const int n = i == 0 ? c.x : i == 1 ? c.y : i == 2 ? c.z : c.w;
             const double *gp = d.shp + (size_t)i * E + e;
-            const Op v0 = N::op(d.vx[n], far), v1 = N::op(d.vy[n], far), v2 = N::op(d.vz[n], far);
+            const Op v0 = unpack(d.vx[n], far), v1 = unpack(d.vy[n], far), v2 = unpack(d.vz[n], far);
             Op g[3];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) g[k] = N::op(gp[4 * k * E], far);
-            const double xx = N::mul(v0, g[0]), yy = N::mul(v1, g[1]), zz = N::mul(v2, g[2]);
+            for (int k = 0; k < 3; ++k) g[k] = unpack(gp[4 * k * E], far);
+            const double xx = prod(v0, g[0]), yy = prod(v1, g[1]), zz = prod(v2, g[2]);
             double tp[3], um[3];
             // (one pair of the three on the integer pipes: E-A takes 861 us on
             // 2.4M elements with none, 830 with one, 833 with two, 858 with all)
-            Num<false>::sum_diff(N::mul(v0, g[1]), N::mul(v1, g[0]), tp[0], um[0], rare);
-            Num<false>::sum_diff(N::mul(v0, g[2]), N::mul(v2, g[0]), tp[1], um[1], rare);
-            N::sum_diff(N::mul(v1, g[2]), N::mul(v2, g[1]), tp[2], um[2], rare);
+            const double xy = prod(v0, g[1]), yx = prod(v1, g[0]), xz = prod(v0, g[2]), zx = prod(v2, g[0]);
+            tp[0] = xy + yx;
+            um[0] = xy - yx;
+            tp[1] = xz + zx;
+            um[1] = xz - zx;
+            sf::sum_diff(prod(v1, g[2]), prod(v2, g[1]), tp[2], um[2], rare);
             if (i == 0) {
                 D[0] = sf::add0(xx);
                 D[1] = sf::add0(yy);
@@ -335,7 +311,7 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0, double *
         }
 #pragma unroll
         for (int k = 0; k < 3; ++k) D[3 + k] = sf::half(t[k]);
-        if (SOFT && (rare || !sf::in_range(far))) {
+        if (rare || !sf::in_range(far)) {
             double r[9];
             ea_rates_exact(d, e, r);
 #pragma unroll
@@ -353,9 +329,9 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0, double *
     // with u) for the others
     if (!(PARTS & (kRotate | kStepRotate)) || ((PARTS & kStepRotate) && !(d.K->rheol & 1))) return;
     uint32_t farw = 0;
-    const Op w3 = N::op(u[0], farw), w4 = N::op(u[1], farw), w5 = N::op(u[2], farw);
+    const Op w3 = unpack(u[0], farw), w4 = unpack(u[1], farw), w5 = unpack(u[2], farw);
     const double dt = (PARTS & kStepRotate) ? d.clk->step_dt : d.clk->dt;
-    const Op odt = N::op(dt, farw), hdt = N::half(odt);
+    const Op odt = unpack(dt, farw), hdt = half_op(odt);
 #pragma unroll 1
     for (int f = 0; f < 2; ++f) {
         double *arr = f ? d.strain : d.stress;
@@ -364,15 +340,15 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_rotate(Dev d, int e0, double *
         uint32_t far = farw;
         Op o[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) o[k] = N::op(s[k], far);
-        const double p3 = N::mul(o[3], w3), p4 = N::mul(o[4], w4), p5 = N::mul(o[5], w5);
-        s[0] += N::mul(odt, N::op(-p3 - p4, far));
-        s[1] += N::mul(odt, N::op(p3 - p5, far));
-        s[2] += N::mul(odt, N::op(p4 + p5, far));
-        s[3] += N::mul(hdt, N::op(N::mul(o[0], w3) - N::mul(o[1], w3) - N::mul(o[4], w5) - N::mul(o[5], w4), far));
-        s[4] += N::mul(hdt, N::op(N::mul(o[0], w4) - N::mul(o[2], w4) + N::mul(o[3], w5) - N::mul(o[5], w3), far));
-        s[5] += N::mul(hdt, N::op(N::mul(o[1], w5) - N::mul(o[2], w5) + N::mul(o[3], w4) + N::mul(o[4], w3), far));
-        if (!SOFT || sf::in_range(far))
+        for (int k = 0; k < 6; ++k) o[k] = unpack(s[k], far);
+        const double p3 = prod(o[3], w3), p4 = prod(o[4], w4), p5 = prod(o[5], w5);
+        s[0] += prod(odt, unpack(-p3 - p4, far));
+        s[1] += prod(odt, unpack(p3 - p5, far));
+        s[2] += prod(odt, unpack(p4 + p5, far));
+        s[3] += prod(hdt, unpack(prod(o[0], w3) - prod(o[1], w3) - prod(o[4], w5) - prod(o[5], w4), far));
+        s[4] += prod(hdt, unpack(prod(o[0], w4) - prod(o[2], w4) + prod(o[3], w5) - prod(o[5], w3), far));
+        s[5] += prod(hdt, unpack(prod(o[1], w5) - prod(o[2], w5) + prod(o[3], w4) + prod(o[4], w3), far));
+        if (sf::in_range(far))
             store6(arr, E, e, s);
         else
             ea_rotate_exact(d, e, arr, dt, 0.5 * u[0], 0.5 * u[1], 0.5 * u[2]);
@@ -399,39 +375,39 @@ static __device__ __noinline__ void ea_conduction_exact(const Dev &d, int e, dou
 // are unrolled (190 -> 174 us for 2.4M elements; the pairs too: 175; the other
 // kernels' loops over nodes unrolled: geometry 229 -> 289, E-C 212 -> 259, for
 // the spills and the longer code).
-template <bool SOFT, int BLK, int MINB>
-__global__ void __launch_bounds__(BLK, MINB) k_ea_conduction(Dev d, int e0)
+__global__ void __launch_bounds__(kEaBlock, 8) k_ea_conduction(Dev d, int e0)
 {
-    using N = Num<SOFT>;
-    using Op = typename N::Op;
-    __shared__ double s_col[18 * BLK];       // the gradients, then the dot products of pairs 01 02 03 12 13 23
-    __shared__ uint32_t s_ex[12 * BLK];
-    const int e = e0 + blockIdx.x * BLK + threadIdx.x;
+    using sf::Op;
+    using sf::prod;
+    using sf::unpack;
+    __shared__ double s_col[18 * kEaBlock];       // the gradients, then the dot products of pairs 01 02 03 12 13 23
+    __shared__ uint32_t s_ex[12 * kEaBlock];
+    const int e = e0 + blockIdx.x * kEaBlock + threadIdx.x;
     if (e >= d.nelem) return;
     const size_t E = d.nelem;
     const int4 c = d.conn[e];
-    double *sg = s_col + threadIdx.x, *sd = sg + 12 * BLK;
+    double *sg = s_col + threadIdx.x, *sd = sg + 12 * kEaBlock;
     uint32_t *sx = s_ex + threadIdx.x;
     uint32_t far = 0;
 #pragma unroll
-    for (int k = 0; k < 12; ++k) N::put(sg + k * BLK, sx + k * BLK, N::op(d.shp[k * E + e], far));   // 4 k + i: dN_i/dx_k
+    for (int k = 0; k < 12; ++k) put_op(sg + k * kEaBlock, sx + k * kEaBlock, unpack(d.shp[k * E + e], far));   // 4 k + i: dN_i/dx_k
 #pragma unroll 1
     for (int q = 0; q < 6; ++q) {
         const int i = (0x211000 >> (4 * q)) & 3, j = (0x332321 >> (4 * q)) & 3;
         double p[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k)
-            p[k] = N::mul(N::get(sg + (4 * k + i) * BLK, sx + (4 * k + i) * BLK),
-                          N::get(sg + (4 * k + j) * BLK, sx + (4 * k + j) * BLK));
-        sd[q * BLK] = p[0] + p[1] + p[2];
+            p[k] = prod(get_op(sg + (4 * k + i) * kEaBlock, sx + (4 * k + i) * kEaBlock),
+                          get_op(sg + (4 * k + j) * kEaBlock, sx + (4 * k + j) * kEaBlock));
+        sd[q * kEaBlock] = p[0] + p[1] + p[2];
     }
     const double kv = sf::mul(d.K->M.mix[d.mix[e]].k, d.vol[e]);
-    const Op okv = N::op(kv, far);
+    const Op okv = unpack(kv, far);
     double Tn[4];
     load_nodal4(d.T, c, Tn);
     Op oT[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) oT[j] = N::op(Tn[j], far);
+    for (int j = 0; j < 4; ++j) oT[j] = unpack(Tn[j], far);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         // the pair number of (i, j), j = 0..3 (the diagonal's nibble unused)
@@ -439,20 +415,20 @@ __global__ void __launch_bounds__(BLK, MINB) k_ea_conduction(Dev d, int e0)
         double p[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const Op g = N::get(sg + (4 * k + i) * BLK, sx + (4 * k + i) * BLK);
-            p[k] = N::mul(g, g);
+            const Op g = get_op(sg + (4 * k + i) * kEaBlock, sx + (4 * k + i) * kEaBlock);
+            p[k] = prod(g, g);
         }
         const double dii = p[0] + p[1] + p[2];
         double diffusion = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const double off = sd[((pairs >> (4 * j)) & 15) * BLK];
-            const double pj = N::mul(N::op(i == j ? dii : off, far), oT[j]);
+            const double off = sd[((pairs >> (4 * j)) & 15) * kEaBlock];
+            const double pj = prod(unpack(i == j ? dii : off, far), oT[j]);
             diffusion = j == 0 ? sf::add0(pj) : diffusion + pj;
         }
-        d.tmp[(size_t)i * E + e] = N::mul(N::op(diffusion, far), okv);
+        d.tmp[(size_t)i * E + e] = prod(unpack(diffusion, far), okv);
     }
-    if (SOFT && !sf::in_range(far)) ea_conduction_exact(d, e, kv);
+    if (!sf::in_range(far)) ea_conduction_exact(d, e, kv);
 }
 
 // ---- E-C: NMD correction, element force vectors ---------------------------------
@@ -466,12 +442,13 @@ static __device__ __noinline__ void ec_force_exact(const Dev &d, int e)
 
 // 12 blocks of 128 per SM (8: 349 us on 3.84M elements, 10: 332, 12: 330)
 // NMD: E-C; without it the force vectors alone (update_force's element half)
-template <bool SOFT, int BLK, int MINB, bool NMD>
-__global__ void __launch_bounds__(BLK, MINB) k_fe_c(Dev d)
+template <bool NMD>
+__global__ void __launch_bounds__(kEaBlock, 12) k_fe_c(Dev d)
 {
-    using N = Num<SOFT>;
-    using Op = typename N::Op;
-    const int e = blockIdx.x * BLK + threadIdx.x;
+    using sf::Op;
+    using sf::prod;
+    using sf::unpack;
+    const int e = blockIdx.x * kEaBlock + threadIdx.x;
     if (e >= d.nelem) return;
     const size_t E = d.nelem;
     const Consts &K = *d.K;
@@ -499,20 +476,20 @@ __global__ void __launch_bounds__(BLK, MINB) k_fe_c(Dev d)
     uint32_t far = 0;
     Op o[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) o[k] = N::op(s[k], far);
-    const Op ov = N::op(d.vol[e], far);
+    for (int k = 0; k < 6; ++k) o[k] = unpack(s[k], far);
+    const Op ov = unpack(d.vol[e], far);
 #pragma unroll 1
     for (int i = 0; i < 4; ++i) {
-        const Op gx = N::op(d.shp[(size_t)i * E + e], far), gy = N::op(d.shp[(size_t)(4 + i) * E + e], far),
-                 gz = N::op(d.shp[(size_t)(8 + i) * E + e], far);
-        const double fx = N::mul(o[0], gx) + N::mul(o[3], gy) + N::mul(o[4], gz);
-        const double fy = N::mul(o[3], gx) + N::mul(o[1], gy) + N::mul(o[5], gz);
-        const double fz = N::mul(o[4], gx) + N::mul(o[5], gy) + N::mul(o[2], gz) + buoy;
-        d.tmp[(size_t)i * E + e] = N::mul(N::op(fx, far), ov);
-        d.tmp[(size_t)(4 + i) * E + e] = N::mul(N::op(fy, far), ov);
-        d.tmp[(size_t)(8 + i) * E + e] = N::mul(N::op(fz, far), ov);
+        const Op gx = unpack(d.shp[(size_t)i * E + e], far), gy = unpack(d.shp[(size_t)(4 + i) * E + e], far),
+                 gz = unpack(d.shp[(size_t)(8 + i) * E + e], far);
+        const double fx = prod(o[0], gx) + prod(o[3], gy) + prod(o[4], gz);
+        const double fy = prod(o[3], gx) + prod(o[1], gy) + prod(o[5], gz);
+        const double fz = prod(o[4], gx) + prod(o[5], gy) + prod(o[2], gz) + buoy;
+        d.tmp[(size_t)i * E + e] = prod(unpack(fx, far), ov);
+        d.tmp[(size_t)(4 + i) * E + e] = prod(unpack(fy, far), ov);
+        d.tmp[(size_t)(8 + i) * E + e] = prod(unpack(fz, far), ov);
     }
-    if (SOFT && !sf::in_range(far)) ec_force_exact(d, e);
+    if (!sf::in_range(far)) ec_force_exact(d, e);
 }
 
 }  // namespace des

@@ -22,7 +22,7 @@ using namespace des;
 
 namespace {
 
-const int kElemBlock = 128;
+const int kElemBlock = kEaBlock;
 const int kNodeBlock = 256;
 const int kStepKernels = 6;
 const int kGraphSteps = 10;  // steps of the larger captured graph
@@ -562,7 +562,7 @@ int begin_fn64(des_gpu *g)
 template <int PARTS>
 void launch_geometry(des_gpu *g, const double *Tsrc)
 {
-    k_ea_geometry<true, 128, 10, PARTS><<<blocks(g->nelem, 128), 128, 0, g->stream>>>(g->d, 0, 0, Tsrc);
+    k_ea_geometry<PARTS><<<blocks(g->nelem, kElemBlock), kElemBlock, 0, g->stream>>>(g->d, 0, 0, Tsrc);
 }
 
 // compute_mass's node half from the element kernel's tmp[0..2]
@@ -577,14 +577,13 @@ void launch_masses(des_gpu *g)
 int prime(des_gpu *g)
 {
     if (g->primed) return DES_OK;
-    if (g->prec == DES_PREC_FP32)
-        kf_prime<<<blocks(g->nelem, kElemBlock), kElemBlock, 0, g->stream>>>(g->f);
-    else
-        {
-            const int eb = blocks(g->nelem, 128);
-            k_ea_rotate<true, 128, 8, kRates | kDvoldt><<<eb, 128, 0, g->stream>>>(g->d, 0, g->d.srate_next);
-            if (g->hK.thermal) k_ea_conduction<true, 128, 8><<<eb, 128, 0, g->stream>>>(g->d, 0);
-        }
+    const int eb = blocks(g->nelem, kElemBlock);
+    if (g->prec == DES_PREC_FP32) {
+        kf_prime<<<eb, kElemBlock, 0, g->stream>>>(g->f);
+    } else {
+        k_ea_rotate<kRates | kDvoldt><<<eb, kElemBlock, 0, g->stream>>>(g->d, 0, g->d.srate_next);
+        if (g->hK.thermal) k_ea_conduction<<<eb, kElemBlock, 0, g->stream>>>(g->d, 0);
+    }
     DES_LAUNCH();
     g->primed = true;
     return DES_OK;
@@ -724,7 +723,7 @@ void launch_pass(des_gpu *g, int k)
             if (quads_ec(g))
                 k_fe_c_quad<<<blocks(4LL * g->nelem, kSmallBlock), kSmallBlock, 0, g->stream>>>(d);
             else
-                k_fe_c<true, 128, 12, true><<<eb, kElemBlock, 0, g->stream>>>(d);
+                k_fe_c<true><<<eb, kElemBlock, 0, g->stream>>>(d);
             break;
         default:
             if (g->hK.stress_bc_sides && d.bf.nbf > 0)
@@ -762,9 +761,9 @@ void launch_ea(des_gpu *g, int b0, int b1)
     } else if (quads_ea(g)) {
         k_ea_quad<<<n * kQuads, kSmallBlock, 0, g->stream>>>(g->d, e0, nb * kQuads);
     } else {
-        k_ea_geometry<true, 128, 10, kStepGeometry><<<n, 128, 0, g->stream>>>(g->d, e0, nb, nullptr);
-        k_ea_rotate<true, 128, 8, kStepRates><<<n, 128, 0, g->stream>>>(g->d, e0, g->d.srate_next);
-        if (g->hK.thermal) k_ea_conduction<true, 128, 8><<<n, 128, 0, g->stream>>>(g->d, e0);
+        k_ea_geometry<kStepGeometry><<<n, kElemBlock, 0, g->stream>>>(g->d, e0, nb, nullptr);
+        k_ea_rotate<kStepRates><<<n, kElemBlock, 0, g->stream>>>(g->d, e0, g->d.srate_next);
+        if (g->hK.thermal) k_ea_conduction<<<n, kElemBlock, 0, g->stream>>>(g->d, e0);
     }
 }
 
@@ -2384,7 +2383,7 @@ int des_gpu_update_temperature(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_ea_conduction<true, 128, 8><<<ELEM_GRID(g)>>>(g->d, 0);
+    k_ea_conduction<<<ELEM_GRID(g)>>>(g->d, 0);
     k_temp_node<<<NODE_GRID(g)>>>(g->d);
     return finish(g);
 }
@@ -2392,7 +2391,7 @@ int des_gpu_update_strain_rate(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_ea_rotate<true, 128, 8, kRates><<<ELEM_GRID(g)>>>(g->d, 0, g->d.srate);
+    k_ea_rotate<kRates><<<ELEM_GRID(g)>>>(g->d, 0, g->d.srate);
     return finish(g);
 }
 int des_gpu_compute_dvoldt(des_gpu *g)
@@ -2434,7 +2433,7 @@ int des_gpu_update_force(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_fe_c<true, 128, 12, false><<<ELEM_GRID(g)>>>(g->d);
+    k_fe_c<false><<<ELEM_GRID(g)>>>(g->d);
     if (g->hK.stress_bc_sides && g->d.bf.nbf > 0)
         k_stress_bc_facets<<<blocks(g->d.bf.nbf, 128), 128, 0, g->stream>>>(g->d);
     k_force_node<<<NODE_GRID(g)>>>(g->d, g->hK.is_qs);
@@ -2497,7 +2496,7 @@ int des_gpu_rotate_stress(des_gpu *g)
 {
     int rc = begin_fn64(g);
     if (rc) return rc;
-    k_ea_rotate<true, 128, 8, kRotate><<<ELEM_GRID(g)>>>(g->d, 0, nullptr);
+    k_ea_rotate<kRotate><<<ELEM_GRID(g)>>>(g->d, 0, nullptr);
     return finish(g);
 }
 int des_gpu_compute_dt(des_gpu *g, double *dt_out)

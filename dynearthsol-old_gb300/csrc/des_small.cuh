@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(kSmallBlock) k_ea_quad(Dev d, int e0, unsigned
     if (rotate) {
         uint32_t farw = 0;
         const sf::Op ow[3] = {sf::unpack(u[0], farw), sf::unpack(u[1], farw), sf::unpack(u[2], farw)};
-        const sf::Op odt = sf::unpack(step_dt, farw), hdt = Num<true>::half(odt);
+        const sf::Op odt = sf::unpack(step_dt, farw), hdt = half_op(odt);
         const sf::Op wk = kk == 0 ? ow[0] : kk == 1 ? ow[1] : ow[2];
         const sf::Op wC = kk == 2 ? ow[1] : ow[2], wD = kk == 0 ? ow[1] : ow[0];       // w5 w5 w4 | w4 w3 w3
         const sf::Op wP = kk == 2 ? ow[1] : ow[0], wQ = kk == 0 ? ow[1] : ow[2];       // w3 w3 w4 | w4 w5 w5
