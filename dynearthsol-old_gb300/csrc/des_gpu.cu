@@ -426,13 +426,14 @@ int build_consts(des_gpu *g)
 // Host rows reachable from the GPU (over NVLink-C2C on GB300) are read and
 // written in place, in one pass with the layout change: page-locked arrays
 // (des_host_register, cudaHostAlloc), and any other host memory where the GPU
-// walks the host's page tables and the pages are there (pages_present).  The rest goes through the staging buffer and
+// walks the host's page tables and the pages are there (pages_present) and
+// may be accessed (pages_allow).  The rest goes through the staging buffer and
 // the copy engine.  The engine moves rows that it has just moved as fast (2.5 GB
 // down 13.9 ms, kernel stores 13.9 from the start of a line on and 16.2 from
 // its middle), but not rows it meets for the first time or after half a second
 // of other work: 48-580 ms for the same 2.5 GB, on one machine and another,
 // where stores take 13.9 ms always.
-const void *mapped(const void *host, size_t bytes)
+const void *mapped(const void *host, size_t bytes, bool write)
 {
     if (reinterpret_cast<uintptr_t>(host) % sizeof(double)) return nullptr;
     cudaPointerAttributes a;
@@ -444,15 +445,15 @@ const void *mapped(const void *host, size_t bytes)
     int dev = 0, walks = 0;
     if (a.type != cudaMemoryTypeUnregistered || cudaGetDevice(&dev) != cudaSuccess) return nullptr;
     cudaDeviceGetAttribute(&walks, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev);
-    return walks && pages_present(host, bytes) ? host : nullptr;
+    return walks && pages_present(host, bytes) && pages_allow(host, bytes, write) ? host : nullptr;
 }
 // the same for n doubles to write, in one range from the first to the last
 double *mapped_rows(double *host, long long n)
 {
     if (n <= 0) return nullptr;
     const size_t last = sizeof(double) * (size_t)(n - 1);
-    const char *first = static_cast<const char *>(mapped(host, last + sizeof(double)));
-    if (!first || mapped(reinterpret_cast<const char *>(host) + last, sizeof(double)) != first + last) return nullptr;
+    const char *first = static_cast<const char *>(mapped(host, last + sizeof(double), true));
+    if (!first || mapped(reinterpret_cast<const char *>(host) + last, sizeof(double), true) != first + last) return nullptr;
     return reinterpret_cast<double *>(const_cast<char *>(first));
 }
 // doubles from the start of dst's 128-byte line to dst
@@ -461,7 +462,7 @@ int past_line(const double *dst) { return (int)(reinterpret_cast<uintptr_t>(dst)
 int upload_field(des_gpu *g, const double *host, double *dst, int ncomp, long long rows)
 {
     if (!host) return DES_ERR_ARG;
-    if (const double *m = static_cast<const double *>(mapped(host, sizeof(double) * rows * ncomp))) {
+    if (const double *m = static_cast<const double *>(mapped(host, sizeof(double) * rows * ncomp, false))) {
         k_aos_to_soa<<<blocks(rows * ncomp, 256), 256, 0, g->stream>>>(m, dst, ncomp, rows, 0, rows);
         DES_LAUNCH();
         return DES_OK;
@@ -502,7 +503,7 @@ int download_field(des_gpu *g, double *host, const double *src, int ncomp, long 
 int upload_field(des_gpu *g, const double *host, float *dst, int ncomp, long long rows)
 {
     if (!host) return DES_ERR_ARG;
-    if (const double *m = static_cast<const double *>(mapped(host, sizeof(double) * rows * ncomp))) {
+    if (const double *m = static_cast<const double *>(mapped(host, sizeof(double) * rows * ncomp, false))) {
         k_aos_to_soa_f<<<blocks(rows * ncomp, 256), 256, 0, g->stream>>>(m, dst, ncomp, rows, 0, rows);
         DES_LAUNCH();
         return DES_OK;
@@ -1384,7 +1385,7 @@ static int upload_fields(des_gpu *g, const des_state_view *h, unsigned mask)
     UP(DES_F_VOLUME, volume_old, d.vol_old, 1, E)
     if (mask & DES_F_STRESS) {
         if (f32) {
-            if (const double *m = static_cast<const double *>(mapped(h->stress, sizeof(double) * 6 * E))) {
+            if (const double *m = static_cast<const double *>(mapped(h->stress, sizeof(double) * 6 * E, false))) {
                 k_stress_split_tiled<<<blocks(E, 256), 256, 0, g->stream>>>(m, f.s0, f.stress, E);
                 DES_LAUNCH();
             } else {

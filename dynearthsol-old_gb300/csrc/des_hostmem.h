@@ -28,4 +28,20 @@ inline bool pages_present(const void *p, size_t bytes)
     return true;
 }
 
+// Whether the first and the last page of the range may be read (written): an
+// array that the program may not write makes the GPU's store a fault of the
+// whole context, where the driver's copy can refuse.  (The pages are brought in
+// as the access would do.  Kernels before Linux 5.14 say no to everything.)
+inline bool pages_allow(const void *p, size_t bytes, bool write)
+{
+#ifndef MADV_POPULATE_READ
+    enum { MADV_POPULATE_READ = 22, MADV_POPULATE_WRITE = 23 };
+#endif
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = reinterpret_cast<uintptr_t>(p) & ~(page - 1),
+                    z = (reinterpret_cast<uintptr_t>(p) + bytes - 1) & ~(page - 1);
+    const int advice = write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ;
+    return !madvise(reinterpret_cast<void *>(a), page, advice) &&
+           (z == a || !madvise(reinterpret_cast<void *>(z), page, advice));
+}
+
 }  // namespace des

@@ -151,7 +151,8 @@ struct Rows {
         int dev = 0, ats = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&ats, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev);
-        host = in_place && ats && reinterpret_cast<uintptr_t>(rows) % 16 == 0 && pages_present(rows, bytes);
+        host = in_place && ats && reinterpret_cast<uintptr_t>(rows) % 16 == 0 && pages_present(rows, bytes) &&
+               pages_allow(rows, bytes, !copy_in);
         if (host) {
             p = const_cast<float *>(rows);
             return DES_OK;

@@ -1,5 +1,6 @@
-// Host check of pages_present (csrc/des_hostmem.h): untouched, touched, partly
-// touched, released and unmapped ranges.  exit 1 on a mismatch.
+// Host check of pages_present and pages_allow (csrc/des_hostmem.h): untouched,
+// touched, partly touched, released, protected and unmapped ranges.  exit 1 on a
+// mismatch.
 #include "des_hostmem.h"
 
 #include <cstdio>
@@ -30,6 +31,27 @@ int main()
     expect("after that page", p + n / 4 + page, n / 2, true);
     munmap(p + n / 2, page);
     expect("one page unmapped", p + n / 4 + page, n / 2, false);
+    auto allow = [&](const char *what, const void *q, size_t bytes, bool write, bool want) {
+        const bool got = des::pages_allow(q, bytes, write);
+        if (got != want) printf("%s, %s: %d\n", what, write ? "write" : "read", got), ++bad;
+    };
+    char *r = p + n / 4 + page;                      // touched pages up to the unmapped one
+    const size_t m = n / 4 - page;
+    r[5] = 17;
+    for (bool write : {false, true}) {
+        allow("ordinary", r, m, write, true);
+        allow("a few bytes", r + 3, 40, write, true);
+        allow("over a page's end", r + page - 8, 16, write, true);
+        allow("into the unmapped page", r, m + 1, write, false);
+    }
+    mprotect(r, page, PROT_READ);
+    allow("first page read-only", r + 8, m - 8, false, true);
+    allow("first page read-only", r + 8, m - 8, true, false);
+    mprotect(r, page, PROT_READ | PROT_WRITE);
+    mprotect(r + m - page, page, PROT_NONE);
+    allow("last page closed", r, m, false, false);
+    allow("last page closed", r, m, true, false);
+    if (r[5] != 17) printf("contents changed\n"), ++bad;
     printf("%d mismatches\n", bad);
     return bad != 0;
 }

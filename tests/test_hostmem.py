@@ -1,5 +1,6 @@
-"""pages_present, which decides whether ordinary host rows are read and written
-in place (untouched pages come in one GPU fault at a time)."""
+"""pages_present and pages_allow, which decide whether ordinary host rows are
+read and written in place (untouched pages come in one GPU fault at a time, and
+a store to a page that the program may not write would end the context)."""
 import subprocess
 from pathlib import Path
 
