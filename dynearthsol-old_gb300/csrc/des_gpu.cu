@@ -426,8 +426,7 @@ int build_consts(des_gpu *g)
 // Host rows reachable from the GPU (over NVLink-C2C on GB300) are read and
 // written in place, in one pass with the layout change: page-locked arrays
 // (des_host_register, cudaHostAlloc), and any other host memory where the GPU
-// walks the host's page tables and the pages are there (pages_present) and
-// may be accessed (pages_allow).  The rest goes through the staging buffer and
+// walks the host's page tables (pages_ready).  The rest goes through the staging buffer and
 // the copy engine.  The engine moves rows that it has just moved as fast (2.5 GB
 // down 13.9 ms, kernel stores 13.9 from the start of a line on and 16.2 from
 // its middle), but not rows it meets for the first time or after half a second
@@ -445,7 +444,7 @@ const void *mapped(const void *host, size_t bytes, bool write)
     int dev = 0, walks = 0;
     if (a.type != cudaMemoryTypeUnregistered || cudaGetDevice(&dev) != cudaSuccess) return nullptr;
     cudaDeviceGetAttribute(&walks, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev);
-    return walks && pages_present(host, bytes) && pages_allow(host, bytes, write) ? host : nullptr;
+    return walks && pages_ready(host, bytes, write) ? host : nullptr;
 }
 // the same for n doubles to write, in one range from the first to the last
 double *mapped_rows(double *host, long long n)

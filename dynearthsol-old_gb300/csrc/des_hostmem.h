@@ -1,47 +1,70 @@
-// Whether a kernel may read or write ordinary host memory in place.
+// Makes ordinary host memory ready for a kernel to read or write in place.
 #pragma once
 #include <sys/mman.h>
 #include <unistd.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <exception>
+#include <thread>
 #include <vector>
+
+#ifndef MADV_POPULATE_READ
+#define MADV_POPULATE_READ 22
+#define MADV_POPULATE_WRITE 23
+#endif
 
 namespace des {
 
-// Whether every page of the range is in memory (true below 1 MB without a
-// look).  A page that nobody has touched yet is brought in by the GPU's access
-// one fault at a time, 5 to 10 times slower than by a copy through the driver:
-// a frame of 2.4M elements into fresh arrays 84 ms against 13.5, uploading
-// untouched zeros 205 against 23, the closure's outputs of 4M samples 42
-// against 7.3; on touched pages it is in place that is faster (frame 2.5
-// against 2.9, upload 3.85 against 4.8).  Unmapped ranges are not in memory.
-inline bool pages_present(const void *p, size_t bytes)
+// whether every page from a to e (page boundaries) is in memory
+inline bool pages_present(uintptr_t a, uintptr_t e)
 {
-    if (bytes < (size_t)1 << 20) return true;
-    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = reinterpret_cast<uintptr_t>(p) & ~(page - 1),
-                    e = reinterpret_cast<uintptr_t>(p) + bytes;
-    std::vector<unsigned char> in((e - a + page - 1) / page);
-    if (mincore(reinterpret_cast<void *>(a), e - a, in.data())) return false;
-    for (unsigned char c : in)
-        if (!(c & 1)) return false;
-    return true;
+    std::vector<unsigned char> in((e - a) / (size_t)sysconf(_SC_PAGESIZE));
+    return !mincore(reinterpret_cast<void *>(a), e - a, in.data()) &&
+           std::all_of(in.begin(), in.end(), [](unsigned char c) { return c & 1; });
 }
 
-// Whether the first and the last page of the range may be read (written): an
-// array that the program may not write makes the GPU's store a fault of the
-// whole context, where the driver's copy can refuse.  (The pages are brought in
-// as the access would do.  Kernels before Linux 5.14 say no to everything.)
-inline bool pages_allow(const void *p, size_t bytes, bool write)
+// the pages from a to e brought in as the access would do, a thread for every
+// 16 MB up to four; false where one may not be accessed
+inline bool populate(uintptr_t a, uintptr_t e, int advice)
 {
-#ifndef MADV_POPULATE_READ
-    enum { MADV_POPULATE_READ = 22, MADV_POPULATE_WRITE = 23 };
-#endif
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const int parts = (int)std::min<size_t>(4, std::max<size_t>(1, (e - a) >> 24));
+    const size_t each = ((e - a) / parts + page - 1) / page * page;
+    std::atomic<bool> ok{true};
+    auto part = [&](uintptr_t from) {
+        if (from < e && madvise(reinterpret_cast<void *>(from), std::min(each, (size_t)(e - from)), advice)) ok = false;
+    };
+    std::vector<std::thread> others;
+    int k = 1;
+    try {
+        others.reserve(parts);
+        for (; k < parts; ++k) others.emplace_back(part, a + k * each);
+    } catch (const std::exception &) {       // (no thread to be had: the rest here)
+    }
+    for (; k < parts; ++k) part(a + k * each);
+    part(a);
+    for (std::thread &t : others) t.join();
+    return ok;
+}
+
+// Whether a kernel may read (write) the range in place.  A page that nobody has
+// touched yet is brought in here: by the GPU's own access it takes a fault of
+// its own, 5 to 10 times as long (a frame of 2.4M elements into fresh arrays 84
+// ms; a copy through the driver 13.4 while the copy engine is warm, three times
+// that while it is not).  And an access that the program may not make itself is
+// left for the driver's copy to refuse: the GPU's would end the context.  Pages
+// that are there cost a look (6 us for 128 MB) and a try of the first and the
+// last.  (Before Linux 5.14: no.)
+inline bool pages_ready(const void *p, size_t bytes, bool write)
+{
     const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = reinterpret_cast<uintptr_t>(p) & ~(page - 1),
-                    z = (reinterpret_cast<uintptr_t>(p) + bytes - 1) & ~(page - 1);
+                    e = (reinterpret_cast<uintptr_t>(p) + bytes + page - 1) & ~(page - 1);
     const int advice = write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ;
-    return !madvise(reinterpret_cast<void *>(a), page, advice) &&
-           (z == a || !madvise(reinterpret_cast<void *>(z), page, advice));
+    if (e - a <= 2 * page || !pages_present(a, e)) return populate(a, e, advice);
+    return populate(a, a + page, advice) && populate(e - page, e, advice);
 }
 
 }  // namespace des

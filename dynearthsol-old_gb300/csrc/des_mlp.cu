@@ -136,8 +136,8 @@ int read_err(const int *derr)
 
 // Rows of the caller's as a kernel reads or writes them: in place where the
 // GPU reaches any host memory through the host's page tables (GB300 over
-// NVLink-C2C), the rows are 16-byte aligned with their pages in memory and the
-// caller allows it, else through a device copy.
+// NVLink-C2C, pages_ready), the rows are 16-byte aligned and the caller allows
+// it, else through a device copy.
 // In place, 250k samples' rows cross the link under the kernel, where a device
 // copy had its own allocation, transfer and release (with the kept Call, below:
 // forward 700 -> 355 us, 135 of it the caller's fresh output pages; loss and
@@ -151,8 +151,8 @@ struct Rows {
         int dev = 0, ats = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&ats, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev);
-        host = in_place && ats && reinterpret_cast<uintptr_t>(rows) % 16 == 0 && pages_present(rows, bytes) &&
-               pages_allow(rows, bytes, !copy_in);
+        host = in_place && ats && reinterpret_cast<uintptr_t>(rows) % 16 == 0 &&
+               pages_ready(rows, bytes, !copy_in);
         if (host) {
             p = const_cast<float *>(rows);
             return DES_OK;

@@ -1,6 +1,6 @@
-// Host check of pages_present and pages_allow (csrc/des_hostmem.h): untouched,
-// touched, partly touched, released, protected and unmapped ranges.  exit 1 on a
-// mismatch.
+// Host check of csrc/des_hostmem.h on untouched, touched, partly touched,
+// released, protected and unmapped ranges: what pages_ready allows, that the
+// pages are there afterwards, and that no byte changes.  exit 1 on a mismatch.
 #include "des_hostmem.h"
 
 #include <cstdio>
@@ -8,50 +8,56 @@
 
 int main()
 {
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE), n = (size_t)64 << 20;
-    char *p = static_cast<char *>(mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
-    if (p == MAP_FAILED) return 1;
-    madvise(p, n, MADV_NOHUGEPAGE);
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE), n = (size_t)34 << 20;
     int bad = 0;
-    auto expect = [&](const char *what, const void *q, size_t bytes, bool want) {
-        const bool got = des::pages_present(q, bytes);
-        if (got != want) printf("%s: %d\n", what, got), ++bad;
+    auto fail = [&](const char *what) { printf("%s\n", what), ++bad; };
+    auto map = [&] { return static_cast<char *>(mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0)); };
+    auto present = [&](const char *p, size_t bytes) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p) & ~(page - 1);
+        return des::pages_present(a, (reinterpret_cast<uintptr_t>(p) + bytes + page - 1) & ~(page - 1));
     };
-    expect("untouched", p, n, false);
-    expect("small, untouched", p, ((size_t)1 << 20) - 1, true);
-    std::memset(p, 1, n / 2);
-    expect("touched half", p, n / 2, true);
-    expect("touched half, off a page", p + 24, n / 2 - 48, true);
-    expect("one page more", p, n / 2 + page, false);
-    expect("one byte more", p + 8, n / 2 - 7, false);
-    std::memset(p, 1, n);
-    expect("touched", p, n, true);
-    madvise(p + n / 4, page, MADV_DONTNEED);
-    expect("one page given back", p, n, false);
-    expect("after that page", p + n / 4 + page, n / 2, true);
-    munmap(p + n / 2, page);
-    expect("one page unmapped", p + n / 4 + page, n / 2, false);
-    auto allow = [&](const char *what, const void *q, size_t bytes, bool write, bool want) {
-        const bool got = des::pages_allow(q, bytes, write);
-        if (got != want) printf("%s, %s: %d\n", what, write ? "write" : "read", got), ++bad;
-    };
-    char *r = p + n / 4 + page;                      // touched pages up to the unmapped one
-    const size_t m = n / 4 - page;
-    r[5] = 17;
+    // untouched ranges of one byte to two threads' worth, from a page's start and its middle
+    for (size_t bytes : {(size_t)1, page, 2 * page + 1, ((size_t)33 << 20) + 5})
+        for (size_t from : {(size_t)0, (size_t)24}) {
+            char *p = map();
+            if (present(p + from, bytes)) fail("untouched pages present");
+            if (!des::pages_ready(p + from, bytes, true)) fail("untouched pages refused");
+            if (!present(p + from, bytes)) fail("pages not brought in");
+            for (size_t i = 0; i < bytes; i += 511)
+                if (p[from + i]) return fail("a byte changed"), 1;
+            munmap(p, n);
+            p = map();
+            if (!des::pages_ready(p + from, bytes, false)) fail("untouched pages refused to a reader");
+            munmap(p, n);
+        }
+    char *p = map();
+    for (size_t i = 0; i < n / 2; ++i) p[i] = (char)(i * 7);
+    madvise(p + n / 4, page, MADV_DONTNEED);         // one page back to zeros
     for (bool write : {false, true}) {
-        allow("ordinary", r, m, write, true);
-        allow("a few bytes", r + 3, 40, write, true);
-        allow("over a page's end", r + page - 8, 16, write, true);
-        allow("into the unmapped page", r, m + 1, write, false);
+        if (!des::pages_ready(p, n, write)) fail("partly touched pages refused");
+        if (write && !present(p, n)) fail("partly touched pages not brought in");
     }
-    mprotect(r, page, PROT_READ);
-    allow("first page read-only", r + 8, m - 8, false, true);
-    allow("first page read-only", r + 8, m - 8, true, false);
-    mprotect(r, page, PROT_READ | PROT_WRITE);
-    mprotect(r + m - page, page, PROT_NONE);
-    allow("last page closed", r, m, false, false);
-    allow("last page closed", r, m, true, false);
-    if (r[5] != 17) printf("contents changed\n"), ++bad;
+    for (size_t i = 0; i < n; ++i)
+        if (p[i] != (i < n / 2 && (i < n / 4 || i >= n / 4 + page) ? (char)(i * 7) : 0)) return fail("a byte changed"), 1;
+    struct {
+        const char *what;
+        char *at;
+        int prot;
+        bool read, write;
+    } const closed[] = {{"first page read-only", p, PROT_READ, true, false},
+                        {"last page read-only", p + n - page, PROT_READ, true, false},
+                        {"first page closed", p, PROT_NONE, false, false},
+                        {"last page closed", p + n - page, PROT_NONE, false, false}};
+    for (const auto &c : closed) {
+        mprotect(c.at, page, c.prot);
+        if (des::pages_ready(p + 8, n - 16, false) != c.read || des::pages_ready(p + 8, n - 16, true) != c.write) fail(c.what);
+        if (des::pages_ready(c.at + 8, 16, false) != c.read || des::pages_ready(c.at + 8, 16, true) != c.write) fail(c.what);
+        mprotect(c.at, page, PROT_READ | PROT_WRITE);
+    }
+    munmap(p + n / 2, page);
+    if (des::pages_ready(p, n, false) || des::pages_ready(p, n, true)) fail("an unmapped page in the middle");
+    if (des::pages_ready(p, n / 2 + 1, false) || des::pages_ready(p, n / 2 + 1, true)) fail("an unmapped page at the end");
+    if (!des::pages_ready(p, n / 2, true)) fail("the pages before it");
     printf("%d mismatches\n", bad);
     return bad != 0;
 }
