@@ -41,7 +41,7 @@ B_NODE = 3 * 8 * 2 * 2 + 8 * 2 + 4
 
 # DRAM bytes (read + written) per element of each FP64 pass from one ncu
 # capture of the pass alone on a 100x100x40 box of config 2's physics
-TRAFFIC_PER_ELEM = {"N-A": 88.2, "E-B": 416.7, "N-B": 26.3, "E-C": 317.5, "N-C": 135.5, "E-A": 638.6}
+TRAFFIC_PER_ELEM = {"N-A": 88.1, "E-B": 416.5, "N-B": 26.3, "E-C": 308.2, "N-C": 135.9, "E-A": 638.4}
 
 
 def peaks():

@@ -8,8 +8,9 @@
 // DMUL or DFMA at 4 to 32 warps per SM; one warp alone gets one per 68
 // clocks), and the reference's arithmetic for E-A is 385 of them per element.
 // Every product and quotient is on the integer pipes here (sf::prod on
-// operands taken apart once, sf::div), which leaves 162 (41 + 89 + 32 over
-// the three kernels; E-C 41).
+// operands taken apart once, sf::div), and one of the rotation's three
+// sum-and-difference pairs, which leaves 154 (41 + 81 + 32 over the three
+// kernels; E-C 41).
 // Three kernels rather than one: the fused pass was limited by instruction
 // fetch (its 2,800 instructions of loop bodies exceed what the instruction
 // caches hold for warps at different places: a quarter of the warps' time
@@ -19,8 +20,9 @@
 // the same reason.
 // On a 100x100x40 box (2.4M elements): E-A 1,248 us before (one kernel, 92
 // products on the integer pipes, 260 FP64 instructions), 971 us fused with
-// all products on them, 839 us split (geometry 228, rates and rotation 418
-// at the FP64 pipe's peak, conduction 193); E-C 258 -> 211 us.
+// all products on them, 796 us split (geometry 231, rates and rotation 386
+// at the FP64 pipe's peak, conduction 175; 829 in the mean over steps, of which
+// every tenth forms dt); E-C 258 -> 211 us.
 #pragma once
 
 #include "des_kernels.cuh"

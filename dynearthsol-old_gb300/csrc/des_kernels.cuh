@@ -985,8 +985,8 @@ __device__ __forceinline__ void node_masses(const Dev &d, int q0, int q1, const 
 // N-A: start of a step (dynearthsol.cxx:358-362, 365 node half).  The masses'
 // additions (12 of the pass's 20 per element) and the two divisions are on
 // the integer pipes, the signed sums on the FP64 unit, so that both work:
-// 25 FP64 instructions per element before, at the pipe's measured peak, 9.7 now
-// (2.4M elements: 130 -> 90 us).  4 blocks of 256 per SM (5: 12 % slower, 6:
+// 23.1 FP64 instructions per element before, at the pipe's measured peak, 8.2 now
+// (2.4M elements: 137 -> 93 us).  4 blocks of 256 per SM (5: 12 % slower, 6:
 // 26 %, for the spills).
 __global__ void __launch_bounds__(256, 4) k_fn_a(Dev d)
 {
@@ -1114,7 +1114,7 @@ __global__ void __launch_bounds__(128, 8) k_fe_b_t(Dev d, int e0)
 
 // N-C: force gather, damping, velocity, velocity BCs, coordinates.  Its
 // products, its three divisions by one mass and a third of its additions are
-// on the integer pipes: 20.6 -> 13 FP64 instructions per element, 118 -> 89 us
+// on the integer pipes: 19.7 -> 10.5 FP64 instructions per element, 118 -> 90 us
 // for 2.4M elements (101 with the additions on the FP64 unit, which then is at
 // its peak).  The FP32 form's N-C lost by the same move (106 -> 128 us).
 __global__ void k_fn_c(Dev d)

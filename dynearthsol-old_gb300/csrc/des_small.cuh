@@ -4,8 +4,8 @@
 // same order, as des_kernels.cuh, des_elem.cuh and des_kernels32.cuh.  (One
 // warp alone gets an FP64 instruction per 68 clocks and about one other per 4.)
 // The FP64 step on 144 elements went from 55 to 31 us, on 9,600 from 65 to
-// 37; the FP32 step on 27,702 from 47 to 35.  E-B in quads gained 1 us of 11
-// at 144 elements and lost above 10k, and is not here.
+// 37; the FP32 step on 27,702 from 47 to 33.  E-B in quads gained 1.4 us of
+// 11.5 at 144 elements and lost 4 of 12.1 at 27k, and is not here.
 #pragma once
 
 #include "des_elem.cuh"
